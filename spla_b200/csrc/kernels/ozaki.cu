@@ -8,18 +8,26 @@
 // Method (Ozaki, Uchino & Imamura, "Ozaki Scheme II: A GEMM-oriented emulation
 // of floating-point matrix multiplication using an integer modular
 // technique", 2025), restated here in our own formulation:
-//   1. Complex products as three real ones (Karatsuba): with a = ar + i ai
-//      and b = br + i bi, P0 = ar.br, P1 = ai.bi, P2 = (ar + s ai).(br + bi),
-//      s = -1 for A^H (Re = P0 + P1, Im = P2 - P0 + P1) and +1 otherwise
-//      (Re = P0 - P1, Im = P2 - P0 - P1). Each is a real GEMM of depth k;
-//      the combination happens on the residues, before the reconstruction.
+//   1. Complex products as two real ones per modulus: the moduli of complex
+//      problems have -1 as a square, j^2 = -1 (mod p), and a = ar + i ai goes
+//      to u = ar + j ai and v = ar - j ai (mod p). Then U = u_a.u_b and
+//      V = v_a.v_b (for A^H, u_a and v_a swapped) are real GEMMs of depth k and
+//      Re = (U + V) / 2, Im = (U - V) / (2j) mod p, with the divisions folded
+//      into the reconstruction's weights: 32 real products for double (45 with
+//      Karatsuba on general moduli), which took the INT8 GEMM from 9.64 to 6.62
+//      ms at m = n = 1024, k = 250000 and, with k = 2048, n = 2048 and 200000 rows,
+//      from 31.9 to 22.0 ms (reconstruction 9.4 to 8.1 ms); float 27 -> 20. An
+//      explicit modulus count other
+//      than the default keeps the moduli of real problems (not of that kind)
+//      and three products (Karatsuba): P0 = ar.br, P1 = ai.bi, P2 = (ar + s ai).
+//      (br + bi), s = -1 for A^H (Re = P0 + P1, Im = P2 - P0 + P1) and +1
+//      otherwise (Re = P0 - P1, Im = P2 - P0 - P1).
 //   2. Scaling. Every row x (complex: its interleaved reals) is scaled by
 //      2^sigma so that ||2^sigma x||_2 < 2^Q and rounded to integers A', B'
 //      (exact in double). By Cauchy-Schwarz every entry of the real product,
 //      and Re and Im of the complex one, is below 2^(2Q) <= P/4.
 //   3. Residues. For pairwise coprime moduli p_t <= 256 with product P, the
-//      residues of A', B' mod p_t (symmetric, int8; the third complex plane
-//      is the reduced sum of the first two) are multiplied exactly on the
+//      residues of A', B' mod p_t (symmetric, int8) are multiplied exactly on the
 //      INT8 tensor cores with INT32 accumulation (k-chunks of at most 124928
 //      so that 128*128*chunk < 2^31), reduced mod p_t and summed over chunks.
 //   4. Reconstruction. The Chinese remainder theorem gives X exactly (|X| <=
@@ -32,7 +40,7 @@
 // int8, K-major, one plane per modulus and product), oz_row_scale_mn /
 // oz_slice_mn (the same for op(A) = N and op(B) = T, C read in place),
 // oz_transpose (op(A) = N copied K-major when k is too long for that),
-// oz_slice_tc (opt-in: digit sums on the tensor cores), oz_gemm_pair / oz_gemm
+// oz_gemm_pair / oz_gemm
 // (tcgen05.mma kind::i8, TMA-fed, TMEM accumulators, warp-specialised
 // persistent kernels), oz_reconstruct_tc (CRT sums on the tensor cores) and
 // oz_reconstruct / oz_reconstruct_staged (CRT on the CUDA cores), each with
@@ -288,13 +296,15 @@ __global__ void oz_row_scale(const TIn* __restrict__ X, int64_t ld_elems, int64_
 
 // Per-modulus constants of the slicer, each stored twice (both halves of an
 // f32x2 operand): -p, 1/p and the digit weights b^i mod p in symmetric form,
-// i = 1..4 (digit base b = 2^15 with four digits, else 2^13).
+// i = 1..4 (digit base b = 2^15 with four digits, else 2^13); with split moduli
+// also the weights of the imaginary part, j b^i mod p, i = 0..4 (-j for A^H).
 struct SliceConsts {
   int n;
   float p0;  // first modulus (256: residue = low byte of the lowest digit)
   unsigned long long neg_p[kMaxModuli];
   unsigned long long inv_p[kMaxModuli];
   unsigned long long c[kMaxModuli][4];
+  unsigned long long cj[kMaxModuli][5];
 };
 
 // Residues are computed on the FP32 pipe from digits of the scaled integer
@@ -380,6 +390,11 @@ __device__ __forceinline__ unsigned long long f2_fma(unsigned long long a, unsig
   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
   return d;
 }
+__device__ __forceinline__ unsigned long long f2_mul(unsigned long long a, unsigned long long b) {
+  unsigned long long d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
 __device__ __forceinline__ unsigned long long f2_add(unsigned long long a, unsigned long long b) {
   unsigned long long d;
   asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
@@ -395,8 +410,8 @@ __device__ __forceinline__ uint32_t pack4(float a, float b, float c, float d) {
 
 // The work of one slicing thread once its EL reals (of one row, starting at
 // real l0) are loaded: scaling by 2^sg, digits, and for every modulus the
-// residues written to res_row + l0 (mode 0) or, in mode 2, to the three
-// planes `plane` bytes apart at complex offset l0 / 2. SSQ: the sum of
+// residues written to res_row + l0 (mode 0) or, in modes 2 and 3, to the three
+// or two planes `plane` bytes apart at complex offset l0 / 2. SSQ: the sum of
 // squares of the scaled values is handed to on_ssq once the digits are made
 // (so that it is not kept in registers through the residue loop).
 struct NoSsq {
@@ -409,7 +424,7 @@ __device__ __forceinline__ void slice_thread(double (&v)[EL], int sg, int8_t* re
                                              int64_t res_mod_stride, const SliceConsts& sc,
                                              int t_begin, int t_end, OnSsq on_ssq = {}) {
   static_assert(EL == 8 || EL == 16, "8 or 16 reals per thread");
-  static_assert(MODE == 0 || MODE == 2, "real rows or complex rows");
+  static_assert(MODE == 0 || MODE == 2 || MODE == 3, "real rows, or complex rows in two forms");
   constexpr int W = EL / 4;  // packed words per modulus
   // 2^sg as a double when representable, else ldexp per element
   const bool direct = sg > -1000 && sg < 1000;
@@ -417,9 +432,9 @@ __device__ __forceinline__ void slice_thread(double (&v)[EL], int sg, int8_t* re
   unsigned long long dp[EL / 2][5];  // digits of the element pairs (see below)
   double ssq = 0.0;
   {
-    // pairs (2i, 2i + 1) in mode 0; in mode 2 the real parts pair up first,
+    // pairs (2i, 2i + 1) in mode 0; for complex rows the real parts pair up first,
     // then the imaginary parts: (re0, re1), (re2, re3), ..., (im0, im1), ...
-    if constexpr (MODE == 2) {
+    if constexpr (MODE != 0) {
       double u[EL];
 #pragma unroll
       for (int i = 0; i < EL / 2; ++i) {
@@ -444,9 +459,51 @@ __device__ __forceinline__ void slice_thread(double (&v)[EL], int sg, int8_t* re
   }
   const unsigned long long M2 = f2_pack(kMagic, kMagic), NM2 = f2_pack(-kMagic, -kMagic);
   int8_t* const out0 = res_row + l0;
+  constexpr int H = EL / 4;  // modes 2, 3: pairs of complex elements
+  // Mode 3, one modulus: with sr and si the digit sums of re and j im, u = sr +
+  // si (accumulated in one chain) and -v = u - 2 sr, each exact in FP32: with
+  // four digits of base 2^15 and weights |c| <= h = (p - 1) / 2 <= 120, |u| and
+  // |v| <= 2^14 (1 + 6 h) < 1.2e7 < 2^24, and less with the others. V's planes
+  // hold -v for both operands, which leaves the products. The quotients are
+  // below 49400, so their error (2^-24 relative from 1/p) is below 0.003: the
+  // nearest integer or, next to a half, its neighbour, |r| <= 121: one signed
+  // byte. 16 operations per complex element and modulus against 19 in mode 2.
+  auto modulus_split = [&](const int t) {
+    const unsigned long long np = sc.neg_p[t], ip = sc.inv_p[t];
+    const unsigned long long TWO = f2_pack(-2.0f, -2.0f);
+    unsigned long long ru[H], rv[H];
+#pragma unroll
+    for (int h = 0; h < H; ++h) {
+      unsigned long long sr = f2_fma(sc.c[t][0], dp[h][1], dp[h][0]);
+#pragma unroll
+      for (int d = 2; d < NDIG; ++d) sr = f2_fma(sc.c[t][d - 1], dp[h][d], sr);
+      unsigned long long u = f2_fma(sc.cj[t][0], dp[H + h][0], sr);
+#pragma unroll
+      for (int d = 1; d < NDIG; ++d) u = f2_fma(sc.cj[t][d], dp[H + h][d], u);
+      const unsigned long long v = f2_fma(sr, TWO, u);
+      const unsigned long long qu = f2_add(f2_fma(u, ip, M2), NM2);
+      const unsigned long long qv = f2_add(f2_fma(v, ip, M2), NM2);
+      ru[h] = f2_add(f2_fma(qu, np, u), M2);
+      rv[h] = f2_add(f2_fma(qv, np, v), M2);
+    }
+    int8_t* o = out0 - l0 + l0 / 2 + t * res_mod_stride;  // complex offset l0 / 2
+#pragma unroll
+    for (int w = 0; w < H / 2; ++w) {
+      float a0, a1, a2, a3;
+      f2_unpack(ru[2 * w], a0, a1);
+      f2_unpack(ru[2 * w + 1], a2, a3);
+      *reinterpret_cast<uint32_t*>(o + 4 * w) = pack4(a0, a1, a2, a3);
+      f2_unpack(rv[2 * w], a0, a1);
+      f2_unpack(rv[2 * w + 1], a2, a3);
+      *reinterpret_cast<uint32_t*>(o + plane + 4 * w) = pack4(a0, a1, a2, a3);
+    }
+  };
   auto modulus = [&](const int t) {
+    if constexpr (MODE == 3) {
+      modulus_split(t);
+      return;
+    }
     int8_t* out = out0 + t * res_mod_stride;
-    constexpr int H = EL / 4;        // mode 2: pairs of complex elements
     unsigned long long rp2[EL / 2];  // MAGIC + residue of elements 2i, 2i + 1
     unsigned long long ri2[H];       // mode 2: residues of the imaginary pairs, unbiased
     if (t == 0 && sc.p0 == 256.0f) {
@@ -540,10 +597,12 @@ __device__ __forceinline__ void slice_thread(double (&v)[EL], int sg, int8_t* re
 //         res[t][2][row][e] = r(re + s_sum im) (residues are linear in the
 //         scaled integers, so the third is r(re) + s_sum r(im) reduced mod p).
 //         The input row then holds 2 kp reals (kp complex elements).
+// mode 3: complex rows with split moduli: res[t][0][row][e] = r(re + j im),
+//         res[t][1][row][e] = -r(re - j im).
 // TIn: double (|x| < 2^62, five digits) or float (|x| < 2^38, three digits).
 // NMU > 0: moduli 0 .. NMU-1 in one fully unrolled pass (the per-modulus
 // constants become fixed parameter operands); 0: t_begin .. t_end-1 in a loop.
-// MODE (0 or 2, the mode above) is a template parameter so that the unrolled
+// MODE (the mode above) is a template parameter so that the unrolled
 // modulus loop carries no branch on it.
 // The EL reals of one row at real l0 (zeros past len); VEC: 16-byte loads.
 template <typename TIn, bool VEC, int EL>
@@ -581,7 +640,7 @@ __global__ void __launch_bounds__(256, EL == 8 ? 4 : 2)
              const int* __restrict__ sigma, int s_sum, int8_t* __restrict__ res,
              int64_t res_mod_stride, SliceConsts sc, int t_begin, int t_end,
              double* __restrict__ rowssq) {
-  const int64_t groups = (MODE == 2 ? 2 * kp : kp) / EL;
+  const int64_t groups = (MODE != 0 ? 2 * kp : kp) / EL;
   const int64_t gid = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
   if constexpr (!SSQ) {
     const int row = int(gid / groups);
@@ -644,7 +703,7 @@ __global__ void __launch_bounds__(256, EL == 8 ? 4 : 2)
                   int64_t kp, const int* __restrict__ sigma, int s_sum,
                   int8_t* __restrict__ res, int64_t res_mod_stride, SliceConsts sc,
                   const int* __restrict__ list, const int* __restrict__ count) {
-  const int64_t groups = (MODE == 2 ? 2 * kp : kp) / EL;
+  const int64_t groups = (MODE != 0 ? 2 * kp : kp) / EL;
   const int64_t total = int64_t(*count) * groups;
   for (int64_t gid = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; gid < total;
        gid += int64_t(gridDim.x) * blockDim.x) {
@@ -787,7 +846,7 @@ __global__ void __launch_bounds__(256, 4)
                 const int* __restrict__ sigma, int s_sum, int conj, int8_t* __restrict__ res,
                 int64_t res_mod_stride, SliceConsts sc, int t_begin, int t_end) {
   constexpr int EL = 8;
-  constexpr int R = MODE == 2 ? 2 : 1;  // reals per element
+  constexpr int R = MODE != 0 ? 2 : 1;  // reals per element
   constexpr int G = EL / R;             // elements per thread
   constexpr int KT = 32 * G;            // elements per row per tile
   constexpr int ESZ = R * int(sizeof(TIn));
@@ -854,344 +913,6 @@ __global__ void __launch_bounds__(256, 4)
 }
 
 // --------------------------------------------------------------------------
-// 2b. residues of complex double rows with the digit sums on the tensor cores
-//
-// The digit sums above are a small integer matrix product. Written in
-// balanced base-256 digits, x = sum_j d_j 256^j with d_j in [-128, 127]
-// (eight digits cover |x| < 2^62), the residue of x mod p is that of
-// sum_j d_j w_j with w_j = 256^j mod p in symmetric form (|w_j| <= 127). A
-// complex element has 16 digits (8 of re, 8 of im), and its three planes are
-// three such sums: re uses w on the re digits, im w on the im digits, the
-// sum plane w on re and s_sum w on im. One tcgen05.mma kind::i8 (exact INT32)
-//   D[128 x 256] = W[128 x K] . Dig[K x 256]
-// computes them for G groups of 256 elements at once: the 16 digit bytes of
-// group g's element n are K bytes 16 g .. 16 g + 15 of B row n, and row
-// (g, t, q) of W holds the weights of modulus t and plane q on group g's
-// bytes; (nmod - 1) * 3 * G <= 128 rows (G = 3 for the default 15 moduli:
-// 126 rows, two K-steps of 32 bytes). The modulus 256 is the low byte of x and
-// is written by the producers directly. The epilogue reduces each sum
-// (|s| < 16 * 128 * 127 < 2^18) mod p on the FP32 pipe with 4 operations
-// per residue (against 7 for the digit-sum form plus 3 for the sum plane),
-// stages the bytes of its 256-element row segment in shared memory and writes
-// it with one bulk copy.
-//
-// Warps 0-7: epilogue (warp w reads TMEM lanes 32 (w % 4) .. + 31, one
-// (group, modulus, plane) row each, and columns 128 (w / 4) .. + 127, two
-// warps per lane quarter so that the TMEM loads and the reduction of one
-// overlap the other's); warps 8-11: producers (row scaling, digits into the
-// 128-byte-swizzled B tile, modulus-256 bytes); warp 12: TMEM allocation and
-// the MMA issue. Digits and accumulators are double-buffered; every wait is
-// bounded and a give-up sets *status. Each epilogue warp stages its 32 row
-// segments of 128 bytes in shared memory and writes them with coalesced
-// 16-byte stores (4 rows of 128 bytes per instruction; one bulk copy per row
-// segment measured 30 % slower: the copy engine's cost per small copy).
-struct SliceTcParams {
-  const double* X;        // rows of interleaved complex doubles
-  int64_t ld;             // row stride in doubles
-  int64_t len;            // complex elements per row
-  int rows;
-  int64_t kp;             // residue row length (complex elements, multiple of 128)
-  const int* sigma;       // row scale exponents
-  int s_sum;              // sign of im in the third plane
-  int8_t* res;            // res[t][q][row][e]
-  int64_t mod_stride;     // bytes between moduli
-  int64_t plane;          // bytes between the planes of one modulus
-  int nmod;               // moduli, p[0] = 256
-  int groups;             // groups of 256 elements per unit
-  int ksteps;             // K-steps of 32 bytes per unit
-  int units_per_row;
-  long long total_units;
-  int p[kMaxModuli];
-  int* status;
-  unsigned long long wait_limit_ns;
-};
-
-constexpr int TC_THREADS = 416;  // warps 0-7 epilogue, 8-11 producers, 12 MMA
-constexpr int TC_W_BYTES = 128 * 128;            // weights: 128 rows x 128 B (SW128)
-constexpr int TC_D_BYTES = 256 * 128;            // digits: 256 rows x 128 B (SW128)
-constexpr int TC_ROW_STAGE = 256 + 16;           // one staged row segment (padded)
-constexpr int TC_S_BYTES = 128 * TC_ROW_STAGE;   // staging of the 128 epilogue rows
-constexpr int TC_SMEM = TC_W_BYTES + 2 * TC_D_BYTES + 2 * TC_S_BYTES + 256 + 1024;
-
-__device__ __forceinline__ int sw128_chunk(int row, int chunk) {
-  return (row >> 3) * 1024 + (row & 7) * 128 + ((chunk ^ (row & 7)) << 4);
-}
-
-// round(y) as a 64-bit integer for |y| < 2^62, without conversion
-// instructions: y = xh 2^30 + xl_d, both parts read from the bits of
-// (value + 1.5 2^52).
-__device__ __forceinline__ long long round_to_int64(double y) {
-  constexpr double kM52 = 6755399441055744.0;  // 1.5 * 2^52: ulp 1
-  constexpr long long kM52Bits = 0x4338000000000000ll;
-  const double t = fma(y, 1.0 / 1073741824.0, kM52);   // kM52 + round(y 2^-30)
-  const double xl_d = fma(t - kM52, -1073741824.0, y);  // exact, |xl_d| <= 2^29
-  const long long xh = __double_as_longlong(t) - kM52Bits;
-  const int xl = int(__double2loint(xl_d + kM52));
-  return xh * 1073741824ll + xl;
-}
-
-// Balanced base-256 digits of x as bytes: d_j = byte_j(x + 0x0080..80) - 128
-// for j < 7 (the XOR flips the offset back), d_7 the signed top byte.
-__device__ __forceinline__ unsigned long long balanced_digits(long long x) {
-  constexpr unsigned long long kOff = 0x0080808080808080ull;
-  return (static_cast<unsigned long long>(x) + kOff) ^ kOff;
-}
-
-__global__ void __launch_bounds__(TC_THREADS, 1) oz_slice_tc(const __grid_constant__ SliceTcParams P) {
-  extern __shared__ unsigned char smem_raw[];
-  const uint32_t raw_addr = smem_u32(smem_raw);
-  const uint32_t base = (raw_addr + 1023u) & ~1023u;
-  unsigned char* bp = smem_raw + (base - raw_addr);
-  unsigned char* Wt = bp;
-  unsigned char* Dg = bp + TC_W_BYTES;
-  unsigned char* St = Dg + 2 * TC_D_BYTES;
-  const uint32_t w_addr = base, d_addr = base + TC_W_BYTES, s_addr = d_addr + 2 * TC_D_BYTES;
-  const uint32_t bar_base = s_addr + 2 * TC_S_BYTES;
-  auto dfull = [&](int b) { return bar_base + 8u * b; };
-  auto dempty = [&](int b) { return bar_base + 8u * (2 + b); };
-  auto accf = [&](int b) { return bar_base + 8u * (4 + b); };
-  auto acce = [&](int b) { return bar_base + 8u * (6 + b); };
-  const uint32_t drain_bar = bar_base + 64;
-  unsigned char* tail = St + 2 * TC_S_BYTES;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tail + 128);
-  volatile int* abort = reinterpret_cast<volatile int*>(tail + 136);
-
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int R3 = 3 * (P.nmod - 1);
-  const int wrows = P.groups * R3;
-
-  // weights: row L = (group g, modulus t >= 1, plane q), K byte k
-  for (int i = threadIdx.x; i < 128 * 128; i += blockDim.x) {
-    const int L = i >> 7, k = i & 127;
-    int w = 0;
-    if (L < wrows) {
-      const int g = L / R3, j = L - g * R3, t = 1 + j / 3, q = j - 3 * (j / 3);
-      const int kg = k - 16 * g;
-      if (kg >= 0 && kg < 16) {
-        const int part = kg >> 3, dj = kg & 7;  // part 0: re digits, 1: im digits
-        const int pt = P.p[t];
-        int c = 1;
-        for (int s = 0; s < dj; ++s) c = (c * 256) % pt;
-        if (c > pt / 2) c -= pt;
-        if (q == 0) w = part == 0 ? c : 0;
-        else if (q == 1) w = part == 1 ? c : 0;
-        else w = part == 0 ? c : P.s_sum * c;
-      }
-    }
-    Wt[sw128_chunk(L, k >> 4) + (k & 15)] = static_cast<unsigned char>(static_cast<signed char>(w));
-  }
-  // digit tiles start at zero: the bytes beyond the groups are read by the
-  // last K-step (against zero weights) and never written
-  for (int i = threadIdx.x; i < 2 * TC_D_BYTES / 16; i += blockDim.x)
-    reinterpret_cast<uint4*>(Dg)[i] = make_uint4(0u, 0u, 0u, 0u);
-  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-  if (threadIdx.x == 0) {
-    for (int b = 0; b < 2; ++b) {
-      mbar_init(dfull(b), 128);
-      mbar_init(dempty(b), 1);
-      mbar_init(accf(b), 1);
-      mbar_init(acce(b), 256);
-    }
-    mbar_init(drain_bar, 1);
-    *abort = 0;
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  if (warp == 12) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(
-                     smem_u32(tmem_slot))
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-  }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
-  const int unit_elems = 256 * P.groups;
-
-  if (warp >= 8 && warp < 12) {
-    // ---- producers: 2 G elements per thread and unit, consecutive threads
-    // on consecutive elements (coalesced 16-byte loads)
-    const int pt = threadIdx.x - 256;
-    const int per = 2 * P.groups;
-    // the elements of unit u, loaded one unit ahead of their use
-    auto load = [&](long long u, double2 (&v)[8]) {
-      const int row = int(u / P.units_per_row);
-      const int64_t e0 = (u - int64_t(row) * P.units_per_row) * unit_elems;
-      const double2* xr = reinterpret_cast<const double2*>(P.X + int64_t(row) * P.ld);
-#pragma unroll
-      for (int r = 0; r < 8; ++r) {
-        if (r < per) {
-          const int64_t e = e0 + pt + 128 * r;
-          v[r] = e < P.len ? __ldcs(xr + e) : make_double2(0.0, 0.0);
-        }
-      }
-    };
-    double2 v[8], vn[8];
-    if (blockIdx.x < P.total_units) load(blockIdx.x, vn);
-    for (long long u = blockIdx.x, it = 0; u < P.total_units; u += gridDim.x, ++it) {
-      const int b = int(it & 1);
-      const uint32_t par = uint32_t((it >> 1) & 1);
-      const int row = int(u / P.units_per_row);
-      const int64_t e0 = (u - int64_t(row) * P.units_per_row) * unit_elems;
-      const int sg = P.sigma[row];
-      const bool direct = sg > -1000 && sg < 1000;
-      const double scale = direct ? __longlong_as_double((long long)(sg + 1023) << 52) : 1.0;
-#pragma unroll
-      for (int r = 0; r < 8; ++r) v[r] = vn[r];
-      if (u + gridDim.x < P.total_units) load(u + gridDim.x, vn);
-      if (!mbar_wait(dempty(b), par ^ 1u, abort, P.wait_limit_ns)) break;
-      unsigned char* dg = Dg + b * TC_D_BYTES;
-      int8_t* r256 = P.res + int64_t(row) * P.kp;  // modulus 0 (256), plane 0
-#pragma unroll
-      for (int r = 0; r < 8; ++r) {
-        if (r < per) {
-          const int el = pt + 128 * r;
-          const int64_t e = e0 + el;
-          const double yr = direct ? v[r].x * scale : ldexp(v[r].x, sg);
-          const double yi = direct ? v[r].y * scale : ldexp(v[r].y, sg);
-          const long long x_re = round_to_int64(yr), x_im = round_to_int64(yi);
-          const unsigned long long dr = balanced_digits(x_re), di = balanced_digits(x_im);
-          *reinterpret_cast<uint4*>(dg + sw128_chunk(el & 255, el >> 8)) =
-              make_uint4(unsigned(dr), unsigned(dr >> 32), unsigned(di), unsigned(di >> 32));
-          if (e < P.kp) {
-            r256[e] = static_cast<int8_t>(x_re);
-            r256[P.plane + e] = static_cast<int8_t>(x_im);
-            r256[2 * P.plane + e] = static_cast<int8_t>(x_re + P.s_sum * x_im);
-          }
-        }
-      }
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      mbar_arrive(dfull(b));
-    }
-  } else if (warp == 12) {
-    if (lane == 0) {
-      // ---- MMA issuer
-      bool ok = true;
-      for (long long u = blockIdx.x, it = 0; u < P.total_units; u += gridDim.x, ++it) {
-        const int b = int(it & 1);
-        const uint32_t par = uint32_t((it >> 1) & 1);
-        if (!mbar_wait(dfull(b), par, abort, P.wait_limit_ns) ||
-            !mbar_wait(acce(b), par ^ 1u, abort, P.wait_limit_ns)) {
-          ok = false;
-          break;
-        }
-        tc_fence_after();
-        const uint32_t d = tmem_base + uint32_t(b * 256);
-        for (int kk = 0; kk < P.ksteps; ++kk)
-          umma_i8(d, umma_desc_sw128(w_addr + kk * 32),
-                  umma_desc_sw128(d_addr + b * TC_D_BYTES + kk * 32), kk > 0 ? 1u : 0u);
-        umma_commit(dempty(b));
-        umma_commit(accf(b));
-      }
-      if (!ok) {
-        umma_commit(drain_bar);  // MMAs may be in flight: wait (bounded) until they retire
-        const unsigned long long t0 = globaltimer();
-        while (!mbar_try_wait(drain_bar, 0) && globaltimer() - t0 < 1000000ull) {
-        }
-      }
-    }
-  } else if (warp < 8) {
-    // ---- epilogue: TMEM lane L = (group, modulus, plane) row, half of the columns
-    const int quarter = warp & 3, half = warp >> 2;
-    const int L = quarter * 32 + lane;
-    const bool active = L < wrows;
-    int g = 0, t = 1, q = 0;
-    if (active) {
-      g = L / R3;
-      const int j = L - g * R3;
-      t = 1 + j / 3;
-      q = j - 3 * (j / 3);
-    }
-    const float pf = float(P.p[t]);
-    const unsigned long long NP2 = f2_pack(-pf, -pf);
-    const unsigned long long IP2 = f2_pack(1.0f / pf, 1.0f / pf);
-    const unsigned long long M2 = f2_pack(kMagic, kMagic), NM2 = f2_pack(-kMagic, -kMagic);
-    const uint32_t seg_stage = uint32_t(L) * TC_ROW_STAGE + uint32_t(half * 128);
-    const uint32_t lane_taddr = tmem_base + (uint32_t(quarter * 32) << 16) + uint32_t(half * 128);
-    // 32 sums -> 32 residue bytes at st
-    auto reduce32 = [&](const uint32_t (&v)[32], unsigned char* st) {
-      uint32_t wv[8];
-#pragma unroll
-      for (int h = 0; h < 8; ++h) {
-        float r[4];
-#pragma unroll
-        for (int e2 = 0; e2 < 2; ++e2) {
-          const int c = 4 * h + 2 * e2;
-          // MAGIC + s exactly (|s| < 2^22), s, its nearest quotient by p,
-          // MAGIC + s - q p = MAGIC + (s mod p)
-          const unsigned long long tM = f2_pack(__int_as_float(0x4B400000 + int(v[c])),
-                                                __int_as_float(0x4B400000 + int(v[c + 1])));
-          const unsigned long long t2 = f2_add(tM, NM2);
-          const unsigned long long q2 = f2_add(f2_fma(t2, IP2, M2), NM2);
-          f2_unpack(f2_fma(q2, NP2, tM), r[2 * e2], r[2 * e2 + 1]);
-        }
-        wv[h] = pack4(r[0], r[1], r[2], r[3]);
-      }
-      *reinterpret_cast<uint4*>(st) = make_uint4(wv[0], wv[1], wv[2], wv[3]);
-      *reinterpret_cast<uint4*>(st + 16) = make_uint4(wv[4], wv[5], wv[6], wv[7]);
-    };
-    for (long long u = blockIdx.x, it = 0; u < P.total_units; u += gridDim.x, ++it) {
-      const int b = int(it & 1);
-      const uint32_t par = uint32_t((it >> 1) & 1);
-      if (!mbar_wait(accf(b), par, abort, P.wait_limit_ns)) break;
-      tc_fence_after();
-      unsigned char* st = St + b * TC_S_BYTES + seg_stage;
-      const uint32_t taddr = lane_taddr + uint32_t(b * 256);
-      // four chunks of 32 columns; the load of chunk c + 1 is in flight while
-      // chunk c is reduced
-      uint32_t va[32], vb[32];
-      tmem_ld32_nowait(taddr, va);
-      tmem_wait_ld();
-      tmem_ld32_nowait(taddr + 32, vb);
-      if (active) reduce32(va, st);
-      tmem_wait_ld();
-      tmem_ld32_nowait(taddr + 64, va);
-      if (active) reduce32(vb, st + 32);
-      tmem_wait_ld();
-      tmem_ld32_nowait(taddr + 96, vb);
-      if (active) reduce32(va, st + 64);
-      tmem_wait_ld();
-      tc_fence_before();
-      mbar_arrive(acce(b));  // TMEM buffer b is free for the MMA of unit it + 2
-      if (active) reduce32(vb, st + 96);
-      const int row = int(u / P.units_per_row);
-      const int64_t e_unit = (u - int64_t(row) * P.units_per_row) * unit_elems;
-      // this lane's row segment: destination and valid bytes (a multiple of 16)
-      const int64_t e = e_unit + 256 * g + 128 * half;
-      const int64_t nb = active ? (P.kp - e < 128 ? P.kp - e : 128) : 0;
-      int8_t* dst = P.res + t * P.mod_stride + q * P.plane + int64_t(row) * P.kp + e;
-      {
-        // coalesced: per instruction 4 rows x 8 lanes x 16 bytes
-        __syncwarp();
-        const unsigned long long dst_u = reinterpret_cast<unsigned long long>(dst);
-        const unsigned char* wst = St + b * TC_S_BYTES + uint32_t(quarter * 32) * TC_ROW_STAGE +
-                                   uint32_t(half * 128);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const int r = 4 * i + (lane >> 3), c = lane & 7;
-          const unsigned long long rd = __shfl_sync(0xffffffffu, dst_u, r);
-          const int64_t rn = __shfl_sync(0xffffffffu, nb, r);
-          if (16 * c < rn)
-            *reinterpret_cast<uint4*>(reinterpret_cast<int8_t*>(rd) + 16 * c) =
-                *reinterpret_cast<const uint4*>(wst + r * TC_ROW_STAGE + 16 * c);
-        }
-        __syncwarp();
-      }
-    }
-  }
-
-  tc_fence_before();
-  __syncthreads();
-  if (*abort && threadIdx.x == 0) atomicExch(P.status, 1);
-  if (warp == 12) {
-    __syncwarp();
-    tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem_base)
-                 : "memory");
-  }
-}
-
-// --------------------------------------------------------------------------
 // 3. INT8 residue GEMM on tcgen05
 
 struct GemmParams {
@@ -1201,7 +922,7 @@ struct GemmParams {
   int nchunks;       // ceil(kblocks / kChunkBlocks)
   int chunk_blocks;  // k-blocks per chunk: ceil(kblocks / nchunks) <= kChunkBlocks
   int nmod;          // products: moduli x nsub (the A/B/R planes in order)
-  int nsub;          // products per modulus (3 complex, 1 real): modulus = product / nsub
+  int nsub;          // products per modulus (Layout::nsub): modulus = product / nsub
   int t0;            // first product of this launch (units cover t0 ..)
   int tiles_m, tiles_n;
   int total_units;   // moduli of the launch * nchunks * tiles
@@ -1752,14 +1473,16 @@ __device__ __forceinline__ void store_c(void* C, int64_t ci, double xr, double x
 }
 
 // Residues of element (i, j) of the real result (real types) or of Re and Im
-// (complex: three product planes per modulus combined by combine3), for
-// modulus t. src points at plane 0 of modulus t, element (i, j); planes of
-// one product are `plane` elements apart. off: p for byte residues, off24 for
-// int32 sums.
-template <bool CPLX, typename RT>
+// (complex: two product planes per modulus combined by combine_split, or three
+// by combine3), for modulus t. src points at plane 0 of modulus t, element
+// (i, j); planes of one product are `plane` elements apart. off: p for byte
+// residues, off24 for int32 sums.
+template <bool CPLX, bool SPLIT, typename RT>
 __device__ __forceinline__ void product_residues(const RT* src, int64_t plane, int off, int conj,
                                                  int& re, int& im) {
-  if (CPLX) {
+  if (SPLIT) {
+    combine_split(int(src[0]), int(src[plane]), off, re, im);
+  } else if (CPLX) {
     combine3(int(src[0]), int(src[plane]), int(src[2 * plane]), off, conj, re, im);
   } else {
     re = int(src[0]);
@@ -1772,7 +1495,7 @@ __device__ __forceinline__ void product_residues(const RT* src, int64_t plane, i
 // int32 sums of per-chunk residues or, with one k-chunk, the residues as
 // bytes (RT). Threads run along i (contiguous in R and C), blocks along j: no
 // index division. NM: the number of moduli when fixed at compile time (the
-// defaults), 0 for rp.n.
+// defaults; the complex ones are the split moduli), 0 for rp.n.
 template <int DT, typename RT, int NM>
 __global__ void __launch_bounds__(256, 2) oz_reconstruct(const RT* __restrict__ R, int m, int n,
                                                          int nb, const int* __restrict__ sigA,
@@ -1782,7 +1505,8 @@ __global__ void __launch_bounds__(256, 2) oz_reconstruct(const RT* __restrict__ 
                                                          int64_t ro, int64_t co, int tile_m,
                                                          int tile_n, ReconParams rp) {
   constexpr bool CPLX = dtype_is_complex(DT);
-  constexpr int NSUB = CPLX ? 3 : 1;
+  constexpr bool SPLIT = CPLX && NM > 0;
+  constexpr int NSUB = SPLIT ? 2 : CPLX ? 3 : 1;
   constexpr bool kBytes = sizeof(RT) == 1;
   constexpr int NMAX = NM > 0 ? NM : kMaxUsableModuli;
   const int nmod = NM > 0 ? NM : rp.n;
@@ -1803,12 +1527,12 @@ __global__ void __launch_bounds__(256, 2) oz_reconstruct(const RT* __restrict__ 
 #pragma unroll
       for (int t = 0; t < NMAX; ++t)
         if (t < nmod)
-          product_residues<CPLX>(src + t * NSUB * plane, plane, kBytes ? rp.p[t] : rp.off24[t],
-                                 rp.conj, rr[t], ri[t]);
+          product_residues<CPLX, SPLIT>(src + t * NSUB * plane, plane,
+                                        kBytes ? rp.p[t] : rp.off24[t], rp.conj, rr[t], ri[t]);
       const int si = sigA[i];
       const int e = -(si + tauj);
       double xr = scale_pow2(crt_value<NM, kBytes>(rr, rp), e);
-      double xi = CPLX ? scale_pow2(crt_value<NM, kBytes>(ri, rp), e) : 0.0;
+      double xi = CPLX ? scale_pow2(crt_value<NM, kBytes, SPLIT>(ri, rp), e) : 0.0;
       if (si == kSigmaNonFinite || tauj == kSigmaNonFinite) xr = xi = __longlong_as_double(kNaNBits);
       store_c<DT>(C, i + int64_t(j) * ldc, xr, xi, alr, ali, ber, bei, read_c);
     }
@@ -1855,7 +1579,8 @@ __global__ void __launch_bounds__(256, 2)
                           int64_t ldc, double alr, double ali, double ber, double bei, int fill,
                           int64_t ro, int64_t co, int tile_m, int tile_n, ReconParams rp) {
   constexpr bool CPLX = dtype_is_complex(DT);
-  constexpr int NSUB = CPLX ? 3 : 1;
+  constexpr bool SPLIT = CPLX && NM > 0;
+  constexpr int NSUB = SPLIT ? 2 : CPLX ? 3 : 1;
   constexpr int NMAX = NM > 0 ? NM : kMaxUsableModuli;
   constexpr int WPP = kStageRows / 4;  // 32-bit words per staged plane
   extern __shared__ uint4 stage_smem[];
@@ -1910,7 +1635,11 @@ __global__ void __launch_bounds__(256, 2)
           if (t < nmod) {
             const unsigned* wt = w + t * NSUB * WPP;
             const int r0 = int((wt[0] >> (8 * q)) & 255u);
-            if (CPLX) {
+            if (SPLIT) {
+              int re, im;
+              combine_split(r0, int((wt[WPP] >> (8 * q)) & 255u), rp.p[t], re, im);
+              r[t] = part ? im : re;
+            } else if (CPLX) {
               const int r1 = int((wt[WPP] >> (8 * q)) & 255u);
               const int r2 = int((wt[2 * WPP] >> (8 * q)) & 255u);
               int re, im;
@@ -1932,7 +1661,7 @@ __global__ void __launch_bounds__(256, 2)
         double xi = 0.0;
         if (CPLX) {
           part_residues(q, 1, r);
-          xi = scale_pow2(crt_value<NM, true>(r, rp), e);
+          xi = scale_pow2(crt_value<NM, true, SPLIT>(r, rp), e);
         }
         if (si == kSigmaNonFinite || tauj == kSigmaNonFinite) xr = xi = __longlong_as_double(kNaNBits);
         store_c<DT>(C, i + q + int64_t(j) * ldc, xr, xi, alr, ali, ber, bei, read_c);
@@ -1944,19 +1673,17 @@ __global__ void __launch_bounds__(256, 2)
   cp_async_wait<0>();
 }
 
-inline int staged_smem_bytes(bool cplx, int nmod) {
-  return 2 * (cplx ? 3 : 1) * nmod * kStageRows;
-}
+inline int staged_smem_bytes(int planes) { return 2 * planes * kStageRows; }
 
 // --------------------------------------------------------------------------
 // 4b. CRT reconstruction on the tensor cores (byte residues, m % 16 == 0)
 //
 // By linearity the CRT sum needs no reduction of the product combination:
-// with V_k the weight of product plane k, W_t for the plane's modulus t where
-// the product enters Re or Im with a plus sign and P - W_t where it enters
-// with a minus (Re = P0 -+ P1, Im = P2 - P0 -+ P1, see combine3; p_t W_t = 0
-// mod P), S = sum_k r_k V_k is congruent mod P to the sum the CUDA-core
-// kernels form. Written in the bytes of V_k, S = sum_j 256^j S_j with
+// with V_k the weight of product plane k, W_t (or the Im weight of a split
+// modulus) for the plane's modulus t where the product enters Re or Im with a
+// plus sign and P - W_t where it enters with a minus (see combine_split and
+// combine3; p_t W_t = 0 mod P), S = sum_k r_k V_k is congruent mod P to the sum
+// the CUDA-core kernels form. Written in the bytes of V_k, S = sum_j 256^j S_j with
 // S_j = sum_k r_k byte_j(V_k), and for 128 consecutive rows of one column of
 // C one tcgen05.mma kind::i8 (unsigned bytes, exact INT32 sums below 2^22)
 //   D[128 x NO] = R[128 x KP] . V[KP x NO]
@@ -2245,7 +1972,8 @@ __global__ void __launch_bounds__(RT_THREADS, 3)
 
 struct Layout {
   int nmod;
-  int nsub;                // products per modulus: 3 (complex, Karatsuba) or 1 (real)
+  bool split;              // complex with the split moduli
+  int nsub;                // products per modulus: 1 (real), 2 (split) or 3 (Karatsuba)
   int64_t K2, kp;          // reals per operand row; residue row length (k padded to 128)
   int rowsA, rowsB, nb;    // A rows, B rows, B residue rows per product
   bool at;                 // op(A) = N too long for in-place tiles: A copied k-major
@@ -2262,6 +1990,8 @@ struct Layout {
 };
 
 size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
+
+Crt crt_of(const Layout& L) { return L.split ? make_crt_split(L.nmod) : make_crt(L.nmod); }
 
 // In-place reading of an m-major operand: the transposing slicer's tiles of
 // 128 (complex) or 256 (real) elements along k must fit the grid's y extent.
@@ -2282,10 +2012,17 @@ int norm_slices(int64_t rows, int64_t k) {
 
 Layout layout_of(const GemmProblem& p, int moduli) {
   Layout L{};
-  L.nmod = moduli > 0 ? std::min(moduli, kMaxUsableModuli)
-                      : (dtype_is_double(p.dtype) ? kDefaultModuli : kDefaultModuliFloat);
-  const bool cplx = dtype_is_complex(p.dtype);
-  L.nsub = cplx ? 3 : 1;
+  const bool dbl = dtype_is_double(p.dtype), cplx = dtype_is_complex(p.dtype);
+  const int def = dbl ? kDefaultModuli : kDefaultModuliFloat;
+  const int count = moduli > 0 ? std::min(moduli, kMaxUsableModuli) : def;
+  // complex problems at the default precision take the split moduli; another
+  // count names that many moduli of the general table
+  L.split = cplx && count == def;
+  L.nmod = L.split ? (dbl ? kSplitCount : kSplitCountFloat) : count;
+  L.nsub = L.split ? 2 : cplx ? 3 : 1;
+  // The workspace keeps the size of the three-product form for callers that
+  // hold one sized for it (32 planes of the split form lie in the room of 45)
+  const size_t planes = size_t(count) * (cplx ? 3 : 1);
   L.K2 = cplx ? 2 * p.k : p.k;
   L.kp = (p.k + BKB - 1) / BKB * BKB;
   L.rowsA = int(p.m);
@@ -2306,11 +2043,11 @@ Layout layout_of(const GemmProblem& p, int moduli) {
   L.off_sigB = off;
   off = align256(off + sizeof(int) * L.rowsB);
   L.off_resA = off;
-  off = align256(off + size_t(L.nmod) * L.nsub * L.rowsA * L.kp);
+  off = align256(off + planes * L.rowsA * L.kp);
   L.off_resB = off;
-  off = align256(off + size_t(L.nmod) * L.nsub * L.nb * L.kp);
+  off = align256(off + planes * L.nb * L.kp);
   L.off_R = off;
-  off = align256(off + (L.r8 ? 1 : sizeof(int)) * size_t(L.nmod) * L.nsub * L.nb * L.rowsA);
+  off = align256(off + (L.r8 ? 1 : sizeof(int)) * planes * L.nb * L.rowsA);
   L.off_At = off;
   off = align256(off + size_t(dtype_bytes(p.dtype)) * size_t(L.rowsA) * size_t(L.ldAt));
   L.off_status = off;
@@ -2406,8 +2143,17 @@ int slice_elems() {
   return el;
 }
 
-// The default modulus count of the input type (15 for double, 9 for float)
-// over all moduli runs unrolled (SPLAB_OZAKI_SLICE_UNROLL=0 keeps the loop).
+// Moduli of the unrolled slicers: the default counts of the input type, real
+// (MODE 0) or complex with split moduli (MODE 3); 0 in MODE 2 (always a loop).
+template <typename TIn, int MODE>
+constexpr int unrolled_moduli() {
+  return MODE == 0   ? (sizeof(TIn) == 8 ? oz::kDefaultModuli : oz::kDefaultModuliFloat)
+         : MODE == 3 ? (sizeof(TIn) == 8 ? oz::kSplitCount : oz::kSplitCountFloat)
+                     : 0;
+}
+
+// The default modulus counts over all moduli run unrolled
+// (SPLAB_OZAKI_SLICE_UNROLL=0 keeps the loop).
 bool slice_unroll() {
   static const bool on = [] {
     const char* v = std::getenv("SPLAB_OZAKI_SLICE_UNROLL");
@@ -2421,16 +2167,18 @@ void launch_slice_el(int ndig, unsigned grid, cudaStream_t st, const TIn* X, int
                      int64_t len, int rows, int64_t kp, const int* sig, int s_sign, int8_t* res,
                      int64_t stride, const oz::SliceConsts& sc, int t0, int t1, double* ssq) {
   using namespace oz;
-  constexpr int kNU = sizeof(TIn) == 8 ? kDefaultModuli : kDefaultModuliFloat;
+  constexpr int kNU = unrolled_moduli<TIn, MODE>();
   constexpr int kDigU = sizeof(TIn) == 8 ? 4 : 3;  // digits of the default scaling
-  if (t0 == 0 && t1 == kNU && sc.n == kNU && ndig == kDigU && slice_unroll()) {
-    if (ssq)
-      oz_slice<TIn, VEC, kDigU, EL, kNU, MODE, true><<<grid, 256, 0, st>>>(
-          X, ld, len, rows, kp, sig, s_sign, res, stride, sc, t0, t1, ssq);
-    else
-      oz_slice<TIn, VEC, kDigU, EL, kNU, MODE><<<grid, 256, 0, st>>>(
-          X, ld, len, rows, kp, sig, s_sign, res, stride, sc, t0, t1, nullptr);
-    return;
+  if constexpr (kNU > 0) {
+    if (t0 == 0 && t1 == kNU && sc.n == kNU && ndig == kDigU && slice_unroll()) {
+      if (ssq)
+        oz_slice<TIn, VEC, kDigU, EL, kNU, MODE, true><<<grid, 256, 0, st>>>(
+            X, ld, len, rows, kp, sig, s_sign, res, stride, sc, t0, t1, ssq);
+      else
+        oz_slice<TIn, VEC, kDigU, EL, kNU, MODE><<<grid, 256, 0, st>>>(
+            X, ld, len, rows, kp, sig, s_sign, res, stride, sc, t0, t1, nullptr);
+      return;
+    }
   }
   if (ndig <= 3)
     oz_slice<TIn, VEC, 3, EL, 0, MODE><<<grid, 256, 0, st>>>(
@@ -2449,7 +2197,7 @@ void launch_slice(int ndig, cudaStream_t st, const TIn* X, int64_t ld, int64_t l
                   int64_t kp, const int* sig, int mode, int s_sign, int8_t* res, int64_t stride,
                   const oz::SliceConsts& sc, int t0, int t1, double* ssq = nullptr) {
   const int el = slice_elems();
-  const int64_t kreal = mode == 2 ? 2 * kp : kp;  // reals per row a thread group covers
+  const int64_t kreal = mode != 0 ? 2 * kp : kp;  // reals per row a thread group covers
   const unsigned grid = unsigned((int64_t(rows) * (kreal / el) + 255) / 256);
   auto run = [&](auto el_tag, auto mode_tag) {
     launch_slice_el<TIn, VEC, decltype(el_tag)::value, decltype(mode_tag)::value>(
@@ -2459,13 +2207,14 @@ void launch_slice(int ndig, cudaStream_t st, const TIn* X, int64_t ld, int64_t l
   using E16 = std::integral_constant<int, 16>;
   using M0 = std::integral_constant<int, 0>;
   using M2 = std::integral_constant<int, 2>;
-  if (el == 16) {
-    if (mode == 2) run(E16{}, M2{});
-    else run(E16{}, M0{});
-  } else {
-    if (mode == 2) run(E8{}, M2{});
-    else run(E8{}, M0{});
-  }
+  using M3 = std::integral_constant<int, 3>;
+  auto by_mode = [&](auto el_tag) {
+    if (mode == 3) run(el_tag, M3{});
+    else if (mode == 2) run(el_tag, M2{});
+    else run(el_tag, M0{});
+  };
+  if (el == 16) by_mode(E16{});
+  else by_mode(E8{});
 }
 
 // Residues of m-major rows (op(A) = N read in place): oz_slice_mn
@@ -2474,12 +2223,14 @@ void launch_slice_mn_v(int ndig, dim3 grid, cudaStream_t st, const TIn* X, int64
                        int64_t k, int64_t kp, const int* sig, int s_sign, int conj, int8_t* res,
                        int64_t stride, const oz::SliceConsts& sc, int t0, int t1) {
   using namespace oz;
-  constexpr int kNU = sizeof(TIn) == 8 ? kDefaultModuli : kDefaultModuliFloat;
+  constexpr int kNU = unrolled_moduli<TIn, MODE>();
   constexpr int kDigU = sizeof(TIn) == 8 ? 4 : 3;
-  if (t0 == 0 && t1 == kNU && sc.n == kNU && ndig == kDigU && slice_unroll()) {
-    oz_slice_mn<TIn, VEC, kDigU, kNU, MODE>
-        <<<grid, 256, 0, st>>>(X, ld, m, k, kp, sig, s_sign, conj, res, stride, sc, t0, t1);
-    return;
+  if constexpr (kNU > 0) {
+    if (t0 == 0 && t1 == kNU && sc.n == kNU && ndig == kDigU && slice_unroll()) {
+      oz_slice_mn<TIn, VEC, kDigU, kNU, MODE>
+          <<<grid, 256, 0, st>>>(X, ld, m, k, kp, sig, s_sign, conj, res, stride, sc, t0, t1);
+      return;
+    }
   }
   if (ndig <= 3)
     oz_slice_mn<TIn, VEC, 3, 0, MODE>
@@ -2496,19 +2247,24 @@ template <typename TIn>
 void launch_slice_mn(int ndig, cudaStream_t st, const TIn* X, int64_t ld, int m, int64_t k,
                      int64_t kp, const int* sig, int mode, int s_sign, int conj, int8_t* res,
                      int64_t stride, const oz::SliceConsts& sc, int t0, int t1) {
-  const int64_t kt = mode == 2 ? 128 : 256;  // elements per row per tile
+  const int64_t kt = mode != 0 ? 128 : 256;  // elements per row per tile
   const dim3 grid(unsigned((m + 7) / 8), unsigned((kp + kt - 1) / kt));
-  if (mode == 2) {
-    // 16-byte element loads for complex double with a 16-byte aligned base
-    if (sizeof(TIn) == 8 && reinterpret_cast<uintptr_t>(X) % 16 == 0)
-      launch_slice_mn_v<TIn, true, 2>(ndig, grid, st, X, ld, m, k, kp, sig, s_sign, conj, res,
-                                      stride, sc, t0, t1);
-    else
-      launch_slice_mn_v<TIn, false, 2>(ndig, grid, st, X, ld, m, k, kp, sig, s_sign, conj, res,
-                                       stride, sc, t0, t1);
+  auto run = [&](auto vec_tag, auto mode_tag) {
+    launch_slice_mn_v<TIn, decltype(vec_tag)::value, decltype(mode_tag)::value>(
+        ndig, grid, st, X, ld, m, k, kp, sig, s_sign, conj, res, stride, sc, t0, t1);
+  };
+  using T = std::true_type;
+  using F = std::false_type;
+  // 16-byte element loads for complex double with a 16-byte aligned base
+  const bool vec = sizeof(TIn) == 8 && reinterpret_cast<uintptr_t>(X) % 16 == 0;
+  if (mode == 3) {
+    if (vec) run(T{}, std::integral_constant<int, 3>{});
+    else run(F{}, std::integral_constant<int, 3>{});
+  } else if (mode == 2) {
+    if (vec) run(T{}, std::integral_constant<int, 2>{});
+    else run(F{}, std::integral_constant<int, 2>{});
   } else {
-    launch_slice_mn_v<TIn, false, 0>(ndig, grid, st, X, ld, m, k, kp, sig, s_sign, conj, res,
-                                     stride, sc, t0, t1);
+    run(F{}, std::integral_constant<int, 0>{});
   }
 }
 
@@ -2547,56 +2303,10 @@ void scale_operands(const oz::Layout& L, const oz::Crt& crt, const GemmProblem& 
                                                L.rowsB, crt.q_bits, sigB);
 }
 
-// Residue slicing of complex double rows with the digit sums on the tensor
-// cores (oz_slice_tc), selected by SPLAB_OZAKI_SLICE_TC=1 (read per call, so
-// that tests compare both slicers in one process); used for all moduli at once
-// when the modulus 256 comes first and the rows are 16-byte aligned. The FP32
-// digit-sum slicer (oz_slice) is the default: on B200 it measured faster
-// (headline problem: 5.25 + 4.75 ms against 5.77 + 5.10 ms for the residues
-// of A and B), the tensor-core form being bound by instruction issue and
-// latency (TMEM round trip, staging, synchronisation) rather than by the FP32
-// pipe it relieves.
-bool slice_tc_enabled() {
-  const char* v = std::getenv("SPLAB_OZAKI_SLICE_TC");
-  return v && v[0] == '1';
-}
-
-cudaError_t launch_slice_tc(const double* X, int64_t ld, int64_t len, int rows, int64_t kp,
-                            const int* sig, int s_sum, int8_t* res, int64_t mod_stride,
-                            int64_t plane, const oz::Crt& crt, int nmod, int* status,
-                            cudaStream_t st) {
-  using namespace oz;
-  SliceTcParams P{};
-  P.X = X;
-  P.ld = ld;
-  P.len = len;
-  P.rows = rows;
-  P.kp = kp;
-  P.sigma = sig;
-  P.s_sum = s_sum;
-  P.res = res;
-  P.mod_stride = mod_stride;
-  P.plane = plane;
-  P.nmod = nmod;
-  const int r3 = 3 * (nmod - 1);
-  P.groups = std::min(4, 128 / r3);
-  P.ksteps = (16 * P.groups + 31) / 32;
-  P.units_per_row = int((kp + 256 * P.groups - 1) / (256 * P.groups));
-  P.total_units = (long long)rows * P.units_per_row;
-  for (int t = 0; t < nmod; ++t) P.p[t] = crt.p[t];
-  P.status = status;
-  P.wait_limit_ns = kWaitLimitNs;
-  if (P.total_units <= 0) return cudaSuccess;
-  cudaError_t e = set_dynamic_smem(reinterpret_cast<const void*>(oz_slice_tc), TC_SMEM);
-  if (e != cudaSuccess) return e;
-  const long long grid = std::min<long long>(P.total_units, sm_count());
-  oz_slice_tc<<<unsigned(grid), TC_THREADS, TC_SMEM, st>>>(P);
-  return cudaGetLastError();
-}
-
-// Slicer constants of the moduli, and the digit count covering |x| <= 2^Q:
-// 3 of 13 bits, 4 balanced of 15 bits, or 5 of 13.
-oz::SliceConsts slice_consts(const oz::Layout& L, const oz::Crt& crt, int* ndig_out) {
+// Slicer constants of the moduli (s_sign: the sign of j, split moduli), and the
+// digit count covering |x| <= 2^Q: 3 of 13 bits, 4 balanced of 15 bits, or 5 of
+// 13.
+oz::SliceConsts slice_consts(const oz::Layout& L, const oz::Crt& crt, int s_sign, int* ndig_out) {
   using namespace oz;
   SliceConsts sc{};
   sc.n = L.nmod;
@@ -2610,11 +2320,16 @@ oz::SliceConsts slice_consts(const oz::Layout& L, const oz::Crt& crt, int* ndig_
   const long long base = ndig == 4 ? 32768 : 8192;
   for (int t = 0; t < L.nmod; ++t) {
     const int pt = crt.p[t];
-    long long w = 1;
-    for (int i = 0; i < 4; ++i) {
-      w = (w * base) % pt;  // base^(i+1) mod p
+    auto centred = [pt](long long w) {
       const float c = float(w > pt / 2 ? w - pt : w);
-      sc.c[t][i] = f2_pack(c, c);
+      return f2_pack(c, c);
+    };
+    const int j = s_sign > 0 ? crt.j[t] : pt - crt.j[t];
+    long long w = 1;
+    for (int i = 0; i < 5; ++i) {  // w = base^i mod p
+      if (i > 0) sc.c[t][i - 1] = centred(w);
+      if (L.split) sc.cj[t][i] = centred(w * j % pt);
+      w = (w * base) % pt;
     }
   }
   *ndig_out = ndig;
@@ -2632,43 +2347,28 @@ void slice_operands(const oz::Layout& L, const oz::Crt& crt, const GemmProblem& 
   const TIn* B = static_cast<const TIn*>(p.B);
   const int64_t ldA = cplx ? 2 * p.lda : p.lda;  // in real elements
   const int64_t ldB = cplx ? 2 * p.ldb : p.ldb;
-  if (std::is_same<TIn, double>::value && cplx && t0 == 0 && t1 == L.nmod && crt.p[0] == 256 &&
-      L.nmod >= 2 && !((which & 1) && L.mn) && !((which & 2) && L.mnB) && slice_tc_enabled()) {
-    const double* Ad = reinterpret_cast<const double*>(A);
-    const double* Bd = reinterpret_cast<const double*>(B);
-    const bool okA = reinterpret_cast<uintptr_t>(Ad) % 16 == 0;
-    const bool okB = reinterpret_cast<uintptr_t>(Bd) % 16 == 0;
-    if ((!(which & 1) || okA) && (!(which & 2) || okB)) {
-      const int64_t planeA = int64_t(L.rowsA) * L.kp, planeB = int64_t(L.nb) * L.kp;
-      if (which & 1)
-        launch_slice_tc(Ad, ldA, p.k, L.rowsA, L.kp, sigA, p.opA == 2 ? -1 : 1, resA,
-                        int64_t(L.nsub) * planeA, planeA, crt, L.nmod, status, st);
-      if (which & 2)
-        launch_slice_tc(Bd, ldB, p.k, L.rowsB, L.kp, sigB, 1, resB, int64_t(L.nsub) * planeB,
-                        planeB, crt, L.nmod, status, st);
-      return;
-    }
-  }
-  int ndig = 0;
-  const SliceConsts sc = slice_consts(L, crt, &ndig);
   const int vec_elems = 16 / int(sizeof(TIn));
   const bool vecA = (reinterpret_cast<uintptr_t>(A) % 16 == 0) && (ldA % vec_elems == 0);
   const bool vecB = (reinterpret_cast<uintptr_t>(B) % 16 == 0) && (ldB % vec_elems == 0);
-  // complex: three planes per modulus, A's third is re(a) - im(a) for A^H
-  // (conj(a) b: Im = r2 - r0 + r1) and re(a) + im(a) otherwise; B's is re + im
-  const int mode = cplx ? 2 : 0;
+  // complex, split moduli: A's planes take -j for A^H (conj(a) swaps u and v);
+  // three products: A's third plane is re(a) - im(a) for A^H (conj(a) b: Im =
+  // r2 - r0 + r1) and re(a) + im(a) otherwise, B's is re + im
+  const int mode = L.split ? 3 : cplx ? 2 : 0;
   const int sumA = p.opA == 2 ? -1 : 1;
+  int ndig = 0;
+  const SliceConsts scA = slice_consts(L, crt, sumA, &ndig);
+  const SliceConsts sc = slice_consts(L, crt, 1, &ndig);
   const int64_t strideA = int64_t(L.nsub) * L.rowsA * L.kp;
   const int64_t strideB = int64_t(L.nsub) * L.nb * L.kp;
   if ((which & 1) && L.mn)
     launch_slice_mn<TIn>(ndig, st, A, p.lda, L.rowsA, p.k, L.kp, sigA, mode, sumA, 0, resA,
-                         strideA, sc, t0, t1);
+                         strideA, scA, t0, t1);
   else if ((which & 1) && vecA)
     launch_slice<TIn, true>(ndig, st, A, ldA, L.K2, L.rowsA, L.kp, sigA, mode, sumA, resA,
-                            strideA, sc, t0, t1, ssqA);
+                            strideA, scA, t0, t1, ssqA);
   else if (which & 1)
     launch_slice<TIn, false>(ndig, st, A, ldA, L.K2, L.rowsA, L.kp, sigA, mode, sumA, resA,
-                             strideA, sc, t0, t1, ssqA);
+                             strideA, scA, t0, t1, ssqA);
   if ((which & 2) && L.mnB)  // op(B) = T or C: n-major rows, conjugated for C
     launch_slice_mn<TIn>(ndig, st, B, p.ldb, L.rowsB, p.k, L.kp, sigB, mode, 1,
                          p.opB == 2 ? 1 : 0, resB, strideB, sc, t0, t1);
@@ -2708,9 +2408,8 @@ int onepass_operands(const oz::Layout& L, const GemmProblem& p, int groups) {
   const char* v = std::getenv("SPLAB_OZAKI_ONEPASS");
   if (v && v[0] == '0') return 0;
   const int nu = dtype_is_double(p.dtype) ? oz::kDefaultModuli : oz::kDefaultModuliFloat;
-  if (!(p.k > 0 && groups == 1 && L.nmod == nu && slice_unroll() && !slice_tc_enabled() &&
-        L.K2 >= kOnePassMinLen))
-    return 0;
+  const bool unrolled = dtype_is_complex(p.dtype) ? L.split : L.nmod == nu;
+  if (!(p.k > 0 && groups == 1 && unrolled && slice_unroll() && L.K2 >= kOnePassMinLen)) return 0;
   return (L.mn ? 0 : 1) | (L.mnB ? 0 : 2);
 }
 
@@ -2738,7 +2437,7 @@ void launch_slice_rows_el(cudaStream_t st, const TIn* X, int64_t ld, int64_t len
                           int64_t kp, const int* sig, int s_sign, int8_t* res, int64_t stride,
                           const oz::SliceConsts& sc, const int* list, const int* count) {
   using namespace oz;
-  constexpr int kNU = sizeof(TIn) == 8 ? kDefaultModuli : kDefaultModuliFloat;
+  constexpr int kNU = unrolled_moduli<TIn, MODE>();
   constexpr int kDigU = sizeof(TIn) == 8 ? 4 : 3;
   const unsigned grid = unsigned((EL == 8 ? 4 : 2) * sm_count());  // one resident wave
   oz_slice_rows<TIn, VEC, kDigU, EL, kNU, MODE>
@@ -2747,9 +2446,11 @@ void launch_slice_rows_el(cudaStream_t st, const TIn* X, int64_t ld, int64_t len
 
 // The listed rows of one operand: exact exponent, then residues again
 template <typename TIn>
-void onepass_redo(const oz::Layout& L, const oz::Crt& crt, const oz::SliceConsts& sc,
-                  const TIn* X, int64_t ld, int rows, int* sig, int s_sign, int8_t* res,
-                  int64_t stride, int mode, const int* list, const int* count, cudaStream_t st) {
+void onepass_redo(const oz::Layout& L, const oz::Crt& crt, const TIn* X, int64_t ld, int rows,
+                  int* sig, int s_sign, int8_t* res, int64_t stride, const int* list,
+                  const int* count, cudaStream_t st) {
+  int ndig = 0;
+  const oz::SliceConsts sc = slice_consts(L, crt, s_sign, &ndig);
   oz::oz_row_scale<TIn><<<unsigned(std::min(rows, 2 * oz::sm_count())), 256, 0, st>>>(
       X, ld, L.K2, rows, crt.q_bits, sig, list, count);
   const bool vec = reinterpret_cast<uintptr_t>(X) % 16 == 0 && ld % (16 / int(sizeof(TIn))) == 0;
@@ -2763,14 +2464,14 @@ void onepass_redo(const oz::Layout& L, const oz::Crt& crt, const oz::SliceConsts
   using E8 = std::integral_constant<int, 8>;
   using E16 = std::integral_constant<int, 16>;
   using M0 = std::integral_constant<int, 0>;
-  using M2 = std::integral_constant<int, 2>;
+  using M3 = std::integral_constant<int, 3>;
   const bool e16 = slice_elems() == 16;
   if (vec) {
-    if (e16) mode == 2 ? run(T{}, E16{}, M2{}) : run(T{}, E16{}, M0{});
-    else mode == 2 ? run(T{}, E8{}, M2{}) : run(T{}, E8{}, M0{});
+    if (e16) L.split ? run(T{}, E16{}, M3{}) : run(T{}, E16{}, M0{});
+    else L.split ? run(T{}, E8{}, M3{}) : run(T{}, E8{}, M0{});
   } else {
-    if (e16) mode == 2 ? run(F{}, E16{}, M2{}) : run(F{}, E16{}, M0{});
-    else mode == 2 ? run(F{}, E8{}, M2{}) : run(F{}, E8{}, M0{});
+    if (e16) L.split ? run(F{}, E16{}, M3{}) : run(F{}, E16{}, M0{});
+    else L.split ? run(F{}, E8{}, M3{}) : run(F{}, E8{}, M0{});
   }
 }
 
@@ -2799,17 +2500,13 @@ void onepass_fixup(const oz::Layout& L, const oz::Crt& crt, const GemmProblem& p
   if (which & 2)
     oz_onepass_check<<<unsigned((L.rowsB + 255) / 256), 256, 0, st>>>(
         ssq + L.rowsA, exactB, L.rowsB, lo, hi, listB, cnt + 1);
-  int ndig = 0;
-  const SliceConsts sc = slice_consts(L, crt, &ndig);
-  const int mode = cplx ? 2 : 0;
   const int64_t ldA = cplx ? 2 * p.lda : p.lda, ldB = cplx ? 2 * p.ldb : p.ldb;
   if (which & 1)
-    onepass_redo<TIn>(L, crt, sc, static_cast<const TIn*>(p.A), ldA, L.rowsA, sigA,
-                      p.opA == 2 ? -1 : 1, resA, int64_t(L.nsub) * L.rowsA * L.kp, mode, listA,
-                      cnt, st);
+    onepass_redo<TIn>(L, crt, static_cast<const TIn*>(p.A), ldA, L.rowsA, sigA,
+                      p.opA == 2 ? -1 : 1, resA, int64_t(L.nsub) * L.rowsA * L.kp, listA, cnt, st);
   if (which & 2)
-    onepass_redo<TIn>(L, crt, sc, static_cast<const TIn*>(p.B), ldB, L.rowsB, sigB, 1, resB,
-                      int64_t(L.nsub) * L.nb * L.kp, mode, listB, cnt + 1, st);
+    onepass_redo<TIn>(L, crt, static_cast<const TIn*>(p.B), ldB, L.rowsB, sigB, 1, resB,
+                      int64_t(L.nsub) * L.nb * L.kp, listB, cnt + 1, st);
 }
 
 // Side streams may be used by this host thread (off while a batch captures
@@ -2916,14 +2613,17 @@ cudaError_t launch_recon_tc(const GemmProblem& p, const oz::Layout& L, const oz:
   P.tile_n = cplx ? BN / 2 : BN;
   P.rp = rp;
   // weight bytes: plane k = t * nsub + s takes W_t or P - W_t (the combination
-  // of combine3 with its signs carried by the weights)
+  // of combine_split or combine3 with its signs carried by the weights)
   const unsigned __int128 Pm = (unsigned __int128)crt.P_hi << 64 | crt.P_lo;
   for (int t = 0; t < L.nmod; ++t) {
     const unsigned __int128 W = (unsigned __int128)crt.w_hi[t] << 64 | crt.w_lo[t];
     const unsigned __int128 Wn = Pm - W;
     for (int s = 0; s < L.nsub; ++s) {
       unsigned __int128 vre = W, vim = 0;
-      if (cplx) {
+      if (L.split) {
+        vim = (unsigned __int128)crt.wi_hi[t] << 64 | crt.wi_lo[t];
+        if (s == 1) vim = Pm - vim;
+      } else if (cplx) {
         if (s == 0) {
           vre = W;
           vim = Wn;
@@ -2987,7 +2687,7 @@ cudaError_t ozaki_gemm(const GemmProblem& p_in, int moduli, void* ws, size_t ws_
   if (p_in.m <= 0 || p_in.n <= 0) return cudaSuccess;
   const Layout L = layout_of(p_in, moduli);
   if (ws_bytes < L.total || !ws) return cudaErrorInvalidValue;
-  const Crt crt = make_crt(L.nmod);
+  const Crt crt = crt_of(L);
   const bool cplx = dtype_is_complex(p_in.dtype);
   char* w = static_cast<char*>(ws);
   int* sigA = reinterpret_cast<int*>(w + L.off_sigA);
@@ -3305,7 +3005,8 @@ cudaError_t ozaki_gemm(const GemmProblem& p_in, int moduli, void* ws, size_t ws_
   const bool staged = R8 && L.rowsA % 16 == 0;
   const unsigned gy = unsigned(std::min<int64_t>(p.n, 65535));
   const unsigned gx = unsigned(std::max<int64_t>(1, (p.m + threads - 1) / threads));
-  const bool fixed = L.nmod == (dtype_is_double(p.dtype) ? kDefaultModuli : kDefaultModuliFloat);
+  const bool fixed =
+      cplx ? L.split : L.nmod == (dbl ? kDefaultModuli : kDefaultModuliFloat);
   if (tc_recon) {
     if ((e = launch_recon_tc(p, L, crt, rp, rmap, sigA, sigB, status, st)) != cudaSuccess)
       return e;
@@ -3313,7 +3014,7 @@ cudaError_t ozaki_gemm(const GemmProblem& p_in, int moduli, void* ws, size_t ws_
     return cudaGetLastError();
   }
   if (staged) {
-    const int smem = staged_smem_bytes(cplx, L.nmod);
+    const int smem = staged_smem_bytes(L.nmod * L.nsub);
     const int64_t items = (p.m + kStageRows - 1) / kStageRows * p.n;
     const unsigned grid = unsigned(std::min<int64_t>(items, int64_t(2) * sm_count()));
     auto run = [&](auto kern) -> cudaError_t {
@@ -3327,11 +3028,11 @@ cudaError_t ozaki_gemm(const GemmProblem& p_in, int moduli, void* ws, size_t ws_
     };
     switch (p.dtype) {
       case kC64:
-        e = fixed ? run(oz_reconstruct_staged<kC64, kDefaultModuli>)
+        e = fixed ? run(oz_reconstruct_staged<kC64, kSplitCount>)
                   : run(oz_reconstruct_staged<kC64, 0>);
         break;
       case kC32:
-        e = fixed ? run(oz_reconstruct_staged<kC32, kDefaultModuliFloat>)
+        e = fixed ? run(oz_reconstruct_staged<kC32, kSplitCountFloat>)
                   : run(oz_reconstruct_staged<kC32, 0>);
         break;
       case kR64:
@@ -3354,17 +3055,16 @@ cudaError_t ozaki_gemm(const GemmProblem& p_in, int moduli, void* ws, size_t ws_
                                            cplx ? BN / 2 : BN, rp);
   };
   using u8 = unsigned char;
-  // the default modulus counts (15 double, 9 float) run a fully unrolled
-  // reconstruction
+  // the default modulus counts run a fully unrolled reconstruction
   auto by_dtype = [&](auto rt_tag, const auto* Rsrc) {
     using RT = decltype(rt_tag);
     switch (p.dtype) {
       case kC64:
-        fixed ? recon(oz_reconstruct<kC64, RT, kDefaultModuli>, Rsrc)
+        fixed ? recon(oz_reconstruct<kC64, RT, kSplitCount>, Rsrc)
               : recon(oz_reconstruct<kC64, RT, 0>, Rsrc);
         break;
       case kC32:
-        fixed ? recon(oz_reconstruct<kC32, RT, kDefaultModuliFloat>, Rsrc)
+        fixed ? recon(oz_reconstruct<kC32, RT, kSplitCountFloat>, Rsrc)
               : recon(oz_reconstruct<kC32, RT, 0>, Rsrc);
         break;
       case kR64:

@@ -21,6 +21,19 @@ inline constexpr int kModuli[kMaxModuli] = {256, 255, 253, 251, 247, 241, 239, 2
 inline constexpr int kDefaultModuli = 15;       // double: Q = 57
 inline constexpr int kDefaultModuliFloat = 9;   // float: Q = 34
 
+// Split moduli (complex products): pairwise coprime, every prime factor
+// = 1 (mod 4) (221 = 13*17, 205 = 5*41, the rest prime), so that -1 has a
+// square root j modulo each: z = x + iy -> (u, v) = (x + jy, x - jy) mod p maps
+// a complex product to two independent real ones (u_a u_b, v_a v_b; conj(z)
+// swaps u and v), where integers mod a general p need three (Karatsuba). They
+// are smaller on average, so one more of them covers the same range: 16 (2 x 16
+// real products) give the Q = 57 of the 15 (3 x 15) moduli above, 10 (2 x 10)
+// give Q = 37 where 9 (3 x 9) give 34.
+inline constexpr int kSplitCount = 16;       // double
+inline constexpr int kSplitCountFloat = 10;  // float
+inline constexpr int kSplitModuli[kSplitCount] = {241, 233, 229, 221, 205, 197, 193, 181,
+                                                  173, 157, 149, 137, 113, 109, 101, 97};
+
 struct Crt {
   int n;
   int p[kMaxModuli];
@@ -29,24 +42,42 @@ struct Crt {
   unsigned long long P_lo, P_hi;
   double P_d;
   int q_bits;  // Q: scaled rows have 2-norm < 2^Q
+  // split moduli: j with j^2 = -1 (mod p), and the weights of Re = (u + v) / 2
+  // (w above, times 1/2 mod p) and of Im = (u - v) / (2j) (wi)
+  int j[kMaxModuli];
+  unsigned long long wi_lo[kMaxModuli], wi_hi[kMaxModuli];
 };
 
 // --------------------------------------------------------------------------
 // host: CRT constants
 
-inline Crt make_crt(int n) {
+inline int inverse_mod(int a, int p) {  // a, p coprime, p <= 256
+  int y = 1;
+  while ((a * y) % p != 1) ++y;
+  return y;
+}
+
+inline Crt make_crt_of(const int* moduli, int n, bool split) {
   Crt c{};
   c.n = n;
   unsigned __int128 P = 1;
-  for (int t = 0; t < n; ++t) P *= (unsigned __int128)kModuli[t];
+  for (int t = 0; t < n; ++t) P *= (unsigned __int128)moduli[t];
   for (int t = 0; t < n; ++t) {
-    const int p = kModuli[t];
+    const int p = moduli[t];
     c.p[t] = p;
     c.inv_p[t] = 1.0 / double(p);
     const unsigned __int128 Mt = P / (unsigned __int128)p;
-    const int mt_mod = int(Mt % (unsigned __int128)p);
-    int y = 1;
-    while ((mt_mod * y) % p != 1) ++y;  // modular inverse, p <= 256
+    int y = inverse_mod(int(Mt % (unsigned __int128)p), p);
+    if (split) {
+      int j = 1;
+      while ((j * j + 1) % p != 0) ++j;
+      c.j[t] = j;
+      const int yi = (y * inverse_mod((2 * j) % p, p)) % p;
+      y = (y * inverse_mod(2, p)) % p;
+      const unsigned __int128 Wi = Mt * (unsigned __int128)yi;
+      c.wi_lo[t] = (unsigned long long)Wi;
+      c.wi_hi[t] = (unsigned long long)(Wi >> 64);
+    }
     const unsigned __int128 W = Mt * (unsigned __int128)y;  // < P since y < p
     c.w_lo[t] = (unsigned long long)W;
     c.w_hi[t] = (unsigned long long)(W >> 64);
@@ -59,6 +90,9 @@ inline Crt make_crt(int n) {
   c.q_bits = int(std::floor((lp - 2.0) / 2.0));
   return c;
 }
+
+inline Crt make_crt(int n) { return make_crt_of(kModuli, n, false); }
+inline Crt make_crt_split(int n) { return make_crt_of(kSplitModuli, n, true); }
 
 // v mod p in [0, p) for any int32 v and 2 <= p <= 256 without a division:
 // v = hi * 2^16 + lo, t = hi * (2^16 mod p) + lo = v (mod p) with |t| < 2^24,
@@ -97,6 +131,7 @@ struct ReconParams {
   int p[kMaxModuli];
   int off24[kMaxModuli];      // p * ceil(2^24 / p): a multiple of p above any int32 residue sum
   unsigned w[kMaxModuli][4];  // CRT weights W_t < P as 32-bit limbs, least significant first
+  unsigned wi[kMaxModuli][4];  // split moduli: the weights of Im
   unsigned P[4];              // P as 32-bit limbs
   double inv_P32;             // 2^32 / P
   int conj;                   // complex products: A^H B (1) or A^T B / A B (0)
@@ -119,17 +154,27 @@ __host__ __device__ __forceinline__ void combine3(int r0, int r1, int r2, int of
   }
 }
 
+// The same from the two products of a split modulus: Re and Im (before their
+// weights) as u + v and u - v, non-negative and below 2 off.
+__host__ __device__ __forceinline__ void combine_split(int u, int v, int off, int& re, int& im) {
+  re = u + v;
+  im = u + (off - v);
+}
+
 inline ReconParams make_recon(const Crt& c) {
   ReconParams rp{};
+  auto limbs = [](unsigned (&w)[4], unsigned long long lo, unsigned long long hi) {
+    w[0] = unsigned(lo);
+    w[1] = unsigned(lo >> 32);
+    w[2] = unsigned(hi);
+    w[3] = unsigned(hi >> 32);
+  };
   rp.n = c.n;
   for (int t = 0; t < c.n; ++t) {
     rp.p[t] = c.p[t];
     rp.off24[t] = c.p[t] * (((1 << 24) + c.p[t] - 1) / c.p[t]);
-    const unsigned long long lo = c.w_lo[t], hi = c.w_hi[t];
-    rp.w[t][0] = unsigned(lo);
-    rp.w[t][1] = unsigned(lo >> 32);
-    rp.w[t][2] = unsigned(hi);
-    rp.w[t][3] = unsigned(hi >> 32);
+    limbs(rp.w[t], c.w_lo[t], c.w_hi[t]);
+    limbs(rp.wi[t], c.wi_lo[t], c.wi_hi[t]);
   }
   rp.P[0] = unsigned(c.P_lo);
   rp.P[1] = unsigned(c.P_lo >> 32);
@@ -225,17 +270,19 @@ __host__ __device__ __forceinline__ double crt_from_limbs(unsigned long long l0,
   return fma(v, 4294967296.0, u32_to_double(x0));
 }
 
-template <int N, bool BYTES>
+// IM: the weights of Im of the split moduli.
+template <int N, bool BYTES, bool IM = false>
 __host__ __device__ __forceinline__ double crt_value(const int* r, const ReconParams& rp) {
   unsigned long long l0 = 0, l1 = 0, l2 = 0, l3 = 0;
 #pragma unroll
   for (int t = 0; t < (N > 0 ? N : kMaxUsableModuli); ++t) {
     if (N == 0 && t >= rp.n) break;
     const unsigned rt = unsigned(r[t]);
-    l0 += (unsigned long long)rt * rp.w[t][0];
-    l1 += (unsigned long long)rt * rp.w[t][1];
-    l2 += (unsigned long long)rt * rp.w[t][2];
-    l3 += (unsigned long long)rt * rp.w[t][3];
+    const unsigned* w = IM ? rp.wi[t] : rp.w[t];
+    l0 += (unsigned long long)rt * w[0];
+    l1 += (unsigned long long)rt * w[1];
+    l2 += (unsigned long long)rt * w[2];
+    l3 += (unsigned long long)rt * w[3];
   }
   return crt_from_limbs<BYTES>(l0, l1, l2, l3, rp);
 }
