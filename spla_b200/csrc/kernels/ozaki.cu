@@ -37,7 +37,8 @@
 // 2-norm, 2^-Q) and the final conversion of X to double.
 //
 // Kernels: oz_row_scale (row norms -> sigma), oz_slice (scaled residues,
-// int8, K-major, one plane per modulus and product), oz_row_scale_mn /
+// int8, K-major, one plane per modulus and product), oz_slice_mma (the same for
+// complex double: ozaki_slice.cuh), oz_row_scale_mn /
 // oz_slice_mn (the same for op(A) = N and op(B) = T, C read in place),
 // oz_transpose (op(A) = N copied K-major when k is too long for that),
 // oz_gemm_pair / oz_gemm
@@ -60,6 +61,8 @@
 #include "common.cuh"
 #include "ozaki.cuh"
 #include "ozaki_crt.cuh"
+#include "ozaki_layout.cuh"
+#include "ozaki_slice.cuh"
 #include "tcgen05_common.cuh"
 
 namespace splab {
@@ -367,47 +370,6 @@ __device__ __forceinline__ void digits13(double y, float (&d)[5]) {
 
 constexpr float kMagic = 12582912.0f;  // 1.5 * 2^23: ulp 1, low mantissa bits hold r
 
-// Two floats in one 64-bit register for the packed FP32 instructions of
-// sm_100 (fma/add .f32x2: one instruction, two lanes of work).
-__host__ __device__ __forceinline__ unsigned long long f2_pack(float lo, float hi) {
-#ifdef __CUDA_ARCH__
-  unsigned long long r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-  return r;
-#else
-  uint32_t a, b;
-  std::memcpy(&a, &lo, 4);
-  std::memcpy(&b, &hi, 4);
-  return (static_cast<unsigned long long>(b) << 32) | a;
-#endif
-}
-__device__ __forceinline__ void f2_unpack(unsigned long long v, float& lo, float& hi) {
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
-}
-__device__ __forceinline__ unsigned long long f2_fma(unsigned long long a, unsigned long long b,
-                                                     unsigned long long c) {
-  unsigned long long d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-  return d;
-}
-__device__ __forceinline__ unsigned long long f2_mul(unsigned long long a, unsigned long long b) {
-  unsigned long long d;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-__device__ __forceinline__ unsigned long long f2_add(unsigned long long a, unsigned long long b) {
-  unsigned long long d;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-
-__device__ __forceinline__ uint32_t pack4(float a, float b, float c, float d) {
-  const uint32_t t0 = __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x0040);
-  const uint32_t t1 = __byte_perm(__float_as_uint(c), __float_as_uint(d), 0x0040);
-  return __byte_perm(t0, t1, 0x5410);
-}
-
-
 // The work of one slicing thread once its EL reals (of one row, starting at
 // real l0) are loaded: scaling by 2^sg, digits, and for every modulus the
 // residues written to res_row + l0 (mode 0) or, in modes 2 and 3, to the three
@@ -422,7 +384,7 @@ template <typename TIn, int NDIG, int EL, int NMU, int MODE, bool SSQ = false,
 __device__ __forceinline__ void slice_thread(double (&v)[EL], int sg, int8_t* res_row,
                                              int64_t l0, int64_t plane, int s_sum,
                                              int64_t res_mod_stride, const SliceConsts& sc,
-                                             int t_begin, int t_end, OnSsq on_ssq = {}) {
+                                             OnSsq on_ssq = {}) {
   static_assert(EL == 8 || EL == 16, "8 or 16 reals per thread");
   static_assert(MODE == 0 || MODE == 2 || MODE == 3, "real rows, or complex rows in two forms");
   constexpr int W = EL / 4;  // packed words per modulus
@@ -584,7 +546,7 @@ __device__ __forceinline__ void slice_thread(double (&v)[EL], int sg, int8_t* re
 #pragma unroll
     for (int t = 0; t < NMU; ++t) modulus(t);
   } else {
-    for (int t = t_begin; t < t_end; ++t) modulus(t);
+    for (int t = 0; t < sc.n; ++t) modulus(t);
   }
 }
 
@@ -600,8 +562,8 @@ __device__ __forceinline__ void slice_thread(double (&v)[EL], int sg, int8_t* re
 // mode 3: complex rows with split moduli: res[t][0][row][e] = r(re + j im),
 //         res[t][1][row][e] = -r(re - j im).
 // TIn: double (|x| < 2^62, five digits) or float (|x| < 2^38, three digits).
-// NMU > 0: moduli 0 .. NMU-1 in one fully unrolled pass (the per-modulus
-// constants become fixed parameter operands); 0: t_begin .. t_end-1 in a loop.
+// NMU > 0: the moduli in one fully unrolled pass (the per-modulus constants
+// become fixed parameter operands); 0: sc.n moduli in a loop.
 // MODE (the mode above) is a template parameter so that the unrolled
 // modulus loop carries no branch on it.
 // The EL reals of one row at real l0 (zeros past len); VEC: 16-byte loads.
@@ -632,13 +594,22 @@ __device__ __forceinline__ void load_reals(const TIn* __restrict__ x, int64_t l0
   }
 }
 
+// Where slice_thread's row starts, for a thread at real l0 of it: pieces of
+// kc elements (split moduli) lie G kc apart.
+template <int MODE>
+__device__ __forceinline__ int8_t* row_base(int8_t* res, const ResidueLayout& lay, int row,
+                                            int64_t l0) {
+  int8_t* r = res + int64_t(row) * lay.row;
+  return MODE == 3 ? r + (lay.at(l0 / 2) - l0 / 2) : r;
+}
+
 // SSQ: also adds each row's sum of squares of the scaled values to
 // rowssq[row] (one atomic per row and block; blocks of 256 threads).
 template <typename TIn, bool VEC, int NDIG, int EL, int NMU, int MODE, bool SSQ = false>
 __global__ void __launch_bounds__(256, EL == 8 ? 4 : 2)
     oz_slice(const TIn* __restrict__ X, int64_t ld_doubles, int64_t len, int rows, int64_t kp,
              const int* __restrict__ sigma, int s_sum, int8_t* __restrict__ res,
-             int64_t res_mod_stride, SliceConsts sc, int t_begin, int t_end,
+             ResidueLayout lay, int64_t res_mod_stride, SliceConsts sc,
              double* __restrict__ rowssq) {
   const int64_t groups = (MODE != 0 ? 2 * kp : kp) / EL;
   const int64_t gid = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
@@ -648,9 +619,8 @@ __global__ void __launch_bounds__(256, EL == 8 ? 4 : 2)
     const int64_t l0 = (gid % groups) * EL;
     double v[EL];
     load_reals<TIn, VEC, EL>(X + int64_t(row) * ld_doubles + l0, l0, len, v);
-    slice_thread<TIn, NDIG, EL, NMU, MODE>(v, sigma[row], res + int64_t(row) * kp, l0,
-                                           int64_t(rows) * kp, s_sum, res_mod_stride, sc, t_begin,
-                                           t_end);
+    slice_thread<TIn, NDIG, EL, NMU, MODE>(v, sigma[row], row_base<MODE>(res, lay, row, l0), l0,
+                                           lay.plane(1), s_sum, res_mod_stride, sc);
   } else {
     // Threads past the last row redo the last row's last groups (the same
     // bytes to the same places) so that every thread takes part in the
@@ -680,9 +650,9 @@ __global__ void __launch_bounds__(256, EL == 8 ? 4 : 2)
         seg_row[threadIdx.x / W] = past ? -1 : row;
       }
     };
-    slice_thread<TIn, NDIG, EL, NMU, MODE, true>(v, sigma[row], res + int64_t(row) * kp, l0,
-                                                 int64_t(rows) * kp, s_sum, res_mod_stride, sc,
-                                                 t_begin, t_end, on_ssq);
+    slice_thread<TIn, NDIG, EL, NMU, MODE, true>(v, sigma[row], row_base<MODE>(res, lay, row, l0),
+                                                 l0, lay.plane(1), s_sum, res_mod_stride, sc,
+                                                 on_ssq);
     __syncthreads();
     if (int(threadIdx.x) < nseg) {
       const int sgi = threadIdx.x, r = seg_row[sgi];
@@ -701,8 +671,8 @@ template <typename TIn, bool VEC, int NDIG, int EL, int NMU, int MODE>
 __global__ void __launch_bounds__(256, EL == 8 ? 4 : 2)
     oz_slice_rows(const TIn* __restrict__ X, int64_t ld_doubles, int64_t len, int rows,
                   int64_t kp, const int* __restrict__ sigma, int s_sum,
-                  int8_t* __restrict__ res, int64_t res_mod_stride, SliceConsts sc,
-                  const int* __restrict__ list, const int* __restrict__ count) {
+                  int8_t* __restrict__ res, ResidueLayout lay, int64_t res_mod_stride,
+                  SliceConsts sc, const int* __restrict__ list, const int* __restrict__ count) {
   const int64_t groups = (MODE != 0 ? 2 * kp : kp) / EL;
   const int64_t total = int64_t(*count) * groups;
   for (int64_t gid = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; gid < total;
@@ -711,8 +681,8 @@ __global__ void __launch_bounds__(256, EL == 8 ? 4 : 2)
     const int64_t l0 = (gid % groups) * EL;
     double v[EL];
     load_reals<TIn, VEC, EL>(X + int64_t(row) * ld_doubles + l0, l0, len, v);
-    slice_thread<TIn, NDIG, EL, NMU, MODE>(v, sigma[row], res + int64_t(row) * kp, l0,
-                                           int64_t(rows) * kp, s_sum, res_mod_stride, sc, 0, NMU);
+    slice_thread<TIn, NDIG, EL, NMU, MODE>(v, sigma[row], row_base<MODE>(res, lay, row, l0), l0,
+                                           lay.plane(1), s_sum, res_mod_stride, sc);
   }
 }
 
@@ -844,7 +814,7 @@ template <typename TIn, bool VEC, int NDIG, int NMU, int MODE>
 __global__ void __launch_bounds__(256, 4)
     oz_slice_mn(const TIn* __restrict__ X, int64_t ld, int m, int64_t k, int64_t kp,
                 const int* __restrict__ sigma, int s_sum, int conj, int8_t* __restrict__ res,
-                int64_t res_mod_stride, SliceConsts sc, int t_begin, int t_end) {
+                ResidueLayout lay, int64_t res_mod_stride, SliceConsts sc) {
   constexpr int EL = 8;
   constexpr int R = MODE != 0 ? 2 : 1;  // reals per element
   constexpr int G = EL / R;             // elements per thread
@@ -907,9 +877,9 @@ __global__ void __launch_bounds__(256, 4)
       v[q] = double(__uint_as_float(e));
     }
   }
-  slice_thread<TIn, NDIG, EL, NMU, MODE>(v, sigma[row], res + int64_t(row) * kp,
-                                         (kk0 + G * l) * R, int64_t(m) * kp, s_sum,
-                                         res_mod_stride, sc, t_begin, t_end);
+  const int64_t l0 = (kk0 + G * l) * R;
+  slice_thread<TIn, NDIG, EL, NMU, MODE>(v, sigma[row], row_base<MODE>(res, lay, row, l0), l0,
+                                         lay.plane(1), s_sum, res_mod_stride, sc);
 }
 
 // --------------------------------------------------------------------------
@@ -921,11 +891,12 @@ struct GemmParams {
   int kblocks;       // kp / 128
   int nchunks;       // ceil(kblocks / kChunkBlocks)
   int chunk_blocks;  // k-blocks per chunk: ceil(kblocks / nchunks) <= kChunkBlocks
+  int group;         // planes per group, and k-blocks per piece of a plane's row
+  int kc_blocks;     // (ResidueLayout: G, kc / 128)
   int nmod;          // products: moduli x nsub (the A/B/R planes in order)
   int nsub;          // products per modulus (Layout::nsub): modulus = product / nsub
-  int t0;            // first product of this launch (units cover t0 ..)
   int tiles_m, tiles_n;
-  int total_units;   // moduli of the launch * nchunks * tiles
+  int total_units;   // products * nchunks * tiles
   int* R;            // accumulated residues [nmod][nb][m] (int32), or
   unsigned char* R8; // with a single k-chunk: the residues as bytes (no accumulation)
   int* status;       // set to 1 when a bounded wait gave up
@@ -967,7 +938,7 @@ __device__ __forceinline__ Unit decode_unit(int u, const GemmParams& g) {
   const int rest = u / tiles;
   band_tile(tile, g.tiles_m, g.tiles_n, r.tm, r.tn);
   r.c = rest % g.nchunks;
-  r.t = g.t0 + rest / g.nchunks;
+  r.t = rest / g.nchunks;
   return r;
 }
 
@@ -1023,8 +994,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
       const Unit w = decode_unit(u, g);
       const int kb0 = w.c * g.chunk_blocks;
       const int kb1 = min(g.kblocks, kb0 + g.chunk_blocks);
-      const int arow = w.t * g.m + w.tm * BM;
-      const int brow = w.t * g.nb + w.tn * BN;
+      const int tg = w.t / g.group, tq = w.t - tg * g.group;  // the plane's group, place in it
+      int kc = kb0 / g.kc_blocks, kx = kb0 - kc * g.kc_blocks;  // piece, block in it
       for (int kb = kb0; kb < kb1; ++kb) {
         if (!mbar_wait(empty_bar(stage), phase ^ 1u, abort, g.wait_limit_ns)) {
           ok = false;
@@ -1032,8 +1003,12 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
         }
         mbar_arrive_expect_tx(full_bar(stage), STAGE_BYTES);
         const uint32_t sa = base + stage * STAGE_BYTES;
-        tma_load_2d(sa, &tmA, kb * BKB, arow, full_bar(stage));
-        tma_load_2d(sa + A_STAGE, &tmB, kb * BKB, brow, full_bar(stage));
+        tma_load_5d(sa, &tmA, kx * BKB, tq, kc, w.tm * BM, tg, full_bar(stage));
+        tma_load_5d(sa + A_STAGE, &tmB, kx * BKB, tq, kc, w.tn * BN, tg, full_bar(stage));
+        if (++kx == g.kc_blocks) {
+          kx = 0;
+          ++kc;
+        }
         if (++stage == STAGES) {
           stage = 0;
           phase ^= 1u;
@@ -1256,7 +1231,7 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1)
       band_tile(tl, g.tiles_m, g.tiles_n, tm, tn);
     }
     c = rest % g.nchunks;
-    t = g.t0 + rest / g.nchunks;
+    t = rest / g.nchunks;
   };
 
   bool aborted = false;
@@ -1269,8 +1244,10 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1)
       int t, c, tm, tn;
       unit_of(u, t, c, tm, tn);
       const int kb0 = c * g.chunk_blocks, kb1 = min(g.kblocks, kb0 + g.chunk_blocks);
-      const int arow = t * g.m + tm * 256 + int(rank) * 128;
-      const int brow = t * g.nb + tn * (256 * NT) + int(rank) * 128;
+      const int arow = tm * 256 + int(rank) * 128;
+      const int brow = tn * (256 * NT) + int(rank) * 128;
+      const int tg = t / g.group, tq = t - tg * g.group;  // the plane's group, place in it
+      int kc = kb0 / g.kc_blocks, kx = kb0 - kc * g.kc_blocks;  // piece, block in it
       for (int kb = kb0; kb < kb1; ++kb) {
         if (!mbar_wait(empty_bar(stage), phase ^ 1u, abort, g.wait_limit_ns)) {
           ok = false;
@@ -1279,10 +1256,15 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1)
         const uint32_t fb = map_to_rank(full_bar(stage), 0);
         if (rank == 0) mbar_arrive_expect_tx(full_bar(stage), 2 * STAGE2_BYTES);
         const uint32_t sa = base + stage * STAGE2_BYTES;
-        tma_load_2d_pair(sa, &tmA, kb * BKB, arow, fb);
+        tma_load_5d_pair(sa, &tmA, kx * BKB, tq, kc, arow, tg, fb);
 #pragma unroll
         for (int h = 0; h < NT; ++h)
-          tma_load_2d_pair(sa + A_STAGE2 + h * B_HALF2, &tmB, kb * BKB, brow + h * 256, fb);
+          tma_load_5d_pair(sa + A_STAGE2 + h * B_HALF2, &tmB, kx * BKB, tq, kc, brow + h * 256, tg,
+                           fb);
+        if (++kx == g.kc_blocks) {
+          kx = 0;
+          ++kc;
+        }
         if (++stage == STAGES2) {
           stage = 0;
           phase ^= 1u;
@@ -1973,6 +1955,7 @@ __global__ void __launch_bounds__(RT_THREADS, 3)
 struct Layout {
   int nmod;
   bool split;              // complex with the split moduli
+  bool pairs;              // the two planes of a split modulus lie side by side in pieces
   int nsub;                // products per modulus: 1 (real), 2 (split) or 3 (Karatsuba)
   int64_t K2, kp;          // reals per operand row; residue row length (k padded to 128)
   int rowsA, rowsB, nb;    // A rows, B rows, B residue rows per product
@@ -1992,6 +1975,21 @@ struct Layout {
 size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 
 Crt crt_of(const Layout& L) { return L.split ? make_crt_split(L.nmod) : make_crt(L.nmod); }
+
+// Complex double planes with the split moduli come in pairs: the 32 planes of a
+// row are written at once, and as many streams far apart cost the slicer (see
+// oz_slice_mma: 1.43 ms with planes apart, 1.16 in pairs), while the GEMM, which
+// reads one plane of many rows, slows down once a row's pieces of all planes
+// span many pages (m = n = 1024, k = 250000: 6.2 ms apart or in pairs, 6.9 in
+// groups of 4, 9.7 of 8). Pieces of 1 KB, or less for rows so short that the
+// padding of the last piece could outgrow the workspace of the three-product form
+// (45 planes to these 32: up to 3/8 more).
+ResidueLayout residue_layout(const Layout& L, int rows) {
+  if (!L.pairs) return {rows * L.kp, L.kp, L.kp, 62, 1};
+  const int shift = L.kp < 256 ? 7 : L.kp < 2304 ? 8 : 10;
+  const int64_t kc = int64_t(1) << shift, row = (L.kp + kc - 1) / kc * 2 * kc;
+  return {rows * row, row, kc, shift, 2};
+}
 
 // In-place reading of an m-major operand: the transposing slicer's tiles of
 // 128 (complex) or 256 (real) elements along k must fit the grid's y extent.
@@ -2020,6 +2018,7 @@ Layout layout_of(const GemmProblem& p, int moduli) {
   L.split = cplx && count == def;
   L.nmod = L.split ? (dbl ? kSplitCount : kSplitCountFloat) : count;
   L.nsub = L.split ? 2 : cplx ? 3 : 1;
+  L.pairs = L.split && dbl;
   // The workspace keeps the size of the three-product form for callers that
   // hold one sized for it (32 planes of the split form lie in the room of 45)
   const size_t planes = size_t(count) * (cplx ? 3 : 1);
@@ -2080,14 +2079,21 @@ PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
   return fn;
 }
 
-bool make_map(CUtensorMap* map, void* base, int64_t kp, int64_t rows, int box_rows) {
+// Residues of an operand: dims (bytes of a piece, planes of a group, pieces, rows,
+// groups), boxes of one k-block of one plane x box_rows rows (rows past the end
+// read as zeros).
+bool make_map(CUtensorMap* map, void* base, const Layout& L, int rows, int box_rows) {
   auto fn = encode_fn();
   if (!fn) return false;
-  cuuint64_t dims[2] = {cuuint64_t(kp), cuuint64_t(rows)};
-  cuuint64_t strides[1] = {cuuint64_t(kp)};
-  cuuint32_t box[2] = {cuuint32_t(BKB), cuuint32_t(box_rows)};
-  cuuint32_t estr[2] = {1, 1};
-  const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, base, dims, strides, box, estr,
+  const ResidueLayout lay = residue_layout(L, rows);
+  const int64_t pieces = lay.row / (lay.G * lay.kc);
+  cuuint64_t dims[5] = {cuuint64_t(lay.kc), cuuint64_t(lay.G), cuuint64_t(pieces),
+                        cuuint64_t(rows), cuuint64_t(L.nmod * L.nsub / lay.G)};
+  cuuint64_t strides[4] = {cuuint64_t(lay.kc), cuuint64_t(lay.G * lay.kc), cuuint64_t(lay.row),
+                           cuuint64_t(lay.group)};
+  cuuint32_t box[5] = {cuuint32_t(BKB), 1u, 1u, cuuint32_t(box_rows), 1u};
+  cuuint32_t estr[5] = {1, 1, 1, 1, 1};
+  const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 5, base, dims, strides, box, estr,
                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                         CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS;
@@ -2165,43 +2171,45 @@ bool slice_unroll() {
 template <typename TIn, bool VEC, int EL, int MODE>
 void launch_slice_el(int ndig, unsigned grid, cudaStream_t st, const TIn* X, int64_t ld,
                      int64_t len, int rows, int64_t kp, const int* sig, int s_sign, int8_t* res,
-                     int64_t stride, const oz::SliceConsts& sc, int t0, int t1, double* ssq) {
+                     const oz::ResidueLayout& lay, int64_t stride, const oz::SliceConsts& sc,
+                     double* ssq) {
   using namespace oz;
   constexpr int kNU = unrolled_moduli<TIn, MODE>();
   constexpr int kDigU = sizeof(TIn) == 8 ? 4 : 3;  // digits of the default scaling
   if constexpr (kNU > 0) {
-    if (t0 == 0 && t1 == kNU && sc.n == kNU && ndig == kDigU && slice_unroll()) {
+    if (sc.n == kNU && ndig == kDigU && slice_unroll()) {
       if (ssq)
         oz_slice<TIn, VEC, kDigU, EL, kNU, MODE, true><<<grid, 256, 0, st>>>(
-            X, ld, len, rows, kp, sig, s_sign, res, stride, sc, t0, t1, ssq);
+            X, ld, len, rows, kp, sig, s_sign, res, lay, stride, sc, ssq);
       else
         oz_slice<TIn, VEC, kDigU, EL, kNU, MODE><<<grid, 256, 0, st>>>(
-            X, ld, len, rows, kp, sig, s_sign, res, stride, sc, t0, t1, nullptr);
+            X, ld, len, rows, kp, sig, s_sign, res, lay, stride, sc, nullptr);
       return;
     }
   }
   if (ndig <= 3)
     oz_slice<TIn, VEC, 3, EL, 0, MODE><<<grid, 256, 0, st>>>(
-        X, ld, len, rows, kp, sig, s_sign, res, stride, sc, t0, t1, nullptr);
+        X, ld, len, rows, kp, sig, s_sign, res, lay, stride, sc, nullptr);
   else if (ndig == 4)
     oz_slice<TIn, VEC, 4, EL, 0, MODE><<<grid, 256, 0, st>>>(
-        X, ld, len, rows, kp, sig, s_sign, res, stride, sc, t0, t1, nullptr);
+        X, ld, len, rows, kp, sig, s_sign, res, lay, stride, sc, nullptr);
   else
     oz_slice<TIn, VEC, 5, EL, 0, MODE><<<grid, 256, 0, st>>>(
-        X, ld, len, rows, kp, sig, s_sign, res, stride, sc, t0, t1, nullptr);
+        X, ld, len, rows, kp, sig, s_sign, res, lay, stride, sc, nullptr);
 }
 
 // ssq (unrolled default scaling only): also the rows' scaled sums of squares
 template <typename TIn, bool VEC>
 void launch_slice(int ndig, cudaStream_t st, const TIn* X, int64_t ld, int64_t len, int rows,
-                  int64_t kp, const int* sig, int mode, int s_sign, int8_t* res, int64_t stride,
-                  const oz::SliceConsts& sc, int t0, int t1, double* ssq = nullptr) {
+                  int64_t kp, const int* sig, int mode, int s_sign, int8_t* res,
+                  const oz::ResidueLayout& lay, int64_t stride, const oz::SliceConsts& sc,
+                  double* ssq) {
   const int el = slice_elems();
   const int64_t kreal = mode != 0 ? 2 * kp : kp;  // reals per row a thread group covers
   const unsigned grid = unsigned((int64_t(rows) * (kreal / el) + 255) / 256);
   auto run = [&](auto el_tag, auto mode_tag) {
     launch_slice_el<TIn, VEC, decltype(el_tag)::value, decltype(mode_tag)::value>(
-        ndig, grid, st, X, ld, len, rows, kp, sig, s_sign, res, stride, sc, t0, t1, ssq);
+        ndig, grid, st, X, ld, len, rows, kp, sig, s_sign, res, lay, stride, sc, ssq);
   };
   using E8 = std::integral_constant<int, 8>;
   using E16 = std::integral_constant<int, 16>;
@@ -2209,8 +2217,10 @@ void launch_slice(int ndig, cudaStream_t st, const TIn* X, int64_t ld, int64_t l
   using M2 = std::integral_constant<int, 2>;
   using M3 = std::integral_constant<int, 3>;
   auto by_mode = [&](auto el_tag) {
-    if (mode == 3) run(el_tag, M3{});
-    else if (mode == 2) run(el_tag, M2{});
+    if constexpr (sizeof(TIn) == 4) {  // double: oz_slice_mma
+      if (mode == 3) return run(el_tag, M3{});
+    }
+    if (mode == 2) run(el_tag, M2{});
     else run(el_tag, M0{});
   };
   if (el == 16) by_mode(E16{});
@@ -2221,37 +2231,37 @@ void launch_slice(int ndig, cudaStream_t st, const TIn* X, int64_t ld, int64_t l
 template <typename TIn, bool VEC, int MODE>
 void launch_slice_mn_v(int ndig, dim3 grid, cudaStream_t st, const TIn* X, int64_t ld, int m,
                        int64_t k, int64_t kp, const int* sig, int s_sign, int conj, int8_t* res,
-                       int64_t stride, const oz::SliceConsts& sc, int t0, int t1) {
+                       const oz::ResidueLayout& lay, int64_t stride, const oz::SliceConsts& sc) {
   using namespace oz;
   constexpr int kNU = unrolled_moduli<TIn, MODE>();
   constexpr int kDigU = sizeof(TIn) == 8 ? 4 : 3;
   if constexpr (kNU > 0) {
-    if (t0 == 0 && t1 == kNU && sc.n == kNU && ndig == kDigU && slice_unroll()) {
+    if (sc.n == kNU && ndig == kDigU && slice_unroll()) {
       oz_slice_mn<TIn, VEC, kDigU, kNU, MODE>
-          <<<grid, 256, 0, st>>>(X, ld, m, k, kp, sig, s_sign, conj, res, stride, sc, t0, t1);
+          <<<grid, 256, 0, st>>>(X, ld, m, k, kp, sig, s_sign, conj, res, lay, stride, sc);
       return;
     }
   }
   if (ndig <= 3)
     oz_slice_mn<TIn, VEC, 3, 0, MODE>
-        <<<grid, 256, 0, st>>>(X, ld, m, k, kp, sig, s_sign, conj, res, stride, sc, t0, t1);
+        <<<grid, 256, 0, st>>>(X, ld, m, k, kp, sig, s_sign, conj, res, lay, stride, sc);
   else if (ndig == 4)
     oz_slice_mn<TIn, VEC, 4, 0, MODE>
-        <<<grid, 256, 0, st>>>(X, ld, m, k, kp, sig, s_sign, conj, res, stride, sc, t0, t1);
+        <<<grid, 256, 0, st>>>(X, ld, m, k, kp, sig, s_sign, conj, res, lay, stride, sc);
   else
     oz_slice_mn<TIn, VEC, 5, 0, MODE>
-        <<<grid, 256, 0, st>>>(X, ld, m, k, kp, sig, s_sign, conj, res, stride, sc, t0, t1);
+        <<<grid, 256, 0, st>>>(X, ld, m, k, kp, sig, s_sign, conj, res, lay, stride, sc);
 }
 
 template <typename TIn>
 void launch_slice_mn(int ndig, cudaStream_t st, const TIn* X, int64_t ld, int m, int64_t k,
                      int64_t kp, const int* sig, int mode, int s_sign, int conj, int8_t* res,
-                     int64_t stride, const oz::SliceConsts& sc, int t0, int t1) {
+                     const oz::ResidueLayout& lay, int64_t stride, const oz::SliceConsts& sc) {
   const int64_t kt = mode != 0 ? 128 : 256;  // elements per row per tile
   const dim3 grid(unsigned((m + 7) / 8), unsigned((kp + kt - 1) / kt));
   auto run = [&](auto vec_tag, auto mode_tag) {
     launch_slice_mn_v<TIn, decltype(vec_tag)::value, decltype(mode_tag)::value>(
-        ndig, grid, st, X, ld, m, k, kp, sig, s_sign, conj, res, stride, sc, t0, t1);
+        ndig, grid, st, X, ld, m, k, kp, sig, s_sign, conj, res, lay, stride, sc);
   };
   using T = std::true_type;
   using F = std::false_type;
@@ -2336,12 +2346,49 @@ oz::SliceConsts slice_consts(const oz::Layout& L, const oz::Crt& crt, int s_sign
   return sc;
 }
 
-// Residues of moduli t0 .. t1-1 of A (which & 1) and B (which & 2).
+// Residues of k-major complex double rows for the split moduli (oz_slice_mma), with
+// the rows' scaled sums of squares when ssq is given, or of the listed rows only.
+void launch_slice_mma(const oz::Layout& L, const oz::Crt& crt, const double* X, int64_t ld,
+                      int rows, const int* sigma, int sign, int8_t* res, double* ssq,
+                      const int* list, const int* count, cudaStream_t st) {
+  using namespace oz;
+  SliceMmaParams P{};
+  P.X = X;
+  P.ld = ld;
+  P.len = L.K2;
+  P.rows = rows;
+  P.vec = reinterpret_cast<uintptr_t>(X) % 16 == 0 && ld % 2 == 0;
+  P.sigma = sigma;
+  P.res = res;
+  P.lay = residue_layout(L, rows);
+  P.ssq = ssq;
+  P.list = list;
+  P.count = count;
+  P.steps_per_row = int(2 * L.kp / kStepReals);
+  const int wpr = P.steps_per_row >= 4 ? 4 : 2;  // kp >= 128: at least two steps
+  P.warps_per_row = wpr;
+  // V's planes hold -v, as oz_slice's
+  for (int t = 0; t < kSplitCount; ++t) {
+    P.row[2 * t] = make_slice_row(crt.p[t], 1, sign * crt.j[t]);
+    P.row[2 * t + 1] = make_slice_row(crt.p[t], -1, sign * crt.j[t]);
+  }
+  const long long slots = (long long)kSliceBlocks * sm_count();
+  const long long steps = (long long)rows * P.steps_per_row;
+  P.run = int(std::max<long long>(1, std::min<long long>(16, steps / (4 * slots))));
+  const long long segs = (P.steps_per_row + P.run * wpr - 1) / (P.run * wpr);
+  const long long chunks = ((long long)rows * wpr + 3) / 4 * segs;
+  const unsigned grid = unsigned(std::min(slots, chunks));
+  if (ssq)
+    oz_slice_mma<true><<<grid, 128, 0, st>>>(P);
+  else
+    oz_slice_mma<false><<<grid, 128, 0, st>>>(P);
+}
+
+// Residues of A (which & 1) and B (which & 2).
 template <typename TIn>
 void slice_operands(const oz::Layout& L, const oz::Crt& crt, const GemmProblem& p, bool cplx,
-                    const int* sigA, const int* sigB, int8_t* resA, int8_t* resB, int t0, int t1,
-                    int which, cudaStream_t st, int* status, double* ssqA = nullptr,
-                    double* ssqB = nullptr) {
+                    const int* sigA, const int* sigB, int8_t* resA, int8_t* resB, int which,
+                    cudaStream_t st, double* ssqA, double* ssqB) {
   using namespace oz;
   const TIn* A = static_cast<const TIn*>(p.A);
   const TIn* B = static_cast<const TIn*>(p.B);
@@ -2358,26 +2405,38 @@ void slice_operands(const oz::Layout& L, const oz::Crt& crt, const GemmProblem& 
   int ndig = 0;
   const SliceConsts scA = slice_consts(L, crt, sumA, &ndig);
   const SliceConsts sc = slice_consts(L, crt, 1, &ndig);
-  const int64_t strideA = int64_t(L.nsub) * L.rowsA * L.kp;
-  const int64_t strideB = int64_t(L.nsub) * L.nb * L.kp;
+  const ResidueLayout layA = residue_layout(L, L.rowsA), layB = residue_layout(L, L.nb);
+  const int64_t strideA = layA.plane(L.nsub), strideB = layB.plane(L.nsub);
+  if constexpr (std::is_same<TIn, double>::value) {
+    if (L.pairs) {  // k-major complex double: oz_slice_mma
+      if ((which & 1) && !L.mn) {
+        launch_slice_mma(L, crt, A, ldA, L.rowsA, sigA, sumA, resA, ssqA, nullptr, nullptr, st);
+        which &= ~1;
+      }
+      if ((which & 2) && !L.mnB) {
+        launch_slice_mma(L, crt, B, ldB, L.rowsB, sigB, 1, resB, ssqB, nullptr, nullptr, st);
+        which &= ~2;
+      }
+    }
+  }
   if ((which & 1) && L.mn)
     launch_slice_mn<TIn>(ndig, st, A, p.lda, L.rowsA, p.k, L.kp, sigA, mode, sumA, 0, resA,
-                         strideA, scA, t0, t1);
+                         layA, strideA, scA);
   else if ((which & 1) && vecA)
     launch_slice<TIn, true>(ndig, st, A, ldA, L.K2, L.rowsA, L.kp, sigA, mode, sumA, resA,
-                            strideA, scA, t0, t1, ssqA);
+                            layA, strideA, scA, ssqA);
   else if (which & 1)
     launch_slice<TIn, false>(ndig, st, A, ldA, L.K2, L.rowsA, L.kp, sigA, mode, sumA, resA,
-                             strideA, scA, t0, t1, ssqA);
+                             layA, strideA, scA, ssqA);
   if ((which & 2) && L.mnB)  // op(B) = T or C: n-major rows, conjugated for C
     launch_slice_mn<TIn>(ndig, st, B, p.ldb, L.rowsB, p.k, L.kp, sigB, mode, 1,
-                         p.opB == 2 ? 1 : 0, resB, strideB, sc, t0, t1);
+                         p.opB == 2 ? 1 : 0, resB, layB, strideB, sc);
   else if ((which & 2) && vecB)
-    launch_slice<TIn, true>(ndig, st, B, ldB, L.K2, L.rowsB, L.kp, sigB, mode, 1, resB, strideB,
-                            sc, t0, t1, ssqB);
+    launch_slice<TIn, true>(ndig, st, B, ldB, L.K2, L.rowsB, L.kp, sigB, mode, 1, resB, layB, strideB,
+                            sc, ssqB);
   else if (which & 2)
-    launch_slice<TIn, false>(ndig, st, B, ldB, L.K2, L.rowsB, L.kp, sigB, mode, 1, resB, strideB,
-                             sc, t0, t1, ssqB);
+    launch_slice<TIn, false>(ndig, st, B, ldB, L.K2, L.rowsB, L.kp, sigB, mode, 1, resB, layB, strideB,
+                             sc, ssqB);
 }
 
 // One-pass row scaling. The two-pass order reads every row twice: once for
@@ -2396,20 +2455,19 @@ void slice_operands(const oz::Layout& L, const oz::Crt& crt, const GemmProblem& 
 // sliced again. Each row thus ends with the exponent and residues of the
 // two-pass order, whatever the order of the atomic sums. Used for each
 // k-major operand (an operand read in place keeps its norms) with the
-// default modulus count and unrolled slicer, one modulus group and rows of
-// at least kOnePassMinLen reals; SPLAB_OZAKI_ONEPASS=0 (read per call) keeps
+// default modulus count and unrolled slicer and rows of at least kOnePassMinLen reals; SPLAB_OZAKI_ONEPASS=0 (read per call) keeps
 // the two-pass order.
 constexpr int64_t kOnePassMinLen = 131072;
 constexpr int kOnePassRuns = 16;
 
 // The operands scaled in one pass: bit 1 A, bit 2 B (k-major ones only; the
 // rows read in place keep their k-sliced norms)
-int onepass_operands(const oz::Layout& L, const GemmProblem& p, int groups) {
+int onepass_operands(const oz::Layout& L, const GemmProblem& p) {
   const char* v = std::getenv("SPLAB_OZAKI_ONEPASS");
   if (v && v[0] == '0') return 0;
   const int nu = dtype_is_double(p.dtype) ? oz::kDefaultModuli : oz::kDefaultModuliFloat;
   const bool unrolled = dtype_is_complex(p.dtype) ? L.split : L.nmod == nu;
-  if (!(p.k > 0 && groups == 1 && unrolled && slice_unroll() && L.K2 >= kOnePassMinLen)) return 0;
+  if (!(p.k > 0 && unrolled && slice_unroll() && L.K2 >= kOnePassMinLen)) return 0;
   return (L.mn ? 0 : 1) | (L.mnB ? 0 : 2);
 }
 
@@ -2434,30 +2492,39 @@ void onepass_estimate(const oz::Layout& L, const oz::Crt& crt, const GemmProblem
 
 template <typename TIn, bool VEC, int EL, int MODE>
 void launch_slice_rows_el(cudaStream_t st, const TIn* X, int64_t ld, int64_t len, int rows,
-                          int64_t kp, const int* sig, int s_sign, int8_t* res, int64_t stride,
-                          const oz::SliceConsts& sc, const int* list, const int* count) {
+                          int64_t kp, const int* sig, int s_sign, int8_t* res,
+                          const oz::ResidueLayout& lay, int64_t stride, const oz::SliceConsts& sc,
+                          const int* list, const int* count) {
   using namespace oz;
   constexpr int kNU = unrolled_moduli<TIn, MODE>();
   constexpr int kDigU = sizeof(TIn) == 8 ? 4 : 3;
   const unsigned grid = unsigned((EL == 8 ? 4 : 2) * sm_count());  // one resident wave
   oz_slice_rows<TIn, VEC, kDigU, EL, kNU, MODE>
-      <<<grid, 256, 0, st>>>(X, ld, len, rows, kp, sig, s_sign, res, stride, sc, list, count);
+      <<<grid, 256, 0, st>>>(X, ld, len, rows, kp, sig, s_sign, res, lay, stride, sc, list, count);
 }
 
 // The listed rows of one operand: exact exponent, then residues again
 template <typename TIn>
 void onepass_redo(const oz::Layout& L, const oz::Crt& crt, const TIn* X, int64_t ld, int rows,
-                  int* sig, int s_sign, int8_t* res, int64_t stride, const int* list,
-                  const int* count, cudaStream_t st) {
-  int ndig = 0;
-  const oz::SliceConsts sc = slice_consts(L, crt, s_sign, &ndig);
+                  int* sig, int s_sign, int8_t* res, const int* list, const int* count,
+                  cudaStream_t st) {
   oz::oz_row_scale<TIn><<<unsigned(std::min(rows, 2 * oz::sm_count())), 256, 0, st>>>(
       X, ld, L.K2, rows, crt.q_bits, sig, list, count);
+  if constexpr (std::is_same<TIn, double>::value) {
+    if (L.pairs) {
+      launch_slice_mma(L, crt, X, ld, rows, sig, s_sign, res, nullptr, list, count, st);
+      return;
+    }
+  }
+  int ndig = 0;
+  const oz::SliceConsts sc = slice_consts(L, crt, s_sign, &ndig);
+  const oz::ResidueLayout lay = residue_layout(L, rows);
+  const int64_t stride = lay.plane(L.nsub);
   const bool vec = reinterpret_cast<uintptr_t>(X) % 16 == 0 && ld % (16 / int(sizeof(TIn))) == 0;
   auto run = [&](auto vec_tag, auto el_tag, auto mode_tag) {
     launch_slice_rows_el<TIn, decltype(vec_tag)::value, decltype(el_tag)::value,
                          decltype(mode_tag)::value>(st, X, ld, L.K2, rows, L.kp, sig, s_sign,
-                                                    res, stride, sc, list, count);
+                                                    res, lay, stride, sc, list, count);
   };
   using T = std::true_type;
   using F = std::false_type;
@@ -2466,12 +2533,18 @@ void onepass_redo(const oz::Layout& L, const oz::Crt& crt, const TIn* X, int64_t
   using M0 = std::integral_constant<int, 0>;
   using M3 = std::integral_constant<int, 3>;
   const bool e16 = slice_elems() == 16;
+  auto by_mode = [&](auto vec_tag, auto el_tag) {
+    if constexpr (sizeof(TIn) == 4) {
+      if (L.split) return run(vec_tag, el_tag, M3{});
+    }
+    run(vec_tag, el_tag, M0{});
+  };
   if (vec) {
-    if (e16) L.split ? run(T{}, E16{}, M3{}) : run(T{}, E16{}, M0{});
-    else L.split ? run(T{}, E8{}, M3{}) : run(T{}, E8{}, M0{});
+    if (e16) by_mode(T{}, E16{});
+    else by_mode(T{}, E8{});
   } else {
-    if (e16) L.split ? run(F{}, E16{}, M3{}) : run(F{}, E16{}, M0{});
-    else L.split ? run(F{}, E8{}, M3{}) : run(F{}, E8{}, M0{});
+    if (e16) by_mode(F{}, E16{});
+    else by_mode(F{}, E8{});
   }
 }
 
@@ -2503,24 +2576,21 @@ void onepass_fixup(const oz::Layout& L, const oz::Crt& crt, const GemmProblem& p
   const int64_t ldA = cplx ? 2 * p.lda : p.lda, ldB = cplx ? 2 * p.ldb : p.ldb;
   if (which & 1)
     onepass_redo<TIn>(L, crt, static_cast<const TIn*>(p.A), ldA, L.rowsA, sigA,
-                      p.opA == 2 ? -1 : 1, resA, int64_t(L.nsub) * L.rowsA * L.kp, listA, cnt, st);
+                      p.opA == 2 ? -1 : 1, resA, listA, cnt, st);
   if (which & 2)
     onepass_redo<TIn>(L, crt, static_cast<const TIn*>(p.B), ldB, L.rowsB, sigB, 1, resB,
-                      int64_t(L.nsub) * L.nb * L.kp, listB, cnt + 1, st);
+                      listB, cnt + 1, st);
 }
 
 // Side streams may be used by this host thread (off while a batch captures
 // its sequence of contractions into a CUDA graph on one stream).
 thread_local bool t_side_streams = true;
 
-// Side streams of the modulus-group pipeline (per device): residues of group
-// g + 1 are produced on `lo` while the GEMM of group g runs on `hi` (highest
-// priority, so that its persistent CTAs are placed first and the slicing
-// blocks fill the registers and issue slots the GEMM leaves free).
+// Side stream (per device): the row norms of B, a pure read, run there beside
+// the slicing of A (arithmetic-bound) when both are large.
 struct PipeStreams {
-  cudaStream_t hi = nullptr, lo = nullptr;
-  cudaEvent_t ev_start = nullptr, ev_done = nullptr, ev_scaled = nullptr,
-              ev_sliced[oz::kMaxModuli] = {};
+  cudaStream_t lo = nullptr;
+  cudaEvent_t ev_start = nullptr, ev_scaled = nullptr;
   std::mutex mu;  // one enqueue sequence at a time
   bool ok = false;
 };
@@ -2536,17 +2606,10 @@ PipeStreams* pipe_streams() {
   static std::mutex init_mu;
   std::lock_guard<std::mutex> lk(init_mu);
   if (!ps.ok) {
-    int lo_prio = 0, hi_prio = 0;
-    bool good = cudaDeviceGetStreamPriorityRange(&lo_prio, &hi_prio) == cudaSuccess &&
-                cudaStreamCreateWithPriority(&ps.hi, cudaStreamNonBlocking, hi_prio) ==
-                    cudaSuccess &&
-                cudaStreamCreateWithPriority(&ps.lo, cudaStreamNonBlocking, lo_prio) ==
-                    cudaSuccess &&
-                cudaEventCreateWithFlags(&ps.ev_start, cudaEventDisableTiming) == cudaSuccess &&
-                cudaEventCreateWithFlags(&ps.ev_done, cudaEventDisableTiming) == cudaSuccess &&
-                cudaEventCreateWithFlags(&ps.ev_scaled, cudaEventDisableTiming) == cudaSuccess;
-    for (int g = 0; good && g < oz::kMaxModuli; ++g)
-      good = cudaEventCreateWithFlags(&ps.ev_sliced[g], cudaEventDisableTiming) == cudaSuccess;
+    const bool good =
+        cudaStreamCreateWithFlags(&ps.lo, cudaStreamNonBlocking) == cudaSuccess &&
+        cudaEventCreateWithFlags(&ps.ev_start, cudaEventDisableTiming) == cudaSuccess &&
+        cudaEventCreateWithFlags(&ps.ev_scaled, cudaEventDisableTiming) == cudaSuccess;
     if (!good) {
       cudaGetLastError();
       return nullptr;
@@ -2556,18 +2619,6 @@ PipeStreams* pipe_streams() {
   return &ps;
 }
 
-// Number of modulus groups. Default 1: overlapping the slicing of one group
-// with the GEMM of the previous one measured slower on B200 (both phases
-// draw on L2 bandwidth; the slicing ran at half speed beside the GEMM).
-// SPLAB_OZAKI_GROUPS = 2 .. number of moduli enables the pipeline.
-int modulus_groups(const oz::Layout& L) {
-  int g = 1;
-  if (const char* v = std::getenv("SPLAB_OZAKI_GROUPS")) {
-    const int f = std::atoi(v);
-    if (f > 0) g = f;
-  }
-  return std::max(1, std::min(g, L.nmod));
-}
 }  // namespace
 
 namespace {
@@ -2710,23 +2761,19 @@ cudaError_t ozaki_gemm(const GemmProblem& p_in, int moduli, void* ws, size_t ws_
     p.opA = 1;
   }
   const bool dbl = dtype_is_double(p.dtype);
-  const int groups = modulus_groups(L);
-  // Large problems use the side streams: the row norms of B (a pure read)
-  // run beside the slicing of A (arithmetic-bound), and with groups > 1 the
-  // modulus-group pipeline below.
+  // Large problems use the side stream: the row norms of B run beside the slicing
+  // of A.
   const bool big = double(L.rowsA + L.rowsB) * double(L.K2) * dtype_bytes(p.dtype) /
                        (cplx ? 2.0 : 1.0) >= 5e8;
   static const bool side_norms = [] {
     const char* v = std::getenv("SPLAB_OZAKI_SIDE_NORMS");
     return !(v && v[0] == '0');
   }();
-  const int onepass = onepass_operands(L, p, groups);
+  const int onepass = onepass_operands(L, p);
   double* ssq = reinterpret_cast<double*>(w + L.off_ssq);
   int* oplist = reinterpret_cast<int*>(w + L.off_list);
   PipeStreams* ps =
-      (p.k > 0 && (groups > 1 || (big && side_norms)) && t_side_streams)
-          ? pipe_streams()
-          : nullptr;
+      p.k > 0 && big && side_norms && t_side_streams ? pipe_streams() : nullptr;
   std::unique_lock<std::mutex> lk;
   if (ps) lk = std::unique_lock<std::mutex>(ps->mu);
   auto scale = [&](int which, cudaStream_t s) {
@@ -2797,17 +2844,14 @@ cudaError_t ozaki_gemm(const GemmProblem& p_in, int moduli, void* ws, size_t ws_
     // with one-pass scaling the slicer also sums the rows' scaled squares
     double* ssqA = (onepass & 1) ? ssq : nullptr;
     double* ssqB = (onepass & 2) ? ssq + L.rowsA : nullptr;
-    auto slice = [&](int t0, int t1, int which, cudaStream_t s) {
+    auto slice = [&](int which) {
       if (dbl)
-        slice_operands<double>(L, crt, p, cplx, sigA, sigB, resA, resB, t0, t1, which, s,
-                               status, ssqA, ssqB);
+        slice_operands<double>(L, crt, p, cplx, sigA, sigB, resA, resB, which, st, ssqA, ssqB);
       else
-        slice_operands<float>(L, crt, p, cplx, sigA, sigB, resA, resB, t0, t1, which, s,
-                              status, ssqA, ssqB);
+        slice_operands<float>(L, crt, p, cplx, sigA, sigB, resA, resB, which, st, ssqA, ssqB);
     };
     CUtensorMap mapA, mapB;
-    if (!make_map(&mapA, resA, L.kp, int64_t(L.nmod) * L.nsub * L.rowsA, BM) ||
-        !make_map(&mapB, resB, L.kp, int64_t(L.nmod) * L.nsub * L.nb, BN))
+    if (!make_map(&mapA, resA, L, L.rowsA, BM) || !make_map(&mapB, resB, L, L.nb, BN))
       return cudaErrorNotSupported;
     GemmParams g{};
     g.m = L.rowsA;
@@ -2816,6 +2860,8 @@ cudaError_t ozaki_gemm(const GemmProblem& p_in, int moduli, void* ws, size_t ws_
     g.nchunks = (g.kblocks + kChunkBlocks - 1) / kChunkBlocks;
     // equal chunks (each within the exact INT32 bound): equal work units
     g.chunk_blocks = std::max(1, (g.kblocks + g.nchunks - 1) / std::max(1, g.nchunks));
+    g.group = residue_layout(L, 1).G;
+    g.kc_blocks = int(residue_layout(L, 1).kc / BKB);
     g.nmod = L.nmod * L.nsub;
     g.nsub = L.nsub;
     g.tiles_m = (L.rowsA + BM - 1) / BM;
@@ -2907,23 +2953,17 @@ cudaError_t ozaki_gemm(const GemmProblem& p_in, int moduli, void* ws, size_t ws_
           (e = set_dynamic_smem(reinterpret_cast<const void*>(oz_gemm_pair<2>),
                                 PairCfg<2>::SMEM)) != cudaSuccess)
         return e;
-      if (!make_map(&mapA2, resA, L.kp, int64_t(L.nmod) * L.nsub * L.rowsA, 128) ||
-          !make_map(&mapB2, resB, L.kp, int64_t(L.nmod) * L.nsub * L.nb, 128))
+      if (!make_map(&mapA2, resA, L, L.rowsA, 128) || !make_map(&mapB2, resB, L, L.nb, 128))
         return cudaErrorNotSupported;
     }
-    const int units_per_mod = g.total_units / L.nmod;  // all products of one modulus
-    // the INT8 GEMM over moduli t0 .. t1-1 on stream s
-    auto launch_gemm = [&](int t0, int t1, cudaStream_t s) -> cudaError_t {
-      GemmParams gg = g;
-      gg.t0 = t0 * L.nsub;
-      gg.total_units = (t1 - t0) * units_per_mod;
+    auto launch_gemm = [&]() -> cudaError_t {
       if (pair) {
-        const int pairs = std::max(1, std::min(gg.total_units, sm_count() / 2));
+        const int pairs = std::max(1, std::min(g.total_units, sm_count() / 2));
         cudaLaunchConfig_t cfg{};
         cfg.gridDim = dim3(unsigned(2 * pairs));
         cfg.blockDim = dim3(PAIR_THREADS);
         cfg.dynamicSmemBytes = nt == 2 ? PairCfg<2>::SMEM : PairCfg<1>::SMEM;
-        cfg.stream = s;
+        cfg.stream = st;
         cudaLaunchAttribute at[1];
         at[0].id = cudaLaunchAttributeClusterDimension;
         at[0].val.clusterDim.x = 2;
@@ -2931,66 +2971,41 @@ cudaError_t ozaki_gemm(const GemmProblem& p_in, int moduli, void* ws, size_t ws_
         at[0].val.clusterDim.z = 1;
         cfg.attrs = at;
         cfg.numAttrs = 1;
-        return nt == 2 ? cudaLaunchKernelEx(&cfg, oz_gemm_pair<2>, mapA2, mapB2, gg)
-                       : cudaLaunchKernelEx(&cfg, oz_gemm_pair<1>, mapA2, mapB2, gg);
+        return nt == 2 ? cudaLaunchKernelEx(&cfg, oz_gemm_pair<2>, mapA2, mapB2, g)
+                       : cudaLaunchKernelEx(&cfg, oz_gemm_pair<1>, mapA2, mapB2, g);
       }
       const cudaError_t ea = set_dynamic_smem(reinterpret_cast<const void*>(oz_gemm), GEMM_SMEM);
       if (ea != cudaSuccess) return ea;
-      const int grid = std::min(gg.total_units, sm_count());
-      oz_gemm<<<grid, GEMM_THREADS, GEMM_SMEM, s>>>(mapA, mapB, gg);
+      const int grid = std::min(g.total_units, sm_count());
+      oz_gemm<<<grid, GEMM_THREADS, GEMM_SMEM, st>>>(mapA, mapB, g);
       return cudaGetLastError();
     };
 
-    if (groups == 1 || !ps) {
-      phase_mark(17, false, st);
-      slice(0, L.nmod, 1, st);  // A on the caller's stream
-      phase_mark(17, true, st);
-      // B once its row norms are done (on the side stream when there is one)
-      if (side_exponents && (e = cudaStreamWaitEvent(st, ps->ev_scaled, 0)) != cudaSuccess)
-        return e;
-      phase_mark(18, false, st);
-      slice(0, L.nmod, 2, st);
-      phase_mark(18, true, st);
-      if (onepass) {
-        phase_mark(19, false, st);
-        if (dbl)
-          onepass_fixup<double>(L, crt, p, cplx, sigA, sigB, resA, resB, ssq, oplist, onepass,
-                                st);
-        else
-          onepass_fixup<float>(L, crt, p, cplx, sigA, sigB, resA, resB, ssq, oplist, onepass,
-                               st);
-        phase_mark(19, true, st);
-      }
-      phase_mark(0, true, st);
-      phase_mark(1, false, st);
-      phase_mark(3, false, st);
-      if ((e = launch_gemm(0, L.nmod, st)) != cudaSuccess) return e;
-      phase_mark(3, true, st);
-      phase_mark(1, true, st);
-    } else {
-      // modulus-group pipeline: slicing of group i + 1 (stream lo) overlaps
-      // the GEMM of group i (stream hi); the caller's stream joins at the end
-      auto bounds = [&](int i) { return i * L.nmod / groups; };
-      // lo has the B row norms queued; it also needs A's row norms and the
-      // memsets of the caller's stream
-      if ((e = cudaEventRecord(ps->ev_start, st)) != cudaSuccess) return e;
-      if ((e = cudaStreamWaitEvent(ps->lo, ps->ev_start, 0)) != cudaSuccess) return e;
-      for (int i = 0; i < groups; ++i) {
-        slice(bounds(i), bounds(i + 1), 3, ps->lo);
-        if ((e = cudaEventRecord(ps->ev_sliced[i], ps->lo)) != cudaSuccess) return e;
-      }
-      phase_mark(0, true, ps->lo);
-      for (int i = 0; i < groups; ++i) {
-        if ((e = cudaStreamWaitEvent(ps->hi, ps->ev_sliced[i], 0)) != cudaSuccess) return e;
-        if (i == 0) phase_mark(1, false, ps->hi);
-        phase_mark(3 + i, false, ps->hi);
-        if ((e = launch_gemm(bounds(i), bounds(i + 1), ps->hi)) != cudaSuccess) return e;
-        phase_mark(3 + i, true, ps->hi);
-      }
-      phase_mark(1, true, ps->hi);
-      if ((e = cudaEventRecord(ps->ev_done, ps->hi)) != cudaSuccess) return e;
-      if ((e = cudaStreamWaitEvent(st, ps->ev_done, 0)) != cudaSuccess) return e;
+    phase_mark(17, false, st);
+    slice(1);
+    phase_mark(17, true, st);
+    // B once its row norms are done (on the side stream when there is one)
+    if (side_exponents && (e = cudaStreamWaitEvent(st, ps->ev_scaled, 0)) != cudaSuccess)
+      return e;
+    phase_mark(18, false, st);
+    slice(2);
+    phase_mark(18, true, st);
+    if (onepass) {
+      phase_mark(19, false, st);
+      if (dbl)
+        onepass_fixup<double>(L, crt, p, cplx, sigA, sigB, resA, resB, ssq, oplist, onepass,
+                              st);
+      else
+        onepass_fixup<float>(L, crt, p, cplx, sigA, sigB, resA, resB, ssq, oplist, onepass,
+                             st);
+      phase_mark(19, true, st);
     }
+    phase_mark(0, true, st);
+    phase_mark(1, false, st);
+    phase_mark(3, false, st);
+    if ((e = launch_gemm()) != cudaSuccess) return e;
+    phase_mark(3, true, st);
+    phase_mark(1, true, st);
   }
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
 

@@ -2,6 +2,7 @@
 modulus): the CRT side (tests/cpp/test_crt_split.cu) and the slicer's residue
 step on the CPU, and the whole path on the GPU at the edges of its tiles."""
 import re
+import shutil
 import subprocess
 
 import numpy as np
@@ -11,14 +12,16 @@ from test_ozaki_crt import HERE
 from test_ozaki_slice_arith import HDR, _centred, _quotient
 
 
-def test_crt_of_split_moduli(tmp_path):
-    import shutil
-    nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
-    if shutil.which(nvcc) is None:
+@pytest.mark.parametrize("source", ["test_crt_split.cu", "test_slice_rows.cu"])
+def test_split_arithmetic_on_the_cpu(tmp_path, source):
+    """The reconstruction's weights (test_crt_split.cu) and the slicer's digit
+    weights and reduction (test_slice_rows.cu), compiled for the host."""
+    nvcc = shutil.which("nvcc") or shutil.which("/usr/local/cuda/bin/nvcc")
+    if nvcc is None:
         pytest.skip("nvcc not available")
-    exe = tmp_path / "test_crt_split"
-    subprocess.run([nvcc, "-std=c++17", "-O2", "-o", str(exe),
-                    str(HERE / "cpp" / "test_crt_split.cu")], check=True, capture_output=True)
+    exe = tmp_path / "check"
+    subprocess.run([nvcc, "-gencode", "arch=compute_100a,code=sm_100a", "-std=c++17", "-O2", "-o",
+                    str(exe), str(HERE / "cpp" / source)], check=True, capture_output=True)
     out = subprocess.run([str(exe)], capture_output=True, text=True)
     assert out.returncode == 0 and out.stdout.startswith("OK"), out.stdout + out.stderr
 
