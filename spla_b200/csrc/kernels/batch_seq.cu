@@ -101,19 +101,16 @@ cudaError_t seq_batch_run(SeqBatch* b, void* ws, cudaStream_t st) {
     if (b->graph) cudaGraphDestroy(b->graph);
     b->exec = nullptr;
     b->graph = nullptr;
-    // no side streams and no phase events inside the captured sequence
+    // no phase events inside the captured sequence
     PhaseEvents saved = phase_events();
     phase_events() = PhaseEvents{};
-    ozaki_allow_side_streams(false);
     if ((e = cudaStreamBeginCapture(b->own, cudaStreamCaptureModeThreadLocal)) != cudaSuccess) {
-      ozaki_allow_side_streams(true);
       phase_events() = saved;
       return e;
     }
     const cudaError_t e1 = enqueue(*b, w, b->own);
     cudaGraph_t g = nullptr;
     e = cudaStreamEndCapture(b->own, &g);
-    ozaki_allow_side_streams(true);
     phase_events() = saved;
     if (e1 != cudaSuccess) {
       if (g) cudaGraphDestroy(g);

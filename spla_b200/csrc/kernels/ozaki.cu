@@ -112,7 +112,7 @@ __device__ __forceinline__ void umma_i8(uint32_t tmem_d, uint64_t adesc, uint64_
 // --------------------------------------------------------------------------
 // 1. row scale exponents
 
-// One block per row: sigma = Q - e where ||row||_2 = f 2^e, f in [0.5, 1).
+// sigma = Q - e (+ 1) for a row with ||row||_2 = f 2^e, f in [0.5, 1) (see Crt::thr).
 // Rows of zeros get sigma = 0, rows holding a NaN or an infinity get
 // kSigmaNonFinite (the reconstruction then writes NaN where they contribute).
 // The sum of squares is kept as S 2^(2E) with E the largest exponent seen
@@ -229,44 +229,101 @@ __device__ __forceinline__ void block_ssq(double& S, int& E, double* redS, int* 
   }
 }
 
+// Bits and threshold of the scale exponents (Crt::q_bits, Crt::thr)
+struct ScaleBits {
+  int q;
+  double thr;
+};
+
+// sigma from the exponent-tracked sum of squares S 2^(2E) of a row
+__device__ __forceinline__ int sigma_of(double S, int E, ScaleBits b) {
+  if (!(S < 1e300)) return kSigmaNonFinite;  // NaN or infinite input
+  if (S > 0.0) {
+    int e0 = 0;
+    const double f = frexp(sqrt(S), &e0);
+    return b.q - (e0 + E) + (f < b.thr ? 1 : 0);
+  }
+  return 0;
+}
+
 // Estimated norms whose mantissa (in [0.5, 1)) lies within this relative
-// distance of either end of its octave take the exact norm instead.
+// distance of where the exponents change take the exact norm instead.
 constexpr double kEstimateBand = 1.0 / 32;
 
-// One block per row (with a list, the blocks walk the rows list[0 .. *count
-// - 1], grid-stride; else block b takes row b); len reals per row.
-// With nruns > 0 the row's exponent is first estimated from a sample (nruns
-// runs of run reals, gap apart; the sum of squares extrapolated to len
-// reals) and kept when its norm's mantissa is clear of the octave's ends by
-// kEstimateBand (exact[row] = 0); otherwise, and for a zero or non-finite
-// sample, the whole row is read (exact[row] = 1) as without a sample.
-template <typename TIn>
-__global__ void oz_row_scale(const TIn* __restrict__ X, int64_t ld_elems, int64_t len, int rows,
-                             int q_bits, int* __restrict__ sigma,
-                             const int* __restrict__ list = nullptr,
-                             const int* __restrict__ count = nullptr, int nruns = 0,
-                             int64_t run = 0, int64_t gap = 0, int* __restrict__ exact = nullptr) {
+// Row scale exponents of up to two k-major operands (len reals per row; rows = 0:
+// none) in one launch.
+struct RowScaleOp {
+  const void* X;
+  int64_t ld;    // reals between rows
+  int rows;
+  int* sigma;
+  // one-pass scaling: whether the exponent is exact, the sums of squares of the
+  // scaled reals, the rows to slice again and their count
+  int* exact;
+  double* ssq;
+  int* list;
+  int* count;
+};
+struct RowScaleParams {
+  RowScaleOp op[2];
+  int64_t len;
+  ScaleBits bits;
+  int nruns;          // kEstimate: runs of `run` reals, `gap` apart
+  int64_t run, gap;
+  double lo, hi;      // kRecheck: range of ssq that proves an estimate
+  int* status;        // cleared by kExact and kEstimate
+};
+
+// kExact: one block per row, the exact exponent. kEstimate: the exponent from a
+// sample of the row (the sum of squares of nruns runs extrapolated to len reals)
+// when the estimated norm is clear of the exponents' change by kEstimateBand
+// (exact[row] = 0), else, and for a zero or non-finite sample, the exact one
+// (exact[row] = 1); clears the rows' sums of squares and the counts. kRecheck
+// (blocks grid-stride over the rows): a row whose exponent was estimated keeps
+// it when its sum of squares at that scale lies within [lo, hi] (the exponent is
+// then the exact one, and clear of the rounding of the sum); otherwise (the
+// estimate was off, the row is zero or not finite, or the sum lies near the
+// exponents' change) it gets its exact exponent and is listed for a second slicing.
+enum RowScaleMode { kExact, kEstimate, kRecheck };
+template <typename TIn, int MODE>
+__global__ void __launch_bounds__(256) oz_row_scale(const __grid_constant__ RowScaleParams P) {
   __shared__ double redS[32];
   __shared__ int redE[32];
   __shared__ int use_estimate;
-  const int nwork = list ? *count : min(rows, int(gridDim.x));
-  for (int bi = blockIdx.x; bi < nwork; bi += gridDim.x) {
-    const int row = list ? list[bi] : bi;
-    const TIn* x = X + int64_t(row) * ld_elems;
+  const int total = P.op[0].rows + P.op[1].rows;
+  if (MODE != kRecheck && blockIdx.x == 0 && threadIdx.x < 3) {
+    if (threadIdx.x == 2)
+      *P.status = 0;
+    else if (MODE == kEstimate && P.op[threadIdx.x].rows > 0)
+      *P.op[threadIdx.x].count = 0;
+  }
+  for (int bi = blockIdx.x; bi < total; bi += gridDim.x) {
+    const int which = bi < P.op[0].rows ? 0 : 1;
+    const RowScaleOp& op = P.op[which];
+    const int row = bi - (which ? P.op[0].rows : 0);
+    const TIn* x = static_cast<const TIn*>(op.X) + int64_t(row) * op.ld;
     double S = 0.0, inv = 0.0;  // sum of (v 2^-E)^2, and 2^-E
     int E = -2100;              // below any exponent: the first batch sets it
-    if (nruns > 0) {
-      ssq_sample(x, nruns, run, gap, S, E, inv);
+    if (MODE == kRecheck) {
+      const double s = op.ssq[row];
+      if (op.exact[row] || (s >= P.lo && s <= P.hi)) continue;  // block-uniform
+    }
+    if (MODE == kEstimate) {
+      ssq_sample(x, P.nruns, P.run, P.gap, S, E, inv);
       block_ssq(S, E, redS, redE);
       if (threadIdx.x == 0) {
         bool use = false;
         if (S > 0.0 && S < 1e300) {
           int e0 = 0;
-          const double f = frexp(sqrt(S * (double(len) / double(nruns * run))), &e0);
-          use = f > 0.5 * (1.0 + kEstimateBand) && f < 1.0 - kEstimateBand;
-          if (use) sigma[row] = q_bits - (e0 + E);
+          const double f =
+              frexp(sqrt(S * (double(P.len) / (double(P.nruns) * double(P.run)))), &e0);
+          // distance to thr, and to its neighbours one octave away
+          const double d = f < P.bits.thr ? f / P.bits.thr : f / (2.0 * P.bits.thr);
+          use = d > 0.5 * (1.0 + kEstimateBand) && d < 1.0 - kEstimateBand;
+          if (use) op.sigma[row] = P.bits.q - (e0 + E) + (f < P.bits.thr ? 1 : 0);
         }
-        exact[row] = use ? 0 : 1;
+        op.exact[row] = use ? 0 : 1;
+        op.ssq[row] = 0.0;
         use_estimate = use;
       }
       __syncthreads();
@@ -277,18 +334,11 @@ __global__ void oz_row_scale(const TIn* __restrict__ X, int64_t ld_elems, int64_
       if (done) continue;  // block-uniform; the next row's first barrier
                            // comes after this row's last read of use_estimate
     }
-    ssq_row(x, len, S, E, inv);
+    ssq_row(x, P.len, S, E, inv);
     block_ssq(S, E, redS, redE);
     if (threadIdx.x == 0) {
-      if (!(S < 1e300)) {  // NaN or infinite input
-        sigma[row] = kSigmaNonFinite;
-      } else if (S > 0.0) {
-        int e0 = 0;
-        frexp(sqrt(S), &e0);
-        sigma[row] = q_bits - (e0 + E);
-      } else {
-        sigma[row] = 0;
-      }
+      op.sigma[row] = sigma_of(S, E, P.bits);
+      if (MODE == kRecheck) op.list[atomicAdd(op.count, 1)] = row;
     }
     __syncthreads();  // redS / redE are reused by the block's next row
   }
@@ -666,7 +716,7 @@ __global__ void __launch_bounds__(256, EL == 8 ? 4 : 2)
 }
 
 // oz_slice over the rows list[0 .. *count - 1] (grid-stride over their
-// thread groups): the rows the one-pass check sent back (see oz_onepass_check)
+// thread groups): the rows the one-pass check sent back (see kRecheck)
 template <typename TIn, bool VEC, int NDIG, int EL, int NMU, int MODE>
 __global__ void __launch_bounds__(256, EL == 8 ? 4 : 2)
     oz_slice_rows(const TIn* __restrict__ X, int64_t ld_doubles, int64_t len, int rows,
@@ -686,38 +736,12 @@ __global__ void __launch_bounds__(256, EL == 8 ? 4 : 2)
   }
 }
 
-// One-pass row scaling: a row whose exponent was estimated (exact[i] = 0)
-// keeps it when its sum of squares at that scale lies within [lo, hi] (the
-// exponent is then the exact one, and clear of the rounding of the sum);
-// otherwise (the estimate was off, the row is zero or not finite, or the sum
-// lies near an exponent boundary) it is listed for its exact norm and a
-// second slicing.
-__global__ void oz_onepass_check(const double* __restrict__ ssq, const int* __restrict__ exact,
-                                 int rows, double lo, double hi, int* __restrict__ list,
-                                 int* __restrict__ count) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= rows) return;
-  const double S = ssq[i];
-  if (!exact[i] && !(S >= lo && S <= hi)) list[atomicAdd(count, 1)] = i;
-}
-
 // --------------------------------------------------------------------------
 // 2a. operands read in place: op(A) = N (A m-major: element (i, kk) at
 // X[i + kk ld], the rows of op(A) are the columns of X) and op(B) = T or C
 // (B n-major the same way). Instead of a k-major copy the norms read them
 // along the rows and the slicer transposes tiles through shared memory.
 constexpr int kMnRows = 65536;  // rows from which the norms need no k-slicing
-
-// sigma from the exponent-tracked sum of squares S 2^(2E) of a row
-__device__ __forceinline__ int sigma_of(double S, int E, int q_bits) {
-  if (!(S < 1e300)) return kSigmaNonFinite;  // NaN or infinite input
-  if (S > 0.0) {
-    int e0 = 0;
-    frexp(sqrt(S), &e0);
-    return q_bits - (e0 + E);
-  }
-  return 0;
-}
 
 // Row scale exponents of m-major rows, as oz_row_scale computes them: one
 // thread per row and k-slice (a warp reads 32 consecutive rows of one kk:
@@ -726,7 +750,8 @@ __device__ __forceinline__ int sigma_of(double S, int E, int q_bits) {
 // partS / partE [slice][row] for oz_row_scale_combine.
 template <typename TIn, bool CPLX>
 __global__ void __launch_bounds__(256) oz_row_scale_mn(const TIn* __restrict__ X, int64_t ld,
-                                                       int m, int64_t k, int64_t kspan, int q_bits,
+                                                       int m, int64_t k, int64_t kspan,
+                                                       ScaleBits bits,
                                                        int* __restrict__ sigma,
                                                        double* __restrict__ partS,
                                                        int* __restrict__ partE) {
@@ -774,25 +799,34 @@ __global__ void __launch_bounds__(256) oz_row_scale_mn(const TIn* __restrict__ X
     }
   }
   if (gridDim.y == 1) {
-    sigma[i] = sigma_of(S, E, q_bits);
+    sigma[i] = sigma_of(S, E, bits);
   } else {
     partS[int64_t(blockIdx.y) * m + i] = S;
     partE[int64_t(blockIdx.y) * m + i] = E;
   }
 }
 
-// sigma of each row from its k-slice partial sums
+// sigma of each row from its k-slice partial sums: 32 rows per block, eight
+// threads (of eight warps) to a row
 __global__ void __launch_bounds__(256) oz_row_scale_combine(const double* __restrict__ partS,
                                                             const int* __restrict__ partE, int m,
-                                                            int slices, int q_bits,
+                                                            int slices, ScaleBits bits,
                                                             int* __restrict__ sigma) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= m) return;
+  __shared__ double sumS[8][32];
+  __shared__ int sumE[8][32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int i = blockIdx.x * 32 + lane;
   double S = 0.0;
   int E = -2100;
-  for (int sl = 0; sl < slices; ++sl)
-    scaled_add(S, E, partS[int64_t(sl) * m + i], partE[int64_t(sl) * m + i]);
-  sigma[i] = sigma_of(S, E, q_bits);
+  if (i < m)
+    for (int sl = w; sl < slices; sl += 8)
+      scaled_add(S, E, partS[int64_t(sl) * m + i], partE[int64_t(sl) * m + i]);
+  sumS[w][lane] = S;
+  sumE[w][lane] = E;
+  __syncthreads();
+  if (w != 0 || i >= m) return;
+  for (int v = 1; v < 8; ++v) scaled_add(S, E, sumS[v][lane], sumE[v][lane]);
+  sigma[i] = sigma_of(S, E, bits);
 }
 
 // Raw element of ESZ bytes (a complex or real value of TIn) in shared memory
@@ -2054,6 +2088,7 @@ Layout layout_of(const GemmProblem& p, int moduli) {
   L.off_tiles = off;
   off = align256(off + sizeof(int) * size_t((L.rowsA + 255) / 256) * ((L.nb + 255) / 256));
   L.off_partA = off;
+  // (reserved: partial sums of the in-place norms, now in the residues' room)
   off = align256(off + (L.ksA > 1 ? size_t(L.ksA) * L.rowsA * (sizeof(double) + sizeof(int)) : 0));
   L.off_partB = off;
   off = align256(off + (L.ksB > 1 ? size_t(L.ksB) * L.rowsB * (sizeof(double) + sizeof(int)) : 0));
@@ -2278,39 +2313,41 @@ void launch_slice_mn(int ndig, cudaStream_t st, const TIn* X, int64_t ld, int m,
   }
 }
 
-// Row scale exponents of A (which & 1) and B (which & 2).
+// k-slices of the in-place row norms: threads (one per row and slice) for two
+// full loads of the GPU, slices of at least 32 elements (a thread's loads go out in
+// batches of 8), at most 4096 (the grid's y extent). The partial sums lie where
+// the operand's residues go next. Slices of 512 elements and more had left a 1501
+// x 1207 operand with 24 blocks (39.8 us; now 5.6).
+int in_place_slices(int64_t rows, int64_t k) {
+  if (rows >= oz::kMnRows) return 1;
+  const int64_t want = (int64_t(oz::sm_count()) * 4096 + rows - 1) / rows;
+  return int(std::max<int64_t>(1, std::min({want, (k + 31) / 32, int64_t(4096)})));
+}
+
+// Row scale exponents of the operands read in place.
 template <typename TIn>
-void scale_operands(const oz::Layout& L, const oz::Crt& crt, const GemmProblem& p, bool cplx,
-                    int* sigA, int* sigB, char* w, int which, cudaStream_t st) {
+void scale_in_place(const oz::Layout& L, const oz::Crt& crt, const GemmProblem& p, bool cplx,
+                    int* sigA, int* sigB, int8_t* resA, int8_t* resB, cudaStream_t st) {
   using namespace oz;
-  const int64_t ldA = cplx ? 2 * p.lda : p.lda;  // in real elements
-  const int64_t ldB = cplx ? 2 * p.ldb : p.ldb;
-  // m-major rows read in place: k-sliced norms, combined when sliced
-  auto in_place = [&](const void* X, int64_t ld, int rows, int ks, size_t off_part, int* sig) {
+  const ScaleBits bits{crt.q_bits, crt.thr};
+  auto scale = [&](const void* X, int64_t ld, int rows, int8_t* scratch, int* sig) {
+    const int ks = in_place_slices(rows, p.k);
     const int64_t kspan = (p.k + ks - 1) / ks;
-    double* partS = reinterpret_cast<double*>(w + off_part);
-    int* partE = reinterpret_cast<int*>(w + off_part + sizeof(double) * size_t(ks) * rows);
+    double* partS = reinterpret_cast<double*>(scratch);
+    int* partE = reinterpret_cast<int*>(scratch + sizeof(double) * size_t(ks) * rows);
     const dim3 grid(unsigned((rows + 255) / 256), unsigned(ks));
     if (cplx)
       oz_row_scale_mn<TIn, true><<<grid, 256, 0, st>>>(static_cast<const TIn*>(X), ld, rows, p.k,
-                                                       kspan, crt.q_bits, sig, partS, partE);
+                                                       kspan, bits, sig, partS, partE);
     else
       oz_row_scale_mn<TIn, false><<<grid, 256, 0, st>>>(static_cast<const TIn*>(X), ld, rows, p.k,
-                                                        kspan, crt.q_bits, sig, partS, partE);
+                                                        kspan, bits, sig, partS, partE);
     if (ks > 1)
-      oz_row_scale_combine<<<unsigned((rows + 255) / 256), 256, 0, st>>>(partS, partE, rows, ks,
-                                                                         crt.q_bits, sig);
+      oz_row_scale_combine<<<unsigned((rows + 31) / 32), 256, 0, st>>>(partS, partE, rows, ks,
+                                                                       bits, sig);
   };
-  if ((which & 1) && L.mn)
-    in_place(p.A, p.lda, L.rowsA, L.ksA, L.off_partA, sigA);
-  else if (which & 1)
-    oz_row_scale<TIn><<<L.rowsA, 256, 0, st>>>(static_cast<const TIn*>(p.A), ldA, L.K2,
-                                               L.rowsA, crt.q_bits, sigA);
-  if ((which & 2) && L.mnB)
-    in_place(p.B, p.ldb, L.rowsB, L.ksB, L.off_partB, sigB);
-  else if (which & 2)
-    oz_row_scale<TIn><<<L.rowsB, 256, 0, st>>>(static_cast<const TIn*>(p.B), ldB, L.K2,
-                                               L.rowsB, crt.q_bits, sigB);
+  if (L.mn) scale(p.A, p.lda, L.rowsA, resA, sigA);
+  if (L.mnB) scale(p.B, p.ldb, L.rowsB, resB, sigB);
 }
 
 // Slicer constants of the moduli (s_sign: the sign of j, split moduli), and the
@@ -2374,8 +2411,12 @@ void launch_slice_mma(const oz::Layout& L, const oz::Crt& crt, const double* X, 
   }
   const long long slots = (long long)kSliceBlocks * sm_count();
   const long long steps = (long long)rows * P.steps_per_row;
-  P.run = int(std::max<long long>(1, std::min<long long>(16, steps / (4 * slots))));
-  const long long segs = (P.steps_per_row + P.run * wpr - 1) / (P.run * wpr);
+  // equal segments of a row, of at most 32 steps per warp, and short enough for
+  // about eight chunks per block (k = 250000: 6.0 ms for both operands with 16, 5.6
+  // with 32; the ring fills anew for each)
+  const long long most = std::max<long long>(1, std::min<long long>(32, steps / (32 * slots)));
+  const long long segs = (P.steps_per_row + most * wpr - 1) / (most * wpr);
+  P.run = int((P.steps_per_row + segs * wpr - 1) / (segs * wpr));
   const long long chunks = ((long long)rows * wpr + 3) / 4 * segs;
   const unsigned grid = unsigned(std::min(slots, chunks));
   if (ssq)
@@ -2388,10 +2429,12 @@ void launch_slice_mma(const oz::Layout& L, const oz::Crt& crt, const double* X, 
 template <typename TIn>
 void slice_operands(const oz::Layout& L, const oz::Crt& crt, const GemmProblem& p, bool cplx,
                     const int* sigA, const int* sigB, int8_t* resA, int8_t* resB, int which,
-                    cudaStream_t st, double* ssqA, double* ssqB) {
+                    cudaStream_t st, double* ssq) {
   using namespace oz;
   const TIn* A = static_cast<const TIn*>(p.A);
   const TIn* B = static_cast<const TIn*>(p.B);
+  double* ssqA = ssq && !L.mn ? ssq : nullptr;
+  double* ssqB = ssq && !L.mnB ? ssq + L.rowsA : nullptr;
   const int64_t ldA = cplx ? 2 * p.lda : p.lda;  // in real elements
   const int64_t ldB = cplx ? 2 * p.ldb : p.ldb;
   const int vec_elems = 16 / int(sizeof(TIn));
@@ -2457,7 +2500,13 @@ void slice_operands(const oz::Layout& L, const oz::Crt& crt, const GemmProblem& 
 // k-major operand (an operand read in place keeps its norms) with the
 // default modulus count and unrolled slicer and rows of at least kOnePassMinLen reals; SPLAB_OZAKI_ONEPASS=0 (read per call) keeps
 // the two-pass order.
-constexpr int64_t kOnePassMinLen = 131072;
+//
+// It pays from about 256 MB of k-major operands: the norms' second read (6 TB/s)
+// against the sample and two more launches (387 x 515 x 60013 complex double, 866
+// MB: 150 us of norms, 27 us of estimates and checks); rows of 16384 reals keep 64
+// reals per run. Rows of 131072 reals always take it.
+constexpr int64_t kOnePassMinLen = 16384, kOnePassLongLen = 131072;
+constexpr double kOnePassMinBytes = 256e6;
 constexpr int kOnePassRuns = 16;
 
 // The operands scaled in one pass: bit 1 A, bit 2 B (k-major ones only; the
@@ -2467,27 +2516,46 @@ int onepass_operands(const oz::Layout& L, const GemmProblem& p) {
   if (v && v[0] == '0') return 0;
   const int nu = dtype_is_double(p.dtype) ? oz::kDefaultModuli : oz::kDefaultModuliFloat;
   const bool unrolled = dtype_is_complex(p.dtype) ? L.split : L.nmod == nu;
-  if (!(p.k > 0 && unrolled && slice_unroll() && L.K2 >= kOnePassMinLen)) return 0;
+  if (p.k <= 0 || !unrolled || !slice_unroll() || L.K2 < kOnePassMinLen) return 0;
+  const double bytes = double((L.mn ? 0 : L.rowsA) + (L.mnB ? 0 : L.rowsB)) * double(L.K2) *
+                       (dtype_is_double(p.dtype) ? 8 : 4);
+  if (L.K2 < kOnePassLongLen && bytes < kOnePassMinBytes) return 0;
   return (L.mn ? 0 : 1) | (L.mnB ? 0 : 2);
 }
 
-// Exponents of A's (which & 1) and B's (which & 2) rows, estimated from the
-// sample where that is safe, else exact (exact[row] = 1; p reads A k-major)
-template <typename TIn>
-void onepass_estimate(const oz::Layout& L, const oz::Crt& crt, const GemmProblem& p, bool cplx,
-                      int* sigA, int* sigB, int* exactA, int* exactB, int which,
+// oz_row_scale's operands: the k-major ones, all or none of them scaled in one pass.
+// onepass: layout of the lists at `list` (A's rows, B's rows, their exact flags, the
+// two counts).
+template <typename TIn, int MODE>
+void launch_row_scale(const oz::Layout& L, const oz::Crt& crt, const GemmProblem& p, bool cplx,
+                      int* sigA, int* sigB, double* ssq, int* list, int* status,
                       cudaStream_t st) {
-  const int64_t run = (L.K2 / (16 * kOnePassRuns) + 7) / 8 * 8;  // reals per run
-  const int64_t gap = L.K2 / kOnePassRuns;                         // run starts
-  const int64_t ldA = cplx ? 2 * p.lda : p.lda, ldB = cplx ? 2 * p.ldb : p.ldb;
-  if (which & 1)
-    oz::oz_row_scale<TIn><<<L.rowsA, 256, 0, st>>>(static_cast<const TIn*>(p.A), ldA, L.K2,
-                                                   L.rowsA, crt.q_bits, sigA, nullptr, nullptr,
-                                                   kOnePassRuns, run, gap, exactA);
-  if (which & 2)
-    oz::oz_row_scale<TIn><<<L.rowsB, 256, 0, st>>>(static_cast<const TIn*>(p.B), ldB, L.K2,
-                                                   L.rowsB, crt.q_bits, sigB, nullptr, nullptr,
-                                                   kOnePassRuns, run, gap, exactB);
+  using namespace oz;
+  RowScaleParams P{};
+  const int64_t re = cplx ? 2 : 1;
+  int* exact = list + L.rowsA + L.rowsB;
+  int* count = exact + L.rowsA + L.rowsB;
+  P.op[0] = {p.A, re * p.lda, L.mn ? 0 : L.rowsA, sigA, exact, ssq, list, count};
+  P.op[1] = {p.B,          re * p.ldb,     L.mnB ? 0 : L.rowsB, sigB, exact + L.rowsA,
+             ssq + L.rowsA, list + L.rowsA, count + 1};
+  P.len = L.K2;
+  P.bits = {crt.q_bits, crt.thr};
+  P.nruns = kOnePassRuns;
+  P.run = (L.K2 / (16 * kOnePassRuns) + 7) / 8 * 8;
+  P.gap = L.K2 / kOnePassRuns;
+  // the two sums of squares (norm kernel: runs of K2 / 256 terms per thread, then
+  // trees; slicers: at most 64 terms per thread, trees, at most K2 / 2048 atomics
+  // per row) differ by at most about (K2 / 256 + K2 / 2048 + 64) units of 2^-53
+  // relative; the margin is 2^-30, or K2 2^-59 for rows beyond 2^29 reals
+  const double delta = std::max(std::ldexp(1.0, -30), std::ldexp(double(L.K2), -59));
+  const double low = std::ldexp(crt.thr, crt.q_bits);  // scaled norms lie in [low, 2 low)
+  P.lo = low * low * (1.0 + delta);
+  P.hi = 4.0 * low * low * (1.0 - delta);
+  P.status = status;
+  const int rows = P.op[0].rows + P.op[1].rows;
+  if (rows == 0) return;
+  const int grid = MODE == kRecheck ? std::min(rows, 2 * sm_count()) : rows;
+  oz_row_scale<TIn, MODE><<<unsigned(grid), 256, 0, st>>>(P);
 }
 
 template <typename TIn, bool VEC, int EL, int MODE>
@@ -2503,13 +2571,11 @@ void launch_slice_rows_el(cudaStream_t st, const TIn* X, int64_t ld, int64_t len
       <<<grid, 256, 0, st>>>(X, ld, len, rows, kp, sig, s_sign, res, lay, stride, sc, list, count);
 }
 
-// The listed rows of one operand: exact exponent, then residues again
+// The listed rows of one operand: residues again
 template <typename TIn>
 void onepass_redo(const oz::Layout& L, const oz::Crt& crt, const TIn* X, int64_t ld, int rows,
-                  int* sig, int s_sign, int8_t* res, const int* list, const int* count,
+                  const int* sig, int s_sign, int8_t* res, const int* list, const int* count,
                   cudaStream_t st) {
-  oz::oz_row_scale<TIn><<<unsigned(std::min(rows, 2 * oz::sm_count())), 256, 0, st>>>(
-      X, ld, L.K2, rows, crt.q_bits, sig, list, count);
   if constexpr (std::is_same<TIn, double>::value) {
     if (L.pairs) {
       launch_slice_mma(L, crt, X, ld, rows, sig, s_sign, res, nullptr, list, count, st);
@@ -2555,24 +2621,10 @@ void onepass_fixup(const oz::Layout& L, const oz::Crt& crt, const GemmProblem& p
                    int* sigA, int* sigB, int8_t* resA, int8_t* resB, double* ssq, int* list,
                    int which, cudaStream_t st) {
   using namespace oz;
-  // the two sums of squares (norm kernel: runs of K2 / 256 terms per thread,
-  // then trees; slicer: 8 terms per thread, trees, K2 / 2048 atomics per
-  // row) differ by at most about (K2 / 256 + K2 / 2048 + 64) units of 2^-53
-  // relative; the margin is 2^-30, or K2 2^-59 for rows beyond 2^29 reals
-  const double delta = std::max(std::ldexp(1.0, -30), std::ldexp(double(L.K2), -59));
-  const double lo = std::ldexp(1.0 + delta, 2 * crt.q_bits - 2);
-  const double hi = std::ldexp(1.0 - delta, 2 * crt.q_bits);
   int* listA = list;
   int* listB = list + L.rowsA;
-  const int* exactA = list + L.rowsA + L.rowsB;
-  const int* exactB = exactA + L.rowsA;
   int* cnt = list + 2 * (L.rowsA + L.rowsB);  // A's count, B's count
-  if (which & 1)
-    oz_onepass_check<<<unsigned((L.rowsA + 255) / 256), 256, 0, st>>>(ssq, exactA, L.rowsA, lo,
-                                                                     hi, listA, cnt);
-  if (which & 2)
-    oz_onepass_check<<<unsigned((L.rowsB + 255) / 256), 256, 0, st>>>(
-        ssq + L.rowsA, exactB, L.rowsB, lo, hi, listB, cnt + 1);
+  launch_row_scale<TIn, kRecheck>(L, crt, p, cplx, sigA, sigB, ssq, list, nullptr, st);
   const int64_t ldA = cplx ? 2 * p.lda : p.lda, ldB = cplx ? 2 * p.ldb : p.ldb;
   if (which & 1)
     onepass_redo<TIn>(L, crt, static_cast<const TIn*>(p.A), ldA, L.rowsA, sigA,
@@ -2582,46 +2634,6 @@ void onepass_fixup(const oz::Layout& L, const oz::Crt& crt, const GemmProblem& p
                       listB, cnt + 1, st);
 }
 
-// Side streams may be used by this host thread (off while a batch captures
-// its sequence of contractions into a CUDA graph on one stream).
-thread_local bool t_side_streams = true;
-
-// Side stream (per device): the row norms of B, a pure read, run there beside
-// the slicing of A (arithmetic-bound) when both are large.
-struct PipeStreams {
-  cudaStream_t lo = nullptr;
-  cudaEvent_t ev_start = nullptr, ev_scaled = nullptr;
-  std::mutex mu;  // one enqueue sequence at a time
-  bool ok = false;
-};
-
-PipeStreams* pipe_streams() {
-  static PipeStreams per_dev[64];
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) {
-    cudaGetLastError();
-    return nullptr;
-  }
-  PipeStreams& ps = per_dev[dev];
-  static std::mutex init_mu;
-  std::lock_guard<std::mutex> lk(init_mu);
-  if (!ps.ok) {
-    const bool good =
-        cudaStreamCreateWithFlags(&ps.lo, cudaStreamNonBlocking) == cudaSuccess &&
-        cudaEventCreateWithFlags(&ps.ev_start, cudaEventDisableTiming) == cudaSuccess &&
-        cudaEventCreateWithFlags(&ps.ev_scaled, cudaEventDisableTiming) == cudaSuccess;
-    if (!good) {
-      cudaGetLastError();
-      return nullptr;
-    }
-    ps.ok = true;
-  }
-  return &ps;
-}
-
-}  // namespace
-
-namespace {
 // Tensor-core CRT reconstruction (oz_reconstruct_tc), the default for byte
 // residues (one k-chunk) with m % 16 == 0, m >= 128 and at most 64 product
 // planes; SPLAB_OZAKI_RECON_TC=0 (read per call) selects the CUDA-core
@@ -2761,80 +2773,42 @@ cudaError_t ozaki_gemm(const GemmProblem& p_in, int moduli, void* ws, size_t ws_
     p.opA = 1;
   }
   const bool dbl = dtype_is_double(p.dtype);
-  // Large problems use the side stream: the row norms of B run beside the slicing
-  // of A.
-  const bool big = double(L.rowsA + L.rowsB) * double(L.K2) * dtype_bytes(p.dtype) /
-                       (cplx ? 2.0 : 1.0) >= 5e8;
-  static const bool side_norms = [] {
-    const char* v = std::getenv("SPLAB_OZAKI_SIDE_NORMS");
-    return !(v && v[0] == '0');
-  }();
   const int onepass = onepass_operands(L, p);
   double* ssq = reinterpret_cast<double*>(w + L.off_ssq);
   int* oplist = reinterpret_cast<int*>(w + L.off_list);
-  PipeStreams* ps =
-      p.k > 0 && big && side_norms && t_side_streams ? pipe_streams() : nullptr;
-  std::unique_lock<std::mutex> lk;
-  if (ps) lk = std::unique_lock<std::mutex>(ps->mu);
-  auto scale = [&](int which, cudaStream_t s) {
-    if (dbl)
-      scale_operands<double>(L, crt, p, cplx, sigA, sigB, w, which, s);
-    else
-      scale_operands<float>(L, crt, p, cplx, sigA, sigB, w, which, s);
-  };
   phase_mark(0, false, st);
   if (L.at && p.k > 0) {
     phase_mark(15, false, st);
     if ((e = transpose_a(p_in, L, w + L.off_At, st)) != cudaSuccess) return e;
     phase_mark(15, true, st);
   }
-  // row exponents of A (which & 1) and B (which & 2): estimated for the
-  // operands scaled in one pass, else the exact norms
-  int* exactA = oplist + L.rowsA + L.rowsB;
-  auto exponents = [&](int which, cudaStream_t s) {
-    if (which & onepass) {
-      if (dbl)
-        onepass_estimate<double>(L, crt, p, cplx, sigA, sigB, exactA, exactA + L.rowsA,
-                                 which & onepass, s);
+  // row exponents (the norms of operands read in place first, alone: beside the
+  // slicing they measured slower)
+  if (p.k > 0) {
+    phase_mark(16, false, st);
+    if (L.mn && L.mnB) cudaMemsetAsync(status, 0, sizeof(int), st);
+    auto exponents = [&](auto tag) {
+      using TIn = decltype(tag);
+      scale_in_place<TIn>(L, crt, p, cplx, sigA, sigB, resA, resB, st);
+      if (onepass)
+        launch_row_scale<TIn, kEstimate>(L, crt, p, cplx, sigA, sigB, ssq, oplist, status, st);
       else
-        onepass_estimate<float>(L, crt, p, cplx, sigA, sigB, exactA, exactA + L.rowsA,
-                                which & onepass, s);
-    }
-    if (which & ~onepass) scale(which & ~onepass, s);
-  };
-  if (onepass && ((e = cudaMemsetAsync(ssq, 0, sizeof(double) * (size_t(L.rowsA) + L.rowsB),
-                                       st)) != cudaSuccess ||
-                  (e = cudaMemsetAsync(oplist + 2 * (L.rowsA + L.rowsB), 0, 2 * sizeof(int),
-                                       st)) != cudaSuccess))
-    return e;
-  const bool side_exponents = p.k > 0 && ps && onepass != 1;
-  if (side_exponents) {
-    // A's exponents alone (norms are pure reads and would share the
-    // bandwidth), then B's on the side stream while A is sliced
-    phase_mark(16, false, st);
-    exponents(1, st);
-    phase_mark(16, true, st);
-    if ((e = cudaEventRecord(ps->ev_start, st)) != cudaSuccess) return e;
-    if ((e = cudaStreamWaitEvent(ps->lo, ps->ev_start, 0)) != cudaSuccess) return e;
-    exponents(2, ps->lo);
-    if ((e = cudaEventRecord(ps->ev_scaled, ps->lo)) != cudaSuccess) return e;
-  } else if (p.k > 0) {
-    // B's exact norms first, alone, when only A is scaled in one pass: beside
-    // A's slicing with its sums of squares they measured slower (op(A) = C,
-    // op(B) = C at the headline size: 18.2 against 18.0 ms for two passes)
-    phase_mark(16, false, st);
-    exponents(2, st);
-    exponents(1, st);
+        launch_row_scale<TIn, kExact>(L, crt, p, cplx, sigA, sigB, ssq, oplist, status, st);
+    };
+    if (dbl)
+      exponents(double{});
+    else
+      exponents(float{});
     phase_mark(16, true, st);
   } else {
     cudaMemsetAsync(sigA, 0, sizeof(int) * L.rowsA, st);
     cudaMemsetAsync(sigB, 0, sizeof(int) * L.rowsB, st);
+    cudaMemsetAsync(status, 0, sizeof(int), st);
   }
   // byte residues are stored, not accumulated: every element the
   // reconstruction reads is written by the GEMM
   if (!L.r8)
     cudaMemsetAsync(R, 0, sizeof(int) * size_t(L.nmod) * L.nsub * L.nb * L.rowsA, st);
-  cudaMemsetAsync(status, 0, sizeof(int), st);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   if (p.k <= 0) {
     phase_mark(0, true, st);
@@ -2842,13 +2816,12 @@ cudaError_t ozaki_gemm(const GemmProblem& p_in, int moduli, void* ws, size_t ws_
     phase_mark(1, true, st);
   } else {
     // with one-pass scaling the slicer also sums the rows' scaled squares
-    double* ssqA = (onepass & 1) ? ssq : nullptr;
-    double* ssqB = (onepass & 2) ? ssq + L.rowsA : nullptr;
+    double* sums = onepass ? ssq : nullptr;
     auto slice = [&](int which) {
       if (dbl)
-        slice_operands<double>(L, crt, p, cplx, sigA, sigB, resA, resB, which, st, ssqA, ssqB);
+        slice_operands<double>(L, crt, p, cplx, sigA, sigB, resA, resB, which, st, sums);
       else
-        slice_operands<float>(L, crt, p, cplx, sigA, sigB, resA, resB, which, st, ssqA, ssqB);
+        slice_operands<float>(L, crt, p, cplx, sigA, sigB, resA, resB, which, st, sums);
     };
     CUtensorMap mapA, mapB;
     if (!make_map(&mapA, resA, L, L.rowsA, BM) || !make_map(&mapB, resB, L, L.nb, BN))
@@ -2984,9 +2957,6 @@ cudaError_t ozaki_gemm(const GemmProblem& p_in, int moduli, void* ws, size_t ws_
     phase_mark(17, false, st);
     slice(1);
     phase_mark(17, true, st);
-    // B once its row norms are done (on the side stream when there is one)
-    if (side_exponents && (e = cudaStreamWaitEvent(st, ps->ev_scaled, 0)) != cudaSuccess)
-      return e;
     phase_mark(18, false, st);
     slice(2);
     phase_mark(18, true, st);
@@ -3104,8 +3074,6 @@ cudaError_t ozaki_gemm(const GemmProblem& p_in, int moduli, void* ws, size_t ws_
 int* ozaki_status_ptr(const GemmProblem& p, int moduli, void* ws) {
   return reinterpret_cast<int*>(static_cast<char*>(ws) + oz::layout_of(p, moduli).off_status);
 }
-
-void ozaki_allow_side_streams(bool allow) { t_side_streams = allow; }
 
 int ozaki_status(const GemmProblem& p, int moduli, void* ws, cudaStream_t st) {
   const oz::Layout L = oz::layout_of(p, moduli);

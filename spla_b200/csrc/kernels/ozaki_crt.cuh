@@ -41,7 +41,13 @@ struct Crt {
   unsigned long long w_lo[kMaxModuli], w_hi[kMaxModuli];  // CRT weights W_t < P
   unsigned long long P_lo, P_hi;
   double P_d;
-  int q_bits;  // Q: scaled rows have 2-norm < 2^Q
+  int q_bits;  // Q: the room for scaled row norms is 2^Q or up to twice that
+  // A row of norm f 2^e, f in [0.5, 1), is scaled by 2^(Q - e), and by one bit more
+  // when f < thr: its scaled norm stays below 2 thr 2^Q (2^Q for thr = 0.5), whose
+  // square is below P/4. So the exponents change at norms of thr 2^e instead of
+  // powers of two, where the norms of normalised rows lie, and rows below it gain
+  // the bit that the floor in Q leaves unused.
+  double thr;
   // split moduli: j with j^2 = -1 (mod p), and the weights of Re = (u + v) / 2
   // (w above, times 1/2 mod p) and of Im = (u - v) / (2j) (wi)
   int j[kMaxModuli];
@@ -88,11 +94,24 @@ inline Crt make_crt_of(const int* moduli, int n, bool split) {
   // |X| <= (2^Q + sqrt(K)/2)^2 must stay below P/2: Q = floor((log2 P - 2) / 2).
   const double lp = std::log2(c.P_d);
   c.q_bits = int(std::floor((lp - 2.0) / 2.0));
+  // 2^((log2 P - 2) / 2) = 2 f 2^Q for f in [0.5, 1), less 1.6 %; without the extra
+  // bit when that would put the exponents' change next to a power of two again
+  const double f = std::exp2((lp - 2.0) / 2.0 - c.q_bits) / 2.0 * (1.0 - 1.0 / 64);
+  c.thr = f < 0.6 ? 0.5 : f;
   return c;
 }
 
 inline Crt make_crt(int n) { return make_crt_of(kModuli, n, false); }
-inline Crt make_crt_split(int n) { return make_crt_of(kSplitModuli, n, true); }
+inline Crt make_crt_split(int n) {
+  Crt c = make_crt_of(kSplitModuli, n, true);
+  // ten moduli: 2^37.26 is next to a power of two; scaled norms below 0.75 2^37
+  // instead keep the change away from it (the nine general moduli give 2^34)
+  if (n == kSplitCountFloat) {
+    c.q_bits -= 1;
+    c.thr = 0.75;
+  }
+  return c;
+}
 
 // v mod p in [0, p) for any int32 v and 2 <= p <= 256 without a division:
 // v = hi * 2^16 + lo, t = hi * (2^16 mod p) + lo = v (mod p) with |t| < 2^24,

@@ -245,9 +245,8 @@ __device__ __forceinline__ int stage_place(int l) {
 // reals each at a time. Each warp keeps the copies of its next four steps in
 // flight in a ring of its own in shared memory, so that the loads do not depend on
 // the registers the residues leave, and has the next step's digits ready (a chain
-// of conversions and a shuffle) when it starts on one. Runs of 16 steps per warp
-// pay for one atomic per warp and segment with SSQ; small operands take shorter
-// ones to fill the GPU, and rows of one to three steps fewer warps each. Four
+// of conversions and a shuffle) when it starts on one. Rows of two or three steps
+// take two warps each. With SSQ one atomic per warp and segment. Four
 // blocks per SM: with more, the few registers spilled per step miss the L1 that
 // the stream of loads and stores goes through (60 % slower).
 template <bool SSQ>
