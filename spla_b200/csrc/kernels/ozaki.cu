@@ -29,7 +29,7 @@
 //   3. Residues. For pairwise coprime moduli p_t <= 256 with product P, the
 //      residues of A', B' mod p_t (symmetric, int8) are multiplied exactly on the
 //      INT8 tensor cores with INT32 accumulation (k-chunks of at most 124928
-//      so that 128*128*chunk < 2^31), reduced mod p_t and summed over chunks.
+//      so that the sums stay below 2^31), reduced mod p_t and summed over chunks.
 //   4. Reconstruction. The Chinese remainder theorem gives X exactly (|X| <=
 //      P/4, so the quotient S/P rounds to the right integer without
 //      correction); C = 2^(-sigma_i - tau_j) X, then alpha/beta.
@@ -44,7 +44,7 @@
 // oz_gemm_pair / oz_gemm
 // (tcgen05.mma kind::i8, TMA-fed, TMEM accumulators, warp-specialised
 // persistent kernels), oz_reconstruct_tc (CRT sums on the tensor cores) and
-// oz_reconstruct / oz_reconstruct_staged (CRT on the CUDA cores), each with
+// oz_reconstruct (CRT on the CUDA cores), each with
 // scaling, alpha/beta and fill-mode tile skipping into C.
 #include <cuda.h>
 #include <cudaTypedefs.h>
@@ -78,8 +78,10 @@ constexpr int B_STAGE = BN * BKB;  // 32 KiB
 constexpr int STAGE_BYTES = A_STAGE + B_STAGE;
 constexpr int GEMM_THREADS = 192;  // warp 0: TMA, warp 1: MMA, warps 2-5: epilogue
 constexpr int GEMM_SMEM = STAGES * STAGE_BYTES + 1024 /*barriers*/ + 1024 /*alignment*/;
-// Max k (bytes) per INT32 accumulation: 127/128 * 128 * 128 * chunk < 2^31.
-constexpr int kChunkBlocks = 976;  // 976 * 128 = 124928
+// Most k-blocks of 128 bytes per INT32 accumulation: 127/128 * 128 * 128 * k < 2^31
+// for the general moduli, 122 * 122 * k < 2^31 for the split ones (p <= 241).
+constexpr int kChunkBlocks = 976;        // 976 * 128 = 124928
+constexpr int kChunkBlocksSplit = 1127;  // 1127 * 128 = 144256
 constexpr unsigned long long kWaitLimitNs = 2000000000ull;  // 2 s bound on any wait
 
 // --------------------------------------------------------------------------
@@ -931,8 +933,10 @@ struct GemmParams {
   int nsub;          // products per modulus (Layout::nsub): modulus = product / nsub
   int tiles_m, tiles_n;
   int total_units;   // products * nchunks * tiles
-  int* R;            // accumulated residues [nmod][nb][m] (int32), or
-  unsigned char* R8; // with a single k-chunk: the residues as bytes (no accumulation)
+  int* R;            // accumulated residues [product][nb][m] (int32), or
+  unsigned char* R8; // bytes [chunk][product][nb][ldr], one plane per k-chunk
+  int ldr;           // elements between the columns of a plane, and between planes
+  int64_t rplane;
   int* status;       // set to 1 when a bounded wait gave up
   const int* active; // CTA-pair kernel: list of tiles to compute (fill mode), or null = all
   int n_active;
@@ -1124,7 +1128,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
       const unsigned M = g.M[mt];
       const int i = w.tm * BM + row;
       const int j0 = w.tn * BN;
-      int* Rt = g.R + int64_t(w.t) * g.nb * g.m;
+      int* Rt = g.R + w.t * g.rplane;
+      unsigned char* R8t = g.R8 + (int64_t(w.c) * g.nmod + w.t) * g.rplane;
       for (int c0 = 0; c0 < BN; c0 += 32) {
         uint32_t v[32];
         tmem_ld32(tmem_base + (uint32_t(quarter * 32) << 16) + uint32_t(accb * BN + c0), v);
@@ -1135,9 +1140,9 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
             if (j < g.nb) {
               const int r = mod_residue(int(v[c]), p, c16, off, M);
               if (g.R8)
-                g.R8[int64_t(w.t) * g.nb * g.m + int64_t(j) * g.m + i] = (unsigned char)r;
+                R8t[int64_t(j) * g.ldr + i] = (unsigned char)r;
               else
-                atomicAdd(Rt + int64_t(j) * g.m + i, r);
+                atomicAdd(Rt + int64_t(j) * g.ldr + i, r);
             }
           }
         }
@@ -1380,7 +1385,7 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1)
       const unsigned M = g.M[mt];
       const int i = tm * 256 + row;
       const int jw = tn * (256 * NT) + half * kCols;
-      const int64_t plane = int64_t(t) * g.nb * g.m;
+      const int64_t plane = (g.R8 ? c * g.nmod + t : t) * g.rplane;
       for (int c0 = 0; c0 < kCols; c0 += 32) {
         uint32_t v[32];
         tmem_ld32(tmem_base + (uint32_t(quarter * 32) << 16) +
@@ -1388,18 +1393,18 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1)
                   v);
         const int jb = jw + c0;
         if (i < g.m && jb < g.nb) {
-          const int64_t base = plane + int64_t(jb) * g.m + i;
+          const int64_t base = plane + int64_t(jb) * g.ldr + i;
           if (jb + 32 <= g.nb) {  // whole group of columns: no per-column test
             if (g.R8) {
               unsigned char* d = g.R8 + base;
 #pragma unroll
               for (int cc = 0; cc < 32; ++cc)
-                d[int64_t(cc) * g.m] = (unsigned char)mod_residue(int(v[cc]), p, c16, off, M);
+                d[int64_t(cc) * g.ldr] = (unsigned char)mod_residue(int(v[cc]), p, c16, off, M);
             } else {
               int* d = g.R + base;
 #pragma unroll
               for (int cc = 0; cc < 32; ++cc)
-                atomicAdd(d + int64_t(cc) * g.m, mod_residue(int(v[cc]), p, c16, off, M));
+                atomicAdd(d + int64_t(cc) * g.ldr, mod_residue(int(v[cc]), p, c16, off, M));
             }
           } else {
 #pragma unroll
@@ -1407,9 +1412,9 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1)
               if (jb + cc < g.nb) {
                 const int r = mod_residue(int(v[cc]), p, c16, off, M);
                 if (g.R8)
-                  g.R8[base + int64_t(cc) * g.m] = (unsigned char)r;
+                  g.R8[base + int64_t(cc) * g.ldr] = (unsigned char)r;
                 else
-                  atomicAdd(g.R + base + int64_t(cc) * g.m, r);
+                  atomicAdd(g.R + base + int64_t(cc) * g.ldr, r);
               }
             }
           }
@@ -1490,31 +1495,42 @@ __device__ __forceinline__ void store_c(void* C, int64_t ci, double xr, double x
 
 // Residues of element (i, j) of the real result (real types) or of Re and Im
 // (complex: two product planes per modulus combined by combine_split, or three
-// by combine3), for modulus t. src points at plane 0 of modulus t, element
-// (i, j); planes of one product are `plane` elements apart. off: p for byte
-// residues, off24 for int32 sums.
+// by combine3), for modulus t, summed over the k-chunks. src points at plane 0 of
+// modulus t, element (i, j); planes of one product are `plane`, those of one
+// k-chunk `chunk` elements apart. off: a multiple of p not below any sum.
 template <bool CPLX, bool SPLIT, typename RT>
-__device__ __forceinline__ void product_residues(const RT* src, int64_t plane, int off, int conj,
-                                                 int& re, int& im) {
+__device__ __forceinline__ void product_residues(const RT* src, int64_t plane, int chunks,
+                                                 int64_t chunk, int off, int conj, int& re,
+                                                 int& im) {
+  int r[3] = {int(src[0]), CPLX ? int(src[plane]) : 0, CPLX && !SPLIT ? int(src[2 * plane]) : 0};
+  if (sizeof(RT) == 1) {  // int32: already summed
+    for (int c = 1; c < chunks; ++c) {
+      src += chunk;
+      r[0] += int(src[0]);
+      if (CPLX) r[1] += int(src[plane]);
+      if (CPLX && !SPLIT) r[2] += int(src[2 * plane]);
+    }
+  }
   if (SPLIT) {
-    combine_split(int(src[0]), int(src[plane]), off, re, im);
+    combine_split(r[0], r[1], off, re, im);
   } else if (CPLX) {
-    combine3(int(src[0]), int(src[plane]), int(src[2 * plane]), off, conj, re, im);
+    combine3(r[0], r[1], r[2], off, conj, re, im);
   } else {
-    re = int(src[0]);
+    re = r[0];
     im = 0;
   }
 }
 
 // C(i, j) <- alpha * 2^(-sigma_i - tau_j) * X + beta * C(i, j), X the CRT
 // value of the product (complex: of Re and Im). R holds, per product plane,
-// int32 sums of per-chunk residues or, with one k-chunk, the residues as
-// bytes (RT). Threads run along i (contiguous in R and C), blocks along j: no
+// int32 sums of per-chunk residues or, per k-chunk and product plane, the
+// residues as bytes (RT), columns ldr elements apart. Threads run along i (contiguous in R and C), blocks along j: no
 // index division. NM: the number of moduli when fixed at compile time (the
 // defaults; the complex ones are the split moduli), 0 for rp.n.
 template <int DT, typename RT, int NM>
 __global__ void __launch_bounds__(256, 2) oz_reconstruct(const RT* __restrict__ R, int m, int n,
-                                                         int nb, const int* __restrict__ sigA,
+                                                         int64_t plane, int64_t ldr, int chunks,
+                                                         const int* __restrict__ sigA,
                                                          const int* __restrict__ sigB, void* C,
                                                          int64_t ldc, double alr, double ali,
                                                          double ber, double bei, int fill,
@@ -1523,10 +1539,8 @@ __global__ void __launch_bounds__(256, 2) oz_reconstruct(const RT* __restrict__ 
   constexpr bool CPLX = dtype_is_complex(DT);
   constexpr bool SPLIT = CPLX && NM > 0;
   constexpr int NSUB = SPLIT ? 2 : CPLX ? 3 : 1;
-  constexpr bool kBytes = sizeof(RT) == 1;
   constexpr int NMAX = NM > 0 ? NM : kMaxUsableModuli;
   const int nmod = NM > 0 ? NM : rp.n;
-  const int64_t plane = int64_t(nb) * m;
   const bool read_c = (ber != 0.0 || bei != 0.0);
   for (int j = blockIdx.y; j < n; j += gridDim.y) {
     const int tauj = sigB[j];
@@ -1539,16 +1553,16 @@ __global__ void __launch_bounds__(256, 2) oz_reconstruct(const RT* __restrict__ 
           continue;
       }
       int rr[NMAX], ri[NMAX];
-      const RT* src = R + int64_t(j) * m + i;
+      const RT* src = R + int64_t(j) * ldr + i;
 #pragma unroll
       for (int t = 0; t < NMAX; ++t)
         if (t < nmod)
-          product_residues<CPLX, SPLIT>(src + t * NSUB * plane, plane,
-                                        kBytes ? rp.p[t] : rp.off24[t], rp.conj, rr[t], ri[t]);
+          product_residues<CPLX, SPLIT>(src + t * NSUB * plane, plane, chunks,
+                                        NSUB * nmod * plane, rp.off24[t], rp.conj, rr[t], ri[t]);
       const int si = sigA[i];
       const int e = -(si + tauj);
-      double xr = scale_pow2(crt_value<NM, kBytes>(rr, rp), e);
-      double xi = CPLX ? scale_pow2(crt_value<NM, kBytes, SPLIT>(ri, rp), e) : 0.0;
+      double xr = scale_pow2(crt_value<NM, false>(rr, rp), e);
+      double xi = CPLX ? scale_pow2(crt_value<NM, false, SPLIT>(ri, rp), e) : 0.0;
       if (si == kSigmaNonFinite || tauj == kSigmaNonFinite) xr = xi = __longlong_as_double(kNaNBits);
       store_c<DT>(C, i + int64_t(j) * ldc, xr, xi, alr, ali, ber, bei, read_c);
     }
@@ -1579,120 +1593,8 @@ __global__ void oz_transpose(const E* __restrict__ A, int64_t lda, int m, int64_
   }
 }
 
-// The same reconstruction for byte residues with m % 16 == 0, staged through
-// shared memory: a work item is one column j of C and a block of 1024 rows;
-// its residues (moduli x product planes x 1024 bytes) are copied with 16-byte
-// asynchronous copies into one of two stages while the previous item is
-// reconstructed from the other, so that the CRT arithmetic does not wait on
-// the loads. Items are spread over a grid of resident blocks (item =
-// blockIdx.x + k * gridDim.x, row blocks fastest). Each thread takes four
-// consecutive rows: byte q of word threadIdx.x of each 1024-byte plane.
-constexpr int kStageRows = 1024;
-template <int DT, int NM>
-__global__ void __launch_bounds__(256, 2)
-    oz_reconstruct_staged(const unsigned char* __restrict__ R, int m, int n, int nb,
-                          const int* __restrict__ sigA, const int* __restrict__ sigB, void* C,
-                          int64_t ldc, double alr, double ali, double ber, double bei, int fill,
-                          int64_t ro, int64_t co, int tile_m, int tile_n, ReconParams rp) {
-  constexpr bool CPLX = dtype_is_complex(DT);
-  constexpr bool SPLIT = CPLX && NM > 0;
-  constexpr int NSUB = SPLIT ? 2 : CPLX ? 3 : 1;
-  constexpr int NMAX = NM > 0 ? NM : kMaxUsableModuli;
-  constexpr int WPP = kStageRows / 4;  // 32-bit words per staged plane
-  extern __shared__ uint4 stage_smem[];
-  const int nmod = NM > 0 ? NM : rp.n;
-  const int stage_words = NSUB * nmod * WPP;
-  unsigned* stage = reinterpret_cast<unsigned*>(stage_smem);
-  const int64_t plane = int64_t(nb) * m;
-  const int row_blocks = (m + kStageRows - 1) / kStageRows;
-  const int64_t items = int64_t(row_blocks) * n;
-  const bool read_c = (ber != 0.0 || bei != 0.0);
-
-  // staged plane pl = t * NSUB + s holds product s of modulus t
-  auto prefetch = [&](int64_t item, int s) {
-    const int rb = int(item % row_blocks), j = int(item / row_blocks);
-    const int i0 = rb * kStageRows;
-    const int chunks = min(kStageRows, m - i0) / 16;  // m % 16 == 0
-    const int total = NSUB * nmod * chunks;
-    unsigned* dst = stage + s * stage_words;
-    for (int c = threadIdx.x; c < total; c += blockDim.x) {
-      const int pl = c / chunks, ch = c - pl * chunks;
-      const unsigned char* src = R + pl * plane + int64_t(j) * m + i0 + ch * 16;
-      cp_async_16_cg(dst + pl * WPP + ch * 4, src);
-    }
-  };
-
-  int64_t item = blockIdx.x;
-  if (item < items) prefetch(item, 0);
-  cp_async_commit();
-  int s = 0;
-  for (; item < items; item += gridDim.x) {
-    const int64_t next = item + gridDim.x;
-    if (next < items) prefetch(next, s ^ 1);
-    cp_async_commit();
-    cp_async_wait<1>();
-    __syncthreads();
-    const int rb = int(item % row_blocks), j = int(item / row_blocks);
-    const int i = rb * kStageRows + 4 * threadIdx.x;
-    bool active = i < m;
-    if (active && fill != 0) {  // tile_m is a multiple of 4: the four rows share a tile
-      const int64_t ti = (i / tile_m) * int64_t(tile_m), tj = (j / tile_n) * int64_t(tile_n);
-      active = tile_is_active(fill, ti, tj, ::min((int64_t)tile_m, (int64_t)m - ti),
-                              ::min((int64_t)tile_n, (int64_t)n - tj), ro, co);
-    }
-    if (active) {
-      const unsigned* w = stage + s * stage_words + threadIdx.x;
-      const int tauj = sigB[j];
-      // residues of Re (part 0) or Im (part 1) of row i + q, from the staged
-      // bytes (the arrays of the two parts are built one after the other)
-      auto part_residues = [&](int q, int part, int (&r)[NMAX]) {
-#pragma unroll
-        for (int t = 0; t < NMAX; ++t) {
-          if (t < nmod) {
-            const unsigned* wt = w + t * NSUB * WPP;
-            const int r0 = int((wt[0] >> (8 * q)) & 255u);
-            if (SPLIT) {
-              int re, im;
-              combine_split(r0, int((wt[WPP] >> (8 * q)) & 255u), rp.p[t], re, im);
-              r[t] = part ? im : re;
-            } else if (CPLX) {
-              const int r1 = int((wt[WPP] >> (8 * q)) & 255u);
-              const int r2 = int((wt[2 * WPP] >> (8 * q)) & 255u);
-              int re, im;
-              combine3(r0, r1, r2, rp.p[t], rp.conj, re, im);
-              r[t] = part ? im : re;
-            } else {
-              r[t] = r0;
-            }
-          }
-        }
-      };
-#pragma unroll 1
-      for (int q = 0; q < 4; ++q) {  // rolled: one row's chain at a time keeps registers
-        const int si = sigA[i + q];
-        const int e = -(si + tauj);
-        int r[NMAX];
-        part_residues(q, 0, r);
-        double xr = scale_pow2(crt_value<NM, true>(r, rp), e);
-        double xi = 0.0;
-        if (CPLX) {
-          part_residues(q, 1, r);
-          xi = scale_pow2(crt_value<NM, true, SPLIT>(r, rp), e);
-        }
-        if (si == kSigmaNonFinite || tauj == kSigmaNonFinite) xr = xi = __longlong_as_double(kNaNBits);
-        store_c<DT>(C, i + q + int64_t(j) * ldc, xr, xi, alr, ali, ber, bei, read_c);
-      }
-    }
-    __syncthreads();  // the stage is refilled by the next iteration's prefetch
-    s ^= 1;
-  }
-  cp_async_wait<0>();
-}
-
-inline int staged_smem_bytes(int planes) { return 2 * planes * kStageRows; }
-
 // --------------------------------------------------------------------------
-// 4b. CRT reconstruction on the tensor cores (byte residues, m % 16 == 0)
+// 4b. CRT reconstruction on the tensor cores (byte residues)
 //
 // By linearity the CRT sum needs no reduction of the product combination:
 // with V_k the weight of product plane k, W_t (or the Im weight of a split
@@ -1718,21 +1620,24 @@ inline int staged_smem_bytes(int planes) { return 2 * planes * kStageRows; }
 constexpr int RT_THREADS = 192;
 constexpr int RT_STAGES = 4;
 constexpr int RT_G = 2;                       // blocks of 128 rows per work unit
-constexpr int RT_KP = 64;                     // planes per block (K), padded
-constexpr int RT_BLOCK = 128 * RT_KP;         // bytes per block of 128 rows
-constexpr int RT_STAGE = RT_G * RT_BLOCK;     // bytes per stage
+constexpr int RT_KP = 64;                     // most planes (K)
 constexpr int RT_W_BYTES = 32 * 128;          // weights: 32 rows x 128 B (SW128)
-constexpr int RT_SMEM = RT_STAGES * RT_STAGE + RT_W_BYTES + 256 + 1024;
-// three CTAs fit an SM's shared memory, so their 2 x RT_G x 32 TMEM columns fit
-static_assert(4 * (RT_SMEM + 1024) > 228 * 1024 && 3 * 2 * RT_G * 32 <= 512,
-              "at most three CTAs per SM, within the TMEM");
+// KP planes per block, padded: 32 or 64. CTAs per SM, within its shared memory and
+// its 512 TMEM columns (2 x RT_G x 32 each).
+template <int KP>
+struct ReconCfg {
+  static constexpr int BLOCK = 128 * KP;      // bytes per block of 128 rows
+  static constexpr int STAGE = RT_G * BLOCK;  // bytes per stage
+  static constexpr int SMEM = RT_STAGES * STAGE + RT_W_BYTES + 256 + 1024;
+  static constexpr int CTAS = KP == 32 ? 4 : 3;
+  static_assert(CTAS * (SMEM + 1024) <= 228 * 1024 && CTAS * 2 * RT_G * 32 <= 512, "fits an SM");
+};
 
 struct ReconTcParams {
   int m, n;
   int row_blocks;         // groups of RT_G blocks of 128 rows: ceil(m / (128 RT_G))
   long long total_units;  // row_blocks * n
   int planes;             // product planes of the residue array (loaded per tile)
-  int kp;                 // K of the MMA: 32 or 64 (planes past `planes` are zero rows)
   const int* sigA;
   const int* sigB;
   void* C;
@@ -1769,11 +1674,12 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map
       : "memory");
 }
 
-template <int DT>
-__global__ void __launch_bounds__(RT_THREADS, 3)
+template <int DT, int KP>
+__global__ void __launch_bounds__(RT_THREADS, ReconCfg<KP>::CTAS)
     oz_reconstruct_tc(const __grid_constant__ CUtensorMap tmR,
                       const __grid_constant__ ReconTcParams P) {
   constexpr bool CPLX = dtype_is_complex(DT);
+  constexpr int RT_BLOCK = ReconCfg<KP>::BLOCK, RT_STAGE = ReconCfg<KP>::STAGE;
   constexpr int NO = CPLX ? 32 : 16;  // output columns of the MMA
   // D S32, A and B unsigned int8, A MN-major, B K-major, N = NO, M = 128
   constexpr uint32_t kIdesc = (2u << 4) | (1u << 15) | (uint32_t(NO >> 3) << 17) |
@@ -1801,10 +1707,10 @@ __global__ void __launch_bounds__(RT_THREADS, 3)
     unsigned char* wp = base_ptr + RT_STAGES * RT_STAGE;
     for (int idx = threadIdx.x; idx < RT_W_BYTES; idx += RT_THREADS) {
       const int o = idx >> 7, k = idx & 127;
-      const unsigned char b = (o < NO && k < P.kp) ? P.v[o][k] : 0;
+      const unsigned char b = (o < NO && k < KP) ? P.v[o][k] : 0;
       wp[(o >> 3) * 1024 + (o & 7) * 128 + (((k >> 4) ^ (o & 7)) << 4) + (k & 15)] = b;
     }
-    const int pad = (P.kp - P.planes) * 128;  // bytes per block, 16-byte words below
+    const int pad = (KP - P.planes) * 128;  // bytes per block, 16-byte words below
     for (int idx = threadIdx.x; idx < RT_STAGES * RT_G * (pad / 16); idx += RT_THREADS) {
       const int blk = idx / (pad / 16), w16 = idx - blk * (pad / 16);  // blk: stage, block
       *reinterpret_cast<uint4*>(base_ptr + blk * RT_BLOCK + P.planes * 128 + 16 * w16) =
@@ -1889,7 +1795,7 @@ __global__ void __launch_bounds__(RT_THREADS, 3)
       const uint32_t sa = base + stage * RT_STAGE;
 #pragma unroll
       for (int g = 0; g < RT_G; ++g)
-        for (int kb = 0; kb < P.kp / 32; ++kb)
+        for (int kb = 0; kb < KP / 32; ++kb)
           umma_i8_desc(tmem_base + uint32_t((b * RT_G + g) * 32),
                        umma_desc_sw128_mn(sa + g * RT_BLOCK + kb * 4096),
                        umma_desc_sw128(w_addr + kb * 32), kIdesc, kb > 0 ? 1u : 0u);
@@ -1986,6 +1892,13 @@ __global__ void __launch_bounds__(RT_THREADS, 3)
 // --------------------------------------------------------------------------
 // host orchestration
 
+int sm_count() {
+  int dev = 0, v = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
+  return v;
+}
+
 struct Layout {
   int nmod;
   bool split;              // complex with the split moduli
@@ -1997,7 +1910,9 @@ struct Layout {
   bool mn;                 // op(A) = N: A read in place (m-major)
   bool mnB;                // op(B) = T or C: B read in place (n-major)
   int ksA, ksB;            // k-slices of the in-place row norms of A and B (1: none)
-  bool r8;                 // one k-chunk: the residues of C are stored as bytes
+  int nchunks, nt;         // k-chunks and tile width of the GEMM (choose_gemm)
+  bool r8;                 // the residues of C are bytes, one plane per product and k-chunk
+  int64_t ldR, planeR;     // elements between the columns of a plane and between planes
   int64_t ldAt;            // leading dimension of At (elements of A's type)
   size_t off_sigA, off_sigB, off_resA, off_resB, off_R, off_At, off_status, off_tiles;
   size_t off_partA, off_partB;  // k-slice partial sums of the in-place row norms
@@ -2023,6 +1938,50 @@ ResidueLayout residue_layout(const Layout& L, int rows) {
   const int shift = L.kp < 256 ? 7 : L.kp < 2304 ? 8 : 10;
   const int64_t kc = int64_t(1) << shift, row = (L.kp + kc - 1) / kc * 2 * kc;
   return {rows * row, row, kc, shift, 2};
+}
+
+size_t residue_bytes(const Layout& L, int rows) {
+  const ResidueLayout lay = residue_layout(L, rows);
+  return size_t(L.nmod * L.nsub / lay.G) * size_t(lay.group);
+}
+
+// Time (us) of the INT8 GEMM over `chunks` k-chunks with pair tiles 256 x 256 nt:
+// rounds of work units over the CTA pairs, a unit taking its k-blocks at the measured
+// rate (0.44 us per 256 x 256 x 128, 8 % less in the wider tile, which loads A once
+// for two MMAs) and its hand-over (the wider tile's single accumulator exposes its
+// drain).
+double gemm_model_us(const Layout& L, int64_t m, int64_t n, int chunks, int nt) {
+  const double units = double(L.nmod * L.nsub) * chunks * double((m + 255) / 256) *
+                       double((n + 256 * nt - 1) / (256 * nt));
+  const double blocks = std::ceil(double(L.kp / BKB) / chunks);
+  const double unit = nt == 2 ? blocks * 0.81 + 5.0 : blocks * 0.443 + 1.2;
+  return std::ceil(units / (sm_count() / 2)) * unit;
+}
+
+// k-chunks and tile width of the GEMM. Chunks stay within the exact INT32 bound;
+// more of them fill the CTA pairs when there are few units (256 x 256 real double: 15
+// units for 74 pairs), as long as all byte planes go to the tensor-core reconstruction.
+// Each costs its planes' write and read, and may add at most 4 MB to the workspace
+// (complex problems have room for them anyway, see layout_of).
+constexpr size_t kMoreChunksBytes = size_t(4) << 20;
+void choose_gemm(Layout& L, int64_t m, int64_t n) {
+  const int64_t blocks = L.kp / BKB, planes = L.nmod * L.nsub;
+  const int64_t limit = L.split ? kChunkBlocksSplit : kChunkBlocks;
+  const int least = int(std::max<int64_t>(1, (blocks + limit - 1) / limit));
+  double best = 0.0;
+  L.nchunks = 0;
+  for (int c = least; c == least || (c <= blocks / 4 && c * planes <= RT_KP); ++c) {
+    const double more = double(c - 1) * planes * m * n;  // bytes
+    if (c > least && !L.split && more > kMoreChunksBytes) break;
+    for (int nt = 1; nt <= (n >= 512 ? 2 : 1); ++nt) {
+      const double t = gemm_model_us(L, m, n, c, nt) + more / 2.5e6;
+      if (L.nchunks == 0 || t < 0.97 * best) {
+        best = t;
+        L.nchunks = c;
+        L.nt = nt;
+      }
+    }
+  }
 }
 
 // In-place reading of an m-major operand: the transposing slicer's tiles of
@@ -2068,19 +2027,35 @@ Layout layout_of(const GemmProblem& p, int moduli) {
   L.mnB = p.opB != 0;
   L.ksA = L.mn ? norm_slices(p.m, p.k) : 1;
   L.ksB = L.mnB ? norm_slices(p.n, p.k) : 1;
-  L.r8 = (L.kp / BKB + kChunkBlocks - 1) / kChunkBlocks == 1;
+  choose_gemm(L, p.m, p.n);
+  // bytes where the tensor-core reconstruction takes all planes (its columns lie on
+  // 16-byte boundaries), else one int32 sum per product
+  L.r8 = L.nmod * L.nsub * L.nchunks <= RT_KP;
+  L.ldR = L.r8 ? (p.m + 15) / 16 * 16 : p.m;
+  // byte planes an odd number of 128-byte lines apart: a box of the reconstruction
+  // reads a line of each, which should not fall on few L2 slices
+  L.planeR = L.r8 ? ((L.ldR * L.nb + 127) / 128 | 1) * 128 : L.ldR * L.nb;
   L.ldAt = L.at ? (p.k + 7) / 8 * 8 : 0;
   size_t off = 0;
   L.off_sigA = off;
   off = align256(off + sizeof(int) * L.rowsA);
   L.off_sigB = off;
   off = align256(off + sizeof(int) * L.rowsB);
+  // The workspace is not smaller than that of the three-product form, for callers that
+  // hold one sized for it: 45 planes to the split form's 32 (and int32 sums from the
+  // second k-chunk on), with room for the planes of its k-chunks in the difference.
+  const bool one_chunk = (L.kp / BKB + kChunkBlocks - 1) / kChunkBlocks <= 1;
+  const size_t reserved = align256(planes * L.rowsA * L.kp) + align256(planes * L.nb * L.kp) +
+                          align256((one_chunk ? 1 : sizeof(int)) * planes * L.nb * L.rowsA);
+  const size_t start = off;
   L.off_resA = off;
-  off = align256(off + planes * L.rowsA * L.kp);
+  off = align256(off + residue_bytes(L, L.rowsA));
   L.off_resB = off;
-  off = align256(off + planes * L.nb * L.kp);
+  off = align256(off + residue_bytes(L, L.nb));
   L.off_R = off;
-  off = align256(off + (L.r8 ? 1 : sizeof(int)) * planes * L.nb * L.rowsA);
+  off = align256(off + (L.r8 ? L.nchunks : sizeof(int)) * size_t(L.nmod) * L.nsub *
+                           L.planeR);
+  off = std::max(off, start + reserved);
   L.off_At = off;
   off = align256(off + size_t(dtype_bytes(p.dtype)) * size_t(L.rowsA) * size_t(L.ldAt));
   L.off_status = off;
@@ -2135,14 +2110,15 @@ bool make_map(CUtensorMap* map, void* base, const Layout& L, int rows, int box_r
 }
 
 // Residue bytes of C for the tensor-core reconstruction: dims (m, nb, planes)
-// with strides (m, nb m) bytes (m % 16 == 0, m >= 128), boxes of 128 rows x 1
-// column x all planes (rows past m read as zeros), 128-byte swizzle: one
-// 128-byte row per plane, the MN-major operand layout.
-bool make_map_recon(CUtensorMap* map, void* base, int m, int nb, int planes) {
+// with strides (ldR, planeR) bytes (multiples of 16), boxes of 128 rows x 1 column
+// x all planes (rows past m read as zeros), 128-byte swizzle: one 128-byte row per
+// plane, the MN-major operand layout.
+bool make_map_recon(CUtensorMap* map, void* base, const Layout& L) {
   auto fn = encode_fn();
   if (!fn) return false;
-  cuuint64_t dims[3] = {cuuint64_t(m), cuuint64_t(nb), cuuint64_t(planes)};
-  cuuint64_t strides[2] = {cuuint64_t(m), cuuint64_t(int64_t(nb) * m)};
+  const int planes = L.nmod * L.nsub * L.nchunks;
+  cuuint64_t dims[3] = {cuuint64_t(L.rowsA), cuuint64_t(L.nb), cuuint64_t(planes)};
+  cuuint64_t strides[2] = {cuuint64_t(L.ldR), cuuint64_t(L.planeR)};
   cuuint32_t box[3] = {128u, 1u, cuuint32_t(planes)};
   cuuint32_t estr[3] = {1, 1, 1};
   const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, base, dims, strides, box, estr,
@@ -2151,12 +2127,6 @@ bool make_map_recon(CUtensorMap* map, void* base, int m, int nb, int planes) {
   return r == CUDA_SUCCESS;
 }
 
-int sm_count() {
-  int dev = 0, v = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
-  return v;
-}
 
 }  // namespace oz
 
@@ -2635,16 +2605,14 @@ void onepass_fixup(const oz::Layout& L, const oz::Crt& crt, const GemmProblem& p
 }
 
 // Tensor-core CRT reconstruction (oz_reconstruct_tc), the default for byte
-// residues (one k-chunk) with m % 16 == 0, m >= 128 and at most 64 product
-// planes; SPLAB_OZAKI_RECON_TC=0 (read per call) selects the CUDA-core
-// kernels. True when it applies and its tensor map was made.
+// residues (at most 64 planes over all k-chunks); SPLAB_OZAKI_RECON_TC=0 (read per
+// call) selects the CUDA-core kernel, as do int32 sums. Columns padded to 16 bytes
+// let every m take it: 1501 x 2003 real double 76 us on the CUDA cores (uncoalesced
+// bytes of 15 planes), 31 us here. True when it applies and its tensor map was made.
 bool recon_tc_plan(const oz::Layout& L, unsigned char* R8, CUtensorMap* map) {
-  using namespace oz;
   const char* v = std::getenv("SPLAB_OZAKI_RECON_TC");
-  if ((v && v[0] == '0') || !R8 || L.nmod * L.nsub > RT_KP || L.rowsA % 16 != 0 ||
-      L.rowsA < 128)
-    return false;
-  return make_map_recon(map, R8, L.rowsA, L.nb, L.nmod * L.nsub);
+  if ((v && v[0] == '0') || !R8) return false;
+  return oz::make_map_recon(map, R8, L);
 }
 
 cudaError_t launch_recon_tc(const GemmProblem& p, const oz::Layout& L, const oz::Crt& crt,
@@ -2652,7 +2620,7 @@ cudaError_t launch_recon_tc(const GemmProblem& p, const oz::Layout& L, const oz:
                             const int* sigB, int* status, cudaStream_t st) {
   using namespace oz;
   const bool cplx = dtype_is_complex(p.dtype);
-  const int planes = L.nmod * L.nsub;
+  const int products = L.nmod * L.nsub, planes = products * L.nchunks;
   static thread_local ReconTcParams P;  // 2.7 KB: kept off the stack
   P = ReconTcParams{};
   P.m = L.rowsA;
@@ -2660,7 +2628,6 @@ cudaError_t launch_recon_tc(const GemmProblem& p, const oz::Layout& L, const oz:
   P.row_blocks = (P.m + 128 * RT_G - 1) / (128 * RT_G);
   P.total_units = (long long)P.row_blocks * P.n;
   P.planes = planes;
-  P.kp = planes <= 32 ? 32 : 64;
   P.sigA = sigA;
   P.sigB = sigB;
   P.C = p.C;
@@ -2698,28 +2665,31 @@ cudaError_t launch_recon_tc(const GemmProblem& p, const oz::Layout& L, const oz:
           vim = W;
         }
       }
-      const int k = t * L.nsub + s;
-      for (int o = 0; o < 16; ++o) {
-        P.v[o][k] = static_cast<unsigned char>(vre >> (8 * o));
-        P.v[16 + o][k] = static_cast<unsigned char>(vim >> (8 * o));
-      }
+      // the planes of all k-chunks of a product alike
+      for (int k = t * L.nsub + s; k < planes; k += products)
+        for (int o = 0; o < 16; ++o) {
+          P.v[o][k] = static_cast<unsigned char>(vre >> (8 * o));
+          P.v[16 + o][k] = static_cast<unsigned char>(vim >> (8 * o));
+        }
     }
   }
   P.status = status;
   P.wait_limit_ns = kWaitLimitNs;
-  auto run = [&](auto kern) -> cudaError_t {
-    const cudaError_t ea = set_dynamic_smem(reinterpret_cast<const void*>(kern), RT_SMEM);
+  auto run = [&](auto kern32, auto kern64) -> cudaError_t {
+    const auto kern = planes <= 32 ? kern32 : kern64;
+    const int smem = planes <= 32 ? ReconCfg<32>::SMEM : ReconCfg<64>::SMEM;
+    const int ctas = planes <= 32 ? ReconCfg<32>::CTAS : ReconCfg<64>::CTAS;
+    const cudaError_t ea = set_dynamic_smem(reinterpret_cast<const void*>(kern), smem);
     if (ea != cudaSuccess) return ea;
-    // three CTAs per SM (their shared memory fits, and so their TMEM)
-    const long long grid = std::min<long long>(P.total_units, 3LL * sm_count());
-    kern<<<unsigned(grid), RT_THREADS, RT_SMEM, st>>>(map, P);
+    const long long grid = std::min<long long>(P.total_units, (long long)ctas * sm_count());
+    kern<<<unsigned(grid), RT_THREADS, smem, st>>>(map, P);
     return cudaGetLastError();
   };
   switch (p.dtype) {
-    case kC64: return run(oz_reconstruct_tc<kC64>);
-    case kC32: return run(oz_reconstruct_tc<kC32>);
-    case kR64: return run(oz_reconstruct_tc<kR64>);
-    default: return run(oz_reconstruct_tc<kR32>);
+    case kC64: return run(oz_reconstruct_tc<kC64, 32>, oz_reconstruct_tc<kC64, 64>);
+    case kC32: return run(oz_reconstruct_tc<kC32, 32>, oz_reconstruct_tc<kC32, 64>);
+    case kR64: return run(oz_reconstruct_tc<kR64, 32>, oz_reconstruct_tc<kR64, 64>);
+    default: return run(oz_reconstruct_tc<kR32, 32>, oz_reconstruct_tc<kR32, 64>);
   }
 }
 
@@ -2806,9 +2776,9 @@ cudaError_t ozaki_gemm(const GemmProblem& p_in, int moduli, void* ws, size_t ws_
     cudaMemsetAsync(status, 0, sizeof(int), st);
   }
   // byte residues are stored, not accumulated: every element the
-  // reconstruction reads is written by the GEMM
-  if (!L.r8)
-    cudaMemsetAsync(R, 0, sizeof(int) * size_t(L.nmod) * L.nsub * L.nb * L.rowsA, st);
+  // reconstruction reads is written by the GEMM (k = 0: there is none)
+  if (!L.r8 || p.k <= 0)
+    cudaMemsetAsync(R, 0, (L.r8 ? 1 : sizeof(int)) * size_t(L.nmod) * L.nsub * L.planeR, st);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   if (p.k <= 0) {
     phase_mark(0, true, st);
@@ -2830,7 +2800,7 @@ cudaError_t ozaki_gemm(const GemmProblem& p_in, int moduli, void* ws, size_t ws_
     g.m = L.rowsA;
     g.nb = L.nb;
     g.kblocks = int(L.kp / BKB);
-    g.nchunks = (g.kblocks + kChunkBlocks - 1) / kChunkBlocks;
+    g.nchunks = L.nchunks;
     // equal chunks (each within the exact INT32 bound): equal work units
     g.chunk_blocks = std::max(1, (g.kblocks + g.nchunks - 1) / std::max(1, g.nchunks));
     g.group = residue_layout(L, 1).G;
@@ -2842,6 +2812,8 @@ cudaError_t ozaki_gemm(const GemmProblem& p_in, int moduli, void* ws, size_t ws_
     g.total_units = g.nmod * g.nchunks * g.tiles_m * g.tiles_n;
     g.R = R;
     g.R8 = R8;
+    g.ldr = int(L.ldR);
+    g.rplane = L.planeR;
     g.status = status;
     g.wait_limit_ns = kWaitLimitNs;
     g.stall_test = 0;
@@ -2869,22 +2841,9 @@ cudaError_t ozaki_gemm(const GemmProblem& p_in, int moduli, void* ws, size_t ws_
     const char* gk = std::getenv("SPLAB_OZAKI_GEMM");
     const bool pair = !(gk && gk[0] == '1');  // "1sm" selects the single-CTA kernel
     CUtensorMap mapA2, mapB2;
-    // pair tile 256 x 512 (one A tile for two MMAs, one 512-column
-    // accumulator drained once per unit) when the units are long enough to
-    // hide the drain (128 k-blocks or more) and it needs at most 5 % more
-    // rounds of work units than the double-buffered 256 x 256 tile; measured
-    // 9 % faster on the INT8 GEMM of m = n = 1024, k = 250000 (complex double
-    // and float) under the power cap (SPLAB_OZAKI_NT=1|2 overrides)
-    int nt = 1;
-    if (L.nb >= 512 && g.chunk_blocks >= 128) {
-      const int pairs = std::max(1, sm_count() / 2);
-      auto rounds = [&](int w) {
-        const long long units = (long long)g.nmod * g.nchunks * ((L.rowsA + 255) / 256) *
-                                ((L.nb + 256 * w - 1) / (256 * w));
-        return double((units + pairs - 1) / pairs);
-      };
-      nt = rounds(2) * 2.0 <= rounds(1) * 1.05 ? 2 : 1;
-    }
+    // pair tile 256 x 512 (one A tile for two MMAs, one 512-column accumulator drained
+    // once per unit) or the double-buffered 256 x 256 one (SPLAB_OZAKI_NT=1|2 overrides)
+    int nt = L.nt;
     if (const char* v = std::getenv("SPLAB_OZAKI_NT")) {
       if (v[0] == '1') nt = 1;
       if (v[0] == '2') nt = 2;
@@ -2983,11 +2942,8 @@ cudaError_t ozaki_gemm(const GemmProblem& p_in, int moduli, void* ws, size_t ws_
   ReconParams rp = make_recon(crt);
   rp.conj = p.opA == 2 ? 1 : 0;
   // threads along the rows of C, one block row covering all of them (no
-  // partial second pass), blocks along the columns (grid-stride beyond
-  // 65535); byte residues with m % 16 == 0 take the shared-memory staged
-  // kernel instead
+  // partial second pass), blocks along the columns (grid-stride beyond 65535)
   const int threads = 256;
-  const bool staged = R8 && L.rowsA % 16 == 0;
   const unsigned gy = unsigned(std::min<int64_t>(p.n, 65535));
   const unsigned gx = unsigned(std::max<int64_t>(1, (p.m + threads - 1) / threads));
   const bool fixed =
@@ -2998,43 +2954,9 @@ cudaError_t ozaki_gemm(const GemmProblem& p_in, int moduli, void* ws, size_t ws_
     phase_mark(2, true, st);
     return cudaGetLastError();
   }
-  if (staged) {
-    const int smem = staged_smem_bytes(L.nmod * L.nsub);
-    const int64_t items = (p.m + kStageRows - 1) / kStageRows * p.n;
-    const unsigned grid = unsigned(std::min<int64_t>(items, int64_t(2) * sm_count()));
-    auto run = [&](auto kern) -> cudaError_t {
-      const cudaError_t ea = set_dynamic_smem(reinterpret_cast<const void*>(kern), smem);
-      if (ea != cudaSuccess) return ea;
-      kern<<<grid, threads, smem, st>>>(R8, L.rowsA, int(p.n), L.nb, sigA, sigB, p.C, p.ldc,
-                                        p.alpha[0], p.alpha[1], p.beta[0], p.beta[1],
-                                        p.fill_mode, p.fill_ro, p.fill_co, BM,
-                                        cplx ? BN / 2 : BN, rp);
-      return cudaGetLastError();
-    };
-    switch (p.dtype) {
-      case kC64:
-        e = fixed ? run(oz_reconstruct_staged<kC64, kSplitCount>)
-                  : run(oz_reconstruct_staged<kC64, 0>);
-        break;
-      case kC32:
-        e = fixed ? run(oz_reconstruct_staged<kC32, kSplitCountFloat>)
-                  : run(oz_reconstruct_staged<kC32, 0>);
-        break;
-      case kR64:
-        e = fixed ? run(oz_reconstruct_staged<kR64, kDefaultModuli>)
-                  : run(oz_reconstruct_staged<kR64, 0>);
-        break;
-      default:
-        e = fixed ? run(oz_reconstruct_staged<kR32, kDefaultModuliFloat>)
-                  : run(oz_reconstruct_staged<kR32, 0>);
-        break;
-    }
-    if (e != cudaSuccess) return e;
-    phase_mark(2, true, st);
-    return cudaGetLastError();
-  }
   auto recon = [&](auto kern, const auto* Rsrc) {
-    kern<<<dim3(gx, gy), threads, 0, st>>>(Rsrc, L.rowsA, int(p.n), L.nb, sigA, sigB, p.C, p.ldc,
+    kern<<<dim3(gx, gy), threads, 0, st>>>(Rsrc, L.rowsA, int(p.n), L.planeR, L.ldR,
+                                           R8 ? L.nchunks : 1, sigA, sigB, p.C, p.ldc,
                                            p.alpha[0], p.alpha[1], p.beta[0], p.beta[1],
                                            p.fill_mode, p.fill_ro, p.fill_co, BM,
                                            cplx ? BN / 2 : BN, rp);
