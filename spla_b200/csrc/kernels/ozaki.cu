@@ -1892,11 +1892,20 @@ __global__ void __launch_bounds__(RT_THREADS, ReconCfg<KP>::CTAS)
 // --------------------------------------------------------------------------
 // host orchestration
 
-int sm_count() {
-  int dev = 0, v = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
-  return v;
+int sm_count() {  // read once per device
+  static int cached[64] = {0};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) {
+    cudaGetLastError();
+    return 148;
+  }
+  if (!cached[dev]) {
+    int v = 0;
+    if (cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || v < 2)
+      v = 148;
+    cached[dev] = v;
+  }
+  return cached[dev];
 }
 
 struct Layout {
@@ -1950,12 +1959,12 @@ size_t residue_bytes(const Layout& L, int rows) {
 // rate (0.44 us per 256 x 256 x 128, 8 % less in the wider tile, which loads A once
 // for two MMAs) and its hand-over (the wider tile's single accumulator exposes its
 // drain).
-double gemm_model_us(const Layout& L, int64_t m, int64_t n, int chunks, int nt) {
+double gemm_model_us(const Layout& L, int64_t m, int64_t n, int chunks, int nt, int pairs) {
   const double units = double(L.nmod * L.nsub) * chunks * double((m + 255) / 256) *
                        double((n + 256 * nt - 1) / (256 * nt));
   const double blocks = std::ceil(double(L.kp / BKB) / chunks);
   const double unit = nt == 2 ? blocks * 0.81 + 5.0 : blocks * 0.443 + 1.2;
-  return std::ceil(units / (sm_count() / 2)) * unit;
+  return std::ceil(units / pairs) * unit;
 }
 
 // k-chunks and tile width of the GEMM. Chunks stay within the exact INT32 bound;
@@ -1968,13 +1977,14 @@ void choose_gemm(Layout& L, int64_t m, int64_t n) {
   const int64_t blocks = L.kp / BKB, planes = L.nmod * L.nsub;
   const int64_t limit = L.split ? kChunkBlocksSplit : kChunkBlocks;
   const int least = int(std::max<int64_t>(1, (blocks + limit - 1) / limit));
+  const int pairs = std::max(1, sm_count() / 2);
   double best = 0.0;
   L.nchunks = 0;
   for (int c = least; c == least || (c <= blocks / 4 && c * planes <= RT_KP); ++c) {
     const double more = double(c - 1) * planes * m * n;  // bytes
     if (c > least && !L.split && more > kMoreChunksBytes) break;
     for (int nt = 1; nt <= (n >= 512 ? 2 : 1); ++nt) {
-      const double t = gemm_model_us(L, m, n, c, nt) + more / 2.5e6;
+      const double t = gemm_model_us(L, m, n, c, nt, pairs) + more / 2.5e6;
       if (L.nchunks == 0 || t < 0.97 * best) {
         best = t;
         L.nchunks = c;
@@ -2991,6 +3001,11 @@ cudaError_t ozaki_gemm(const GemmProblem& p_in, int moduli, void* ws, size_t ws_
   phase_mark(2, true, st);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   return cudaSuccess;
+}
+
+OzakiShape ozaki_shape(const GemmProblem& p) {
+  const oz::Layout L = oz::layout_of(p, 0);
+  return {oz::gemm_model_us(L, p.m, p.n, L.nchunks, L.nt, oz::sm_count() / 2) * 1e-6, L.r8};
 }
 
 int* ozaki_status_ptr(const GemmProblem& p, int moduli, void* ws) {

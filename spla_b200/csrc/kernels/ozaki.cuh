@@ -23,6 +23,14 @@ bool ozaki_supported(const GemmProblem& prob);
 // first copied k-major into the workspace.
 bool ozaki_copies_a(const GemmProblem& prob);
 
+// For path selection: modelled time of the INT8 GEMM, and whether the
+// reconstruction runs on the tensor cores.
+struct OzakiShape {
+  double gemm_seconds;
+  bool bytes;
+};
+OzakiShape ozaki_shape(const GemmProblem& prob);
+
 // Status word of the last ozaki_gemm on this workspace (synchronises
 // `stream`): 0 = ok, 1 = a bounded device wait gave up.
 int ozaki_status(const GemmProblem& prob, int moduli, void* workspace, cudaStream_t stream);

@@ -105,7 +105,12 @@ GemmProblem make_problem(int dtype, int opA, int opB, int64_t m, int64_t n, int6
 // norms' read at 6 TB/s, which rows of 131072 reals or more mostly skip: a
 // 1/16 sample), INT8 GEMM at 2.8 POP/s scaled by how evenly its work
 // units fill the 74 CTA pairs, reconstruction (3e-12 s per real output and
-// modulus) and 0.08 ms; 3xTF32 as splitting (bytes at 5.5 TB/s), three TF32
+// modulus on the CUDA cores; see ozaki_ms for the tensor cores) and 0.08 ms. The
+// CUDA-core rate alone, 90 ps per element of complex double, had kept tall products
+// of modest k on DMMA: 100000 x 512 x 512 took 6.3 ms, 3.0 on the Ozaki path, 50000 x
+// 2048 x 512 12.5 against 4.5. The slicing and three-product GEMM rates are those of
+// earlier kernels and now on the safe side: problems near the crossover stay where
+// they were. 3xTF32 as splitting (bytes at 5.5 TB/s), three TF32
 // products at 480 TFLOP/s scaled by the same fill, and 0.05 ms. The choice only
 // depends on the problem and the device (no free-memory query), so that
 // resolving a path, sizing its workspace and running it agree.
@@ -125,7 +130,8 @@ double dmma_ms(const GemmProblem& p) {
   return flops / (c ? 33e12 : 29e12) * 1e3 + 0.05;
 }
 
-double ozaki_ms(const GemmProblem& p) {
+// At least `most` is returned once the steps before the GEMM take that long.
+double ozaki_ms(const GemmProblem& p, double most) {
   const bool c = dtype_is_complex(p.dtype);
   const int nmod = dtype_is_double(p.dtype) ? 15 : 9;
   const double nsub = c ? 3.0 : 1.0;  // complex: three real products per modulus
@@ -144,13 +150,24 @@ double ozaki_ms(const GemmProblem& p) {
                        norm_rows(p.n, p.opB == 0);
   const double tiles = std::ceil(p.m / 256.0) * std::ceil(p.n / 256.0) * nsub;
   const double chunks = std::ceil(kp / 128.0 / 976.0);
+  if (slice * 1e3 + 0.08 >= most) return slice * 1e3 + 0.08;
   const double gemm = 2.0 * nmod * nsub * p.m * p.n * kp / (2.8e15 * fill(nmod * chunks * tiles));
-  const double recon = (c ? 3e-12 * 2.0 : 2e-12) * p.m * double(p.n) * nmod;
+  const double mn = p.m * double(p.n);
+  const double recon = (c ? 6e-12 : 2e-12) * mn * nmod;
   // op(A) = N beyond the in-place reach: A is first copied k-major (one read,
   // one write)
   const double transpose =
       ozaki_copies_a(p) ? 2.0 * p.m * K2 * (dtype_is_double(p.dtype) ? 8 : 4) / 6e12 : 0.0;
-  return (slice + gemm + recon + transpose) * 1e3 + 0.08;
+  const double t = slice + gemm + recon + transpose;
+  // Tall products of modest k spend their time per element of C: with the
+  // reconstruction on the tensor cores (20, 9.4, 14 and 9 ps for complex and real
+  // double and float) and the GEMM by its units (short k: hand-overs, partial tiles).
+  // Float types keep a tenth in reserve against 3xTF32, whose estimate is the closer.
+  const OzakiShape shape = ozaki_shape(p);
+  const bool dbl = dtype_is_double(p.dtype);
+  const double tall = slice + transpose + std::max(gemm, shape.gemm_seconds) +
+                      (dbl ? (c ? 20e-12 : 9.4e-12) : (c ? 14e-12 : 9e-12)) * mn;
+  return (shape.bytes ? std::min(t, tall * (dbl ? 1.0 : 1.1)) : t) * 1e3 + 0.08;
 }
 
 double tf32x3_ms(const GemmProblem& p) {
@@ -320,16 +337,17 @@ int resolve_path(const GemmProblem& p, int path, int moduli) {
   const double copyA = p.opA == 0 ? 2.0 * p.m * p.k * esz / 6e12 * 1e3 : 0.0;
   int best = SPLAB_PATH_DMMA;
   double best_ms = model::dmma_ms(p);
-  if (oz && path_workspace(p, SPLAB_PATH_OZAKI, moduli) <= cap) {
-    const double t = model::ozaki_ms(k_major_view(p, false));
-    if (t < 0.9 * best_ms) {
+  if (oz) {
+    const double t = model::ozaki_ms(k_major_view(p, false), 0.9 * best_ms);
+    if (t < 0.9 * best_ms && path_workspace(p, SPLAB_PATH_OZAKI, moduli) <= cap) {
       best = SPLAB_PATH_OZAKI;
       best_ms = t;
     }
   }
-  if (tf && path_workspace(p, SPLAB_PATH_TF32X3, moduli) <= cap) {
+  if (tf) {
     const double t = model::tf32x3_ms(k_major_view(p, true)) + copyB + copyA;
-    if (t < 0.9 * best_ms) best = SPLAB_PATH_TF32X3;
+    if (t < 0.9 * best_ms && path_workspace(p, SPLAB_PATH_TF32X3, moduli) <= cap)
+      best = SPLAB_PATH_TF32X3;
   }
   return best;
 }
