@@ -39,6 +39,7 @@ struct DmmaPlan {
   int bm, bn, splits;
   int64_t k_per_split;
   size_t workspace_bytes;
+  bool small;  // the 32 x 32 tile configuration
 };
 
 DmmaPlan dmma_plan(const GemmProblem& prob, int num_sms, int force_splits = 0);
