@@ -128,18 +128,37 @@ _DT_CODES = {"float32": 0, "float64": 1, "complex64": 2, "complex128": 3}
 _PREFIX = {0: "s", 1: "d", 2: "c", 3: "z"}
 
 
+_TORCH, _NUMPY = 1, 2
+_KIND = {}   # buffer type -> _TORCH or _NUMPY
+_CODE = {}   # dtype object -> code or None
+
+
+def _kind(x):
+    k = _KIND.get(type(x))
+    if k is None:
+        mod = type(x).__module__
+        if mod.startswith("torch"):
+            k = _TORCH
+        elif mod.startswith("numpy"):
+            k = _NUMPY
+        else:
+            raise TypeError(f"unsupported buffer type {type(x)}")
+        _KIND[type(x)] = k
+    return k
+
+
 def _addr(x):
     """(address, dtype code or None) of a torch tensor, numpy array, int or None."""
     if x is None:
         return None, None
     if isinstance(x, int):
         return x, None
-    mod = type(x).__module__
-    if mod.startswith("torch"):
-        return x.data_ptr(), _DT_CODES.get(str(x.dtype).replace("torch.", ""))
-    if mod.startswith("numpy"):
-        return x.ctypes.data, _DT_CODES.get(str(x.dtype))
-    raise TypeError(f"unsupported buffer type {type(x)}")
+    address = x.data_ptr() if _kind(x) == _TORCH else x.ctypes.data
+    dtype = x.dtype
+    code = _CODE.get(dtype, -1)
+    if code == -1:
+        code = _CODE[dtype] = _DT_CODES.get(str(dtype).replace("torch.", ""))
+    return address, code
 
 
 def _dtype_of(*bufs, dtype=None):
@@ -158,12 +177,18 @@ def _scalar(v, dt):
     if dt == 1:
         return ct.c_double(float(v.real if isinstance(v, complex) else v))
     v = complex(v)
-    arr = (ct.c_float * 2)(v.real, v.imag) if dt == 2 else (ct.c_double * 2)(v.real, v.imag)
-    return arr
+    return _C32x2(v.real, v.imag) if dt == 2 else _C64x2(v.real, v.imag)
 
 
-def _sarg(s, dt):
-    return s if dt in (0, 1) else ct.cast(s, ct.c_void_p)
+_C32x2, _C64x2 = ct.c_float * 2, ct.c_double * 2
+_FN = {}  # (name, dtype code) -> entry point
+
+
+def _entry(name, dt):
+    f = _FN.get((name, dt))
+    if f is None:
+        f = _FN[name, dt] = getattr(lib(), name.format(_PREFIX[dt]))
+    return f
 
 
 # ---------------------------------------------------------------------------
@@ -323,8 +348,8 @@ def pgemm_ssb(m, n, kLocal, opA, alpha, A, lda, B, ldb, beta, C, ldc, cRowOffset
     """C <- alpha op(A) B + beta C, stripe x stripe -> block (pgemm_ssb.hpp:88-117)."""
     dt = _dtype_of(C, A, B, dtype=dtype)
     a, b = _scalar(alpha, dt), _scalar(beta, dt)
-    check(getattr(lib(), f"spla_p{_PREFIX[dt]}gemm_ssb")(
-        m, n, kLocal, opA, _sarg(a, dt), _addr(A)[0], lda, _addr(B)[0], ldb, _sarg(b, dt),
+    check(_entry("spla_p{}gemm_ssb", dt)(
+        m, n, kLocal, opA, a, _addr(A)[0], lda, _addr(B)[0], ldb, b,
         _addr(C)[0], ldc, cRowOffset, cColOffset, distC.handle, ctx.handle))
 
 
@@ -333,8 +358,8 @@ def pgemm_ssbtr(m, n, kLocal, opA, alpha, A, lda, B, ldb, beta, C, ldc, cRowOffs
     """pgemm_ssb limited to a triangle of C (pgemm_ssbtr.hpp:94-126)."""
     dt = _dtype_of(C, A, B, dtype=dtype)
     a, b = _scalar(alpha, dt), _scalar(beta, dt)
-    check(getattr(lib(), f"spla_p{_PREFIX[dt]}gemm_ssbtr")(
-        m, n, kLocal, opA, _sarg(a, dt), _addr(A)[0], lda, _addr(B)[0], ldb, _sarg(b, dt),
+    check(_entry("spla_p{}gemm_ssbtr", dt)(
+        m, n, kLocal, opA, a, _addr(A)[0], lda, _addr(B)[0], ldb, b,
         _addr(C)[0], ldc, cRowOffset, cColOffset, cFillMode, distC.handle, ctx.handle))
 
 
@@ -343,17 +368,17 @@ def pgemm_sbs(mLocal, n, k, alpha, A, lda, B, ldb, bRowOffset, bColOffset, descB
     """C <- alpha A B + beta C, stripe x block -> stripe (pgemm_sbs.hpp:86-116)."""
     dt = _dtype_of(C, A, B, dtype=dtype)
     a, b = _scalar(alpha, dt), _scalar(beta, dt)
-    check(getattr(lib(), f"spla_p{_PREFIX[dt]}gemm_sbs")(
-        mLocal, n, k, _sarg(a, dt), _addr(A)[0], lda, _addr(B)[0], ldb, bRowOffset, bColOffset,
-        descB.handle, _sarg(b, dt), _addr(C)[0], ldc, ctx.handle))
+    check(_entry("spla_p{}gemm_sbs", dt)(
+        mLocal, n, k, a, _addr(A)[0], lda, _addr(B)[0], ldb, bRowOffset, bColOffset,
+        descB.handle, b, _addr(C)[0], ldc, ctx.handle))
 
 
 def gemm(opA, opB, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, ctx, dtype=None):
     """Local C <- alpha op(A) op(B) + beta C (gemm.hpp:66-97)."""
     dt = _dtype_of(C, A, B, dtype=dtype)
     a, b = _scalar(alpha, dt), _scalar(beta, dt)
-    check(getattr(lib(), f"spla_{_PREFIX[dt]}gemm")(
-        opA, opB, m, n, k, _sarg(a, dt), _addr(A)[0], lda, _addr(B)[0], ldb, _sarg(b, dt),
+    check(_entry("spla_{}gemm", dt)(
+        opA, opB, m, n, k, a, _addr(A)[0], lda, _addr(B)[0], ldb, b,
         _addr(C)[0], ldc, ctx.handle))
 
 

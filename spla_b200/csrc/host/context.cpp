@@ -142,6 +142,7 @@ ContextInternal::~ContextInternal() {
   host_.reset();
   for (auto& ev : events_)
     if (ev) cudaEventDestroy(ev);
+  if (status_) cudaFreeHost(status_);
   if (compute_) cudaStreamDestroy(compute_);
   if (copy_) cudaStreamDestroy(copy_);
   cudaSetDevice(prev);
@@ -161,6 +162,11 @@ cudaEvent_t ContextInternal::event(int i) {
   if (i < 0 || i >= 8) throw InternalError();
   if (!events_[i]) check_cuda(cudaEventCreateWithFlags(&events_[i], cudaEventDisableTiming));
   return events_[i];
+}
+
+int* ContextInternal::status_word() {
+  if (!status_) check_cuda(cudaMallocHost(&status_, sizeof(int)));
+  return status_;
 }
 
 // ---------------------------------------------------------------------------

@@ -19,6 +19,14 @@
 #include "../../../include/splab.h"
 #include "internal.hpp"
 
+namespace splab {
+// splab_api.cu: queue the copy of the status word of the last contraction on
+// `workspace` to `status` (page-locked; left alone on a path that keeps none).
+cudaError_t gemm_status_async(int dtype, int path, int opA, int opB, int64_t m, int64_t n,
+                              int64_t k, int moduli, void* workspace, int* status,
+                              cudaStream_t stream);
+}  // namespace splab
+
 namespace spla {
 
 namespace {
@@ -60,6 +68,18 @@ struct DeviceGuard {
   }
   ~DeviceGuard() { cudaSetDevice(prev); }
 };
+
+// Wait for the contraction on `st` and report a bounded device wait that gave up. The
+// status word comes with one copy behind the kernels, so that one wait does for
+// both.
+void finish(ContextInternal& ctx, int dtype, int path, int opA, int opB, int64_t m, int64_t n,
+            int64_t k, int moduli, void* ws, cudaStream_t st) {
+  int* status = ctx.status_word();
+  *status = 0;
+  check_cuda(splab::gemm_status_async(dtype, path, opA, opB, m, n, k, moduli, ws, status, st));
+  check_cuda(cudaStreamSynchronize(st));
+  if (*status) check_splab(SPLAB_ERR_TIMEOUT);
+}
 
 int path_for(const ContextInternal& ctx, int) { return ctx.fp64_path(); }
 
@@ -121,7 +141,7 @@ void local_gemm(ContextInternal& ctx, SplaOperation opA, SplaOperation opB, int 
     void* w = ws ? ctx.device_pool().get(1, ws) : nullptr;
     check_splab(splab_gemm(dtype, path, opA, opB, m, n, k, &alpha, A, lda, B, ldb, &beta, dC,
                            dldc, fill, ro, co, moduli, w, ws, cs));
-    check_splab(splab_gemm_check(dtype, path, opA, opB, m, n, k, moduli, w, cs));
+    finish(ctx, dtype, path, opA, opB, m, n, k, moduli, w, cs);
   } else {
     // Stream A and B in k-chunks: chunk c is copied on the copy stream into
     // buffer c % 2 while the compute stream contracts chunk c - 1; beta applies
@@ -182,14 +202,15 @@ void local_gemm(ContextInternal& ctx, SplaOperation opA, SplaOperation opB, int 
                              c == 0 ? &beta : &one, dC, dldc, fill, ro, co, moduli, w, ws, cs));
       check_cuda(cudaEventRecord(ctx.event(2 + b), cs));  // buffer b consumed
     }
-    check_splab(splab_gemm_check(dtype, path, opA, opB, m, n, klast, moduli, w, cs));
+    finish(ctx, dtype, path, opA, opB, m, n, klast, moduli, w, cs);
+    check_cuda(cudaStreamSynchronize(xs));
   }
 
-  if (!devC)
+  if (!devC) {
     check_cuda(cudaMemcpy2DAsync(C, size_t(ldc) * sizeof(T), dC, size_t(m) * sizeof(T),
                                  size_t(m) * sizeof(T), n, cudaMemcpyDefault, cs));
-  check_cuda(cudaStreamSynchronize(cs));
-  check_cuda(cudaStreamSynchronize(ctx.copy_stream()));
+    check_cuda(cudaStreamSynchronize(cs));
+  }
 }
 
 template void local_gemm<float>(ContextInternal&, SplaOperation, SplaOperation, int, int, int,

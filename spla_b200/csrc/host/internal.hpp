@@ -95,6 +95,9 @@ public:
   cudaStream_t compute_stream();
   cudaStream_t copy_stream();
   cudaEvent_t event(int i);
+  // One page-locked word for the device status of a contraction (not part of the
+  // pinned pool, whose size callers see).
+  int* status_word();
 
   // Contraction path for double / complex double: SPLAB_PATH_* (default
   // from SPLA_B200_PATH = auto | dmma | ozaki) and Ozaki modulus count.
@@ -116,6 +119,7 @@ private:
   std::unique_ptr<ScratchPool> host_, pinned_, device_;
   cudaStream_t compute_ = nullptr, copy_ = nullptr;
   cudaEvent_t events_[8] = {nullptr};
+  int* status_ = nullptr;
 };
 
 class MatrixDistributionInternal {

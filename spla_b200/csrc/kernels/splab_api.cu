@@ -443,6 +443,27 @@ struct BatchHandle {
 };
 
 }  // namespace
+
+cudaError_t gemm_status_async(int dtype, int path, int opA, int opB, int64_t m, int64_t n,
+                              int64_t k, int moduli, void* workspace, int* status,
+                              cudaStream_t stream) {
+  GemmProblem p{};
+  p.dtype = dtype;
+  p.opA = opA;
+  p.opB = opB;
+  p.m = m;
+  p.n = n;
+  p.k = k;
+  if (m <= 0 || n <= 0 || !workspace) return cudaSuccess;
+  const int rp = resolve_path(p, path, moduli);
+  if (rp != SPLAB_PATH_TF32X3 && rp != SPLAB_PATH_OZAKI) return cudaSuccess;
+  const Normalized N = normalize(p, rp);
+  char* pw = static_cast<char*>(workspace) + N.prefix;
+  const int* word = rp == SPLAB_PATH_TF32X3 ? tf32x3_status_ptr(N.p, pw)
+                                            : ozaki_status_ptr(N.p, moduli, pw);
+  return cudaMemcpyAsync(status, word, sizeof(int), cudaMemcpyDeviceToHost, stream);
+}
+
 }  // namespace splab
 
 using namespace splab;
