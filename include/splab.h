@@ -79,9 +79,9 @@ SPLAB_API size_t splab_gemm_workspace_size(int dtype, int path, int opA, int opB
  * (src/pgemm_ssb/pgemm_ssb_gpu.cpp:259-262, opA in {T,C}, opB = N) and
  * pgemm_sbs (src/pgemm_sbs/pgemm_sbs_gpu.cpp:246-249, N,N) reduce to, plus the
  * fill-mode tile skipping of pgemm_ssbtr (src/block_generation/block.hpp:58-66).
- * ozakiModuli: number of CRT moduli for SPLAB_PATH_OZAKI (0 = default: 15 for
- * double, <= 1e-14 relative error; 9 for float, ~1e-8; range 8..16); ignored
- * otherwise. A bounded device wait
+ * ozakiModuli: number of CRT moduli for SPLAB_PATH_OZAKI (0 = default, <= 1e-14
+ * relative error for double, ~1e-8 for float: 15 and 9 for the real types, 16 and
+ * 10 with -1 a square for the complex ones; range 8..16); ignored otherwise. A bounded device wait
  * that gives up makes the next splab_gemm_check() return SPLAB_ERR_TIMEOUT.
  */
 SPLAB_API int splab_gemm(int dtype, int path, int opA, int opB, int64_t m, int64_t n, int64_t k,
@@ -252,11 +252,10 @@ SPLAB_API int splab_gemm_dd(int dtype, int opA, int opB, int64_t m, int64_t n, i
  * caller) on its stream around phase p, for p < count:
  *   DMMA path : 0 = contraction kernel, 1 = split-K reduction
  *   Ozaki path: 0 = slicing, 1 = INT8 residue GEMMs, 2 = reconstruction,
- *               3 + g = GEMM launch of modulus group g; inside phase 0:
+ *               3 = the GEMM launch; inside phase 0:
  *               15 = k-major copy of A (op(A) = N with k too long to be read in
- *               place), 16 = row norms (of A, and
- *               of B unless they run on a side stream), 17 = residues of A,
- *               18 = residues of B (one modulus group)
+ *               place), 16 = row norms of A and B, 17 = residues of A,
+ *               18 = residues of B
  * Pass events = NULL to stop. Returns SPLAB_OK.
  */
 SPLAB_API int splab_set_phase_events(void **events, int count);

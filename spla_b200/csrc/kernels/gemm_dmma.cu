@@ -567,7 +567,7 @@ DmmaPlan dmma_plan(const GemmProblem& pr, int num_sms, int force_splits) {
   // 0.97 of the default tiles' rate: 1024 x 1024 x 4000 complex double 1059 against 1089
   // us; 129 x 129 x 30000 307 -> 229, 100 x 80 x 20000 110 -> 95, 33 x 500 x 5000 real
   // double 50 -> 40), and where the default plan has fewer CTAs than SMs and theirs
-  // finish sooner (64 x 64 x 64 complex double: one CTA 16.6 us, four 6.3)
+  // finish sooner (64 x 64 x 64 complex double: one CTA 16.6 us, four 7.6)
   const int64_t def_tiles = tiles(def.bm, def.bn);
   const bool padded = double(def_tiles) * def.bm * def.bn >= 1.15 * 1024.0 * double(tiles(32, 32));
   if (!padded && def_tiles * def.splits >= num_sms) return def;

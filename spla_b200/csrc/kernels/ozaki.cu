@@ -2344,7 +2344,7 @@ void launch_slice_mn(int ndig, cudaStream_t st, const TIn* X, int64_t ld, int m,
 // full loads of the GPU, slices of at least 32 elements (a thread's loads go out in
 // batches of 8), at most 4096 (the grid's y extent). The partial sums lie where
 // the operand's residues go next. Slices of 512 elements and more had left a 1501
-// x 1207 operand with 24 blocks (39.8 us; now 5.6).
+// x 1207 operand with 24 blocks (39.8 us; now 9.6).
 int in_place_slices(int64_t rows, int64_t k) {
   if (rows >= oz::kMnRows) return 1;
   const int64_t want = (int64_t(oz::sm_count()) * 4096 + rows - 1) / rows;
@@ -2530,7 +2530,7 @@ void slice_operands(const oz::Layout& L, const oz::Crt& crt, const GemmProblem& 
 //
 // It pays from about 256 MB of k-major operands: the norms' second read (6 TB/s)
 // against the sample and two more launches (387 x 515 x 60013 complex double, 866
-// MB: 150 us of norms, 27 us of estimates and checks); rows of 16384 reals keep 64
+// MB: 150 us of norms, 30 us of estimates and checks); rows of 16384 reals keep 64
 // reals per run. Rows of 131072 reals always take it.
 constexpr int64_t kOnePassMinLen = 16384, kOnePassLongLen = 131072;
 constexpr double kOnePassMinBytes = 256e6;
@@ -2667,7 +2667,7 @@ void onepass_fixup(const oz::Layout& L, const oz::Crt& crt, const GemmProblem& p
 // residues (at most 64 planes over all k-chunks); SPLAB_OZAKI_RECON_TC=0 (read per
 // call) selects the CUDA-core kernel, as do int32 sums. Columns padded to 16 bytes
 // let every m take it: 1501 x 2003 real double 76 us on the CUDA cores (uncoalesced
-// bytes of 15 planes), 31 us here. True when it applies and its tensor map was made.
+// bytes of 15 planes), 32 us here. True when it applies and its tensor map was made.
 bool recon_tc_plan(const oz::Layout& L, unsigned char* R8, CUtensorMap* map) {
   const char* v = std::getenv("SPLAB_OZAKI_RECON_TC");
   if ((v && v[0] == '0') || !R8) return false;

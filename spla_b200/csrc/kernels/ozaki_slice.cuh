@@ -15,7 +15,7 @@
 // instructions per element, its FMA pipe 62 % and issue slots 67 % busy, against
 // about 170 here. m = n = 1024, k = 60000: 1.49 -> 1.16 ms for both operands (5.1
 // TB/s read and written); k = 250000, with the sums of squares of the one-pass
-// scaling, 7.3 -> 5.9 ms. It stays for the other types and for operands read in
+// scaling, 7.3 -> 5.6 ms. It stays for the other types and for operands read in
 // place, where it measured the same or faster (real double 1.11 against 1.14 ms
 // at k = 100000; complex float 1.08 against 1.18 at 60000, where five of its 8
 // digits would do; real float 0.63 against 1.07, 18 of 32 rows used; m-major
