@@ -57,7 +57,9 @@ def set_shape(m, k):
     M = N = m
     K = k
     FLOPS = 8.0 * M * N * K
-OZAKI_MODULI = 15  # default modulus count of the library (<= 1e-14 at this k)
+# residue planes per operand of a complex double call with the default moduli: two real
+# products for each of 16 moduli (<= 1e-14 at this k)
+OZAKI_PLANES = 32
 HEADLINE_METRIC = "ZGEMM-SSB TFLOP/s: Ozaki-INT8 vs FP64-DMMA at ≤1e-14 rel err, 1 B200"
 
 
@@ -1120,35 +1122,33 @@ def main():
     else:
         gemm_launch_ms = hr["phase_ms"][3:]
         k_ms = sum(gemm_launch_ms) or hr["phase_ms"][1] or hr["ms_per_step"]
-        nmod = OZAKI_MODULI
-        # residue GEMMs: three real products of m x n x k per modulus (complex)
-        int8_ops = 2.0 * nmod * 3 * M * N * K
+        # residue GEMMs: one real product of m x n x k per plane
+        int8_ops = 2.0 * OZAKI_PLANES * M * N * K
         achieved = int8_ops / (k_ms / 1e3) / 1e12
         peak = peaks.get("int8_tops")
-        # DRAM bytes of one GEMM launch: 1.286 x the algorithmic residue bytes, the ratio of
+        # DRAM bytes of one GEMM launch: 1.136 x the algorithmic residue bytes, the ratio of
         # an ncu capture of oz_gemm_pair on the same tiling with a shorter k (m = n = 1024,
-        # k = 40000: 4.745 GB for 3.692 GB of residues), scaled by the k-blocks processed
-        alg_bytes = float(OZAKI_MODULI) * 3 * (M + N) * ((K + 127) // 128 * 128)
-        traffic = 1.286 * alg_bytes if (M, N) == (1024, 1024) else None
+        # k = 40000: 2.982 GB for 2.626 GB of residues), scaled by the k-blocks processed
+        alg_bytes = float(OZAKI_PLANES) * (M + N) * ((K + 127) // 128 * 128)
+        traffic = 1.136 * alg_bytes if (M, N) == (1024, 1024) else None
         roof = {"bound": "tensor", "achieved": achieved, "peak": peak, "unit": "TOP/s (int8)",
                 "frac": (achieved / peak) if peak else None, "traffic": traffic,
                 "traffic_source": "ncu dram__bytes_{read,write}.sum of oz_gemm_pair on "
-                                  "m=n=1024 k=40000 (same tiles, one k-chunk), 1.286 x the "
+                                  "m=n=1024 k=40000 (same tiles), 1.136 x the "
                                   "residue bytes, scaled to this launch by its k-blocks "
                                   "(profiles/oz_gemm_pair_int8_traffic_zgemm_m1024_k40000.md)",
-                "algorithmic_residue_bytes": float(OZAKI_MODULI) * 3 * (M + N) * K,
+                "algorithmic_residue_bytes": float(OZAKI_PLANES) * (M + N) * K,
                 "kernel": "oz_gemm_pair (tcgen05.mma.cta_group::2.kind::i8, TMA, TMEM)",
                 "peak_source": "measured here: cuBLASLt int8 GEMM 8192^3 via torch._int_mm",
                 "algorithmic_ops_per_launch": int8_ops}
-        groups = max(1, len(gemm_launch_ms))
-        # 2 row-scale, 2 slice and 1 GEMM per modulus group, 1 reconstruct
-        launches = (3 + 3 * groups) * args.steps
-        roof["gemm_launches_per_step"] = groups
-        roof["note"] = ("achieved = INT8 ops / summed duration of the GEMM launches; with "
-                        "modulus groups those launches overlap the slicing of the next group")
+        # row scales of both operands, two slicers, GEMM, reconstruction; with the one-pass
+        # scaling (rows of 131072 reals and more) also the check and two fix-up slicers
+        launches = (8 if 2 * K >= 131072 else 5) * args.steps
+        roof["gemm_launches_per_step"] = 1
+        roof["note"] = "achieved = INT8 ops / duration of the GEMM launch"
         hr["phase_ms"] = hr["phase_ms"][:3] + gemm_launch_ms
         hr["phase_ms_names"] = (["scale+slice (span)", "int8 GEMM (span)", "reconstruct"] +
-                                [f"int8 GEMM group {i}" for i in range(len(gemm_launch_ms))])
+                                ["int8 GEMM launch"] * len(gemm_launch_ms))
 
     cpu = None
     if not args.no_cpu and world >= 1:

@@ -13,7 +13,7 @@
 //
 // oz_slice (ozaki.cu) forms the digit sums as FP32 chains instead: 305
 // instructions per element, its FMA pipe 62 % and issue slots 67 % busy, against
-// about 170 here. m = n = 1024, k = 60000: 1.49 -> 1.16 ms for both operands (5.1
+// 193 here (with the sums of squares). m = n = 1024, k = 60000: 1.49 -> 1.16 ms for both operands (5.1
 // TB/s read and written); k = 250000, with the sums of squares of the one-pass
 // scaling, 7.3 -> 5.6 ms. It stays for the other types and for operands read in
 // place, where it measured the same or faster (real double 1.11 against 1.14 ms
