@@ -55,7 +55,11 @@ constexpr int STAGE_BYTES = 2 * A_PLANE + 2 * B_PLANE;  // A_hi, A_lo, B_hi, B_l
 constexpr int STAGES = 4;
 constexpr int kWin = 2;                 // k-blocks per FP32 accumulation window
 constexpr int kFold = 4;                // windows per register sum before the 2Sum fold
-constexpr int kMinSuperBlocks = 64;     // smallest k extent of a work unit (2048 reals)
+// Smallest k extent of a work unit, 1024 reals: few tiles need many splits to fill the
+// CTA pairs, and an FP64 partial of a tile costs little. With 2048 reals complex 256 x
+// 256 x 8192 took 117 us (93 now), 128 x 128 x 16384 116 (93), real 256 x 256 x 16384
+// 109 (84); with 1536 reals 106, 105 and 96.
+constexpr int kMinSuperBlocks = 32;
 constexpr int THREADS = 320;            // warp 0 TMA, warp 1 MMA, warps 2-9 epilogue
 constexpr int SMEM = STAGES * STAGE_BYTES + 2048;
 constexpr unsigned long long kWaitLimitNs = 2000000000ull;
