@@ -14,10 +14,13 @@
 // contraction on the compute stream, instead of being copied on the stream
 // that consumes them (src/gpu_util/multiply_gpu.cpp:101-142).
 #include <algorithm>
+#include <complex>
 #include <cstring>
+#include <type_traits>
 
 #include "../../../include/splab.h"
 #include "internal.hpp"
+#include "stream_chunks.hpp"
 
 namespace splab {
 // splab_api.cu: queue the copy of the status word of the last contraction on
@@ -149,15 +152,9 @@ void local_gemm(ContextInternal& ctx, SplaOperation opA, SplaOperation opB, int 
     const bool akm = opA != SPLA_OP_NONE;  // A is k x m (k contiguous)
     const bool bkm = opB == SPLA_OP_NONE;  // B is k x n (k contiguous)
     const int64_t edge = std::max(64, ctx.tile_size_gpu());
-    int64_t kc = std::max<int64_t>(256, (edge * edge * 4) / std::max(1, std::max(m, n)));
-    // at least eight chunks, of 16 MB or more: only the last one's contraction is not
-    // hidden behind a copy (m = n = 256, k = 50000 complex double had been one chunk:
-    // 7.45 ms of copies, then 0.8 ms of contraction)
     const int64_t row_bytes = int64_t(sizeof(T)) * ((devA ? 0 : m) + (devB ? 0 : n));
-    kc = std::min(kc, std::max<int64_t>((k + 7) / 8, ((int64_t(16) << 20) + row_bytes - 1) / row_bytes));
-    kc = std::min<int64_t>(kc, k);
-    kc = (kc + 63) / 64 * 64;
-    if (kc > k) kc = k;
+    const bool fp64 = std::is_same<T, double>::value || std::is_same<T, std::complex<double>>::value;
+    const int64_t kc = stream_chunk(m, n, k, edge, row_bytes, fp64);
     const int64_t chunks = (k + kc - 1) / kc;
     const size_t abytes = sizeof(T) * size_t(kc) * m, bbytes = sizeof(T) * size_t(kc) * n;
     T* bufA[2] = {nullptr, nullptr};
