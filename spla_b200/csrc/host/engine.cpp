@@ -154,7 +154,8 @@ void local_gemm(ContextInternal& ctx, SplaOperation opA, SplaOperation opB, int 
     const int64_t edge = std::max(64, ctx.tile_size_gpu());
     const int64_t row_bytes = int64_t(sizeof(T)) * ((devA ? 0 : m) + (devB ? 0 : n));
     const bool fp64 = std::is_same<T, double>::value || std::is_same<T, std::complex<double>>::value;
-    const int64_t kc = stream_chunk(m, n, k, edge, row_bytes, fp64);
+    const int64_t c_bytes = int64_t(sizeof(T)) * m * n;
+    const int64_t kc = stream_chunk(m, n, k, edge, row_bytes, c_bytes, fp64);
     const int64_t chunks = (k + kc - 1) / kc;
     const size_t abytes = sizeof(T) * size_t(kc) * m, bbytes = sizeof(T) * size_t(kc) * n;
     T* bufA[2] = {nullptr, nullptr};

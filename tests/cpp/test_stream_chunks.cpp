@@ -24,16 +24,20 @@ int main() {
         for (int64_t elem : {4, 8, 16}) {
           const int64_t most = longest_chunk(m, n, k, edge);
           for (bool fp64 : {false, true}) {
-            const int64_t kc = stream_chunk(m, n, k, edge, elem * (m + n), fp64);
+            const int64_t c_bytes = elem * m * n;
+            const int64_t kc = stream_chunk(m, n, k, edge, elem * (m + n), c_bytes, fp64);
             CHECK(kc >= 1 && kc <= most && most <= k);
             CHECK(kc == k || kc % 64 == 0);
             // a float C is rounded once per chunk: no more chunks than the buffers need
             if (!fp64) CHECK(kc == most);
+            // every chunk passes over C: a cut one brings as many bytes
+            if (kc < most) CHECK(kc * elem * (m + n) >= c_bytes);
           }
         }
   // one copy in eight is not hidden
-  CHECK(stream_chunk(256, 256, 50000, edge, 16 * 512, true) == 6272);
-  CHECK(stream_chunk(256, 256, 50000, edge, 8 * 512, false) == 50000);
+  CHECK(stream_chunk(256, 256, 50000, edge, 16 * 512, 16 * 65536, true) == 6272);
+  CHECK(stream_chunk(256, 256, 50000, edge, 8 * 512, 8 * 65536, false) == 50000);
+  CHECK(stream_chunk(8192, 8192, 512, edge, 16 * 16384, int64_t(16) << 26, true) == 512);
   std::printf(failures ? "FAILED\n" : "OK\n");
   return failures != 0;
 }
