@@ -153,8 +153,12 @@ void local_gemm(ContextInternal& ctx, SplaOperation opA, SplaOperation opB, int 
     const bool bkm = opB == SPLA_OP_NONE;  // B is k x n (k contiguous)
     const int64_t edge = std::max(64, ctx.tile_size_gpu());
     const int64_t row_bytes = int64_t(sizeof(T)) * ((devA ? 0 : m) + (devB ? 0 : n));
-    const bool fp64 = std::is_same<T, double>::value || std::is_same<T, std::complex<double>>::value;
     const int64_t c_bytes = int64_t(sizeof(T)) * m * n;
+    // the path of the longest chunk, however short the chunks are
+    const int path = splab_gemm_path(dtype, path_pref, opA, opB, m, n,
+                                     longest_chunk(m, n, k, edge));
+    const bool fp64 = path == SPLAB_PATH_DMMA && (std::is_same<T, double>::value ||
+                                                  std::is_same<T, std::complex<double>>::value);
     const int64_t kc = stream_chunk(m, n, k, edge, row_bytes, c_bytes, fp64);
     const int64_t chunks = (k + kc - 1) / kc;
     const size_t abytes = sizeof(T) * size_t(kc) * m, bbytes = sizeof(T) * size_t(kc) * n;
@@ -165,7 +169,6 @@ void local_gemm(ContextInternal& ctx, SplaOperation opA, SplaOperation opB, int 
       if (!devB) bufB[b] = static_cast<T*>(ctx.device_pool().get(4 + b, bbytes));
     }
     const int64_t klast = k - (chunks - 1) * kc;
-    const int path = splab_gemm_path(dtype, path_pref, opA, opB, m, n, kc);
     const size_t ws =
         std::max(splab_gemm_workspace_size(dtype, path, opA, opB, m, n, kc, moduli),
                  splab_gemm_workspace_size(dtype, path, opA, opB, m, n, klast, moduli));

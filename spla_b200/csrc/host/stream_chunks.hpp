@@ -20,14 +20,16 @@ inline int64_t longest_chunk(int64_t m, int64_t n, int64_t k, int64_t edge) {
 }
 
 // Chunk of the call. Only the last chunk's contraction is not hidden behind a copy, so
-// calls are cut into at least eight chunks, of 16 MB or more (m = n = 256, k = 50000
-// complex double as one chunk: 7.45 ms of copies, then 0.8 ms of contraction). C takes
-// each chunk's product in its own type: FP64 sums stay FP64 sums, but a `float` C would
-// round up to eight times instead of once (128 x 128 x 40000 float, relative to 64 bits:
-// 2.5e-8 as one chunk, 3.8e-8 as eight; 1.6e-4 where the chunks cancel), so the float
-// types keep the longest chunk. A chunk brings no fewer bytes than C has, since each
-// one's contraction reads and writes all of C (8192 x 8192 x 512 complex double: 5.9 ms
-// as one chunk, 15.8 in chunks of 64 rows). row_bytes: bytes copied per row of k.
+// calls whose products are summed in FP64 and stored as FP64 (`fp64`: DMMA with a double
+// type) are cut into at least eight chunks, of 16 MB or more (m = n = 256, k = 50000
+// complex double: 8.3 ms as one chunk, 7.6). Others keep the longest chunk, since C
+// takes each chunk's product in its own type: a float C would round eight times instead
+// of once (128 x 128 x 40000 float, relative to 64 bits: 2.5e-8 as one chunk, 3.8e-8 as
+// eight; 1.6e-4 where the chunks cancel), and the Ozaki path's sums, good to 2^-57 of
+// the rows' norms, would round to C's 2^-53 at every chunk (1024 x 1024 x 16000 complex
+// double 10.25 ms, 9.74 in eight). A chunk brings no fewer bytes than C has, since each
+// one's contraction reads and writes all of C (8192 x 8192 x 512 complex double: 5.2 ms
+// as one chunk, 15.6 in chunks of 64 rows). row_bytes: bytes copied per row of k.
 inline int64_t stream_chunk(int64_t m, int64_t n, int64_t k, int64_t edge, int64_t row_bytes,
                             int64_t c_bytes, bool fp64) {
   const int64_t most = longest_chunk(m, n, k, edge);

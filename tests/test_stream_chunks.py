@@ -35,13 +35,7 @@ def _cancelling(dt, rows, k, ld, seed):
     return A, B + 1e-3 * torch.randn(B.shape, dtype=A.dtype, device="cuda", generator=g)
 
 
-@pytest.mark.gpu
-@pytest.mark.parametrize("dt", ["float32", "complex64"])
-@pytest.mark.parametrize("path", [0, 1, 2, 3], ids=["auto", "dmma", "ozaki", "tf32x3"])
-@pytest.mark.parametrize("m,k,pad", [(128, 40000, 0), (70, 20001, 3)])
-def test_float_results_of_host_operands_are_those_of_device_operands(dt, path, m, k, pad):
-    """One chunk holds all of k: the same kernels on the same values, so C is
-    bit-identical to the call on device operands (rounded to float once)."""
+def _host_and_device_results(dt, path, m, k, pad):
     import torch
     import spla_b200 as spla
     A, B = _cancelling(dt, m, k, k + pad, m)
@@ -56,4 +50,55 @@ def test_float_results_of_host_operands_are_those_of_device_operands(dt, path, m
         spla.gemm(op, 0, m, m, k, 1.0, a, k + pad, b, k + pad, 0.0, C, m, ctx)
         torch.cuda.synchronize()
         out.append(C.cpu())
-    assert torch.equal(*out)
+    return out
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dt", ["float32", "complex64"])
+@pytest.mark.parametrize("path", [0, 1, 2, 3], ids=["auto", "dmma", "ozaki", "tf32x3"])
+@pytest.mark.parametrize("m,k,pad", [(128, 40000, 0), (70, 20001, 3)])
+def test_float_results_of_host_operands_are_those_of_device_operands(dt, path, m, k, pad):
+    """One chunk holds all of k: the same kernels on the same values, so C is
+    bit-identical to the call on device operands (rounded to float once)."""
+    import torch
+    assert torch.equal(*_host_and_device_results(dt, path, m, k, pad))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dt", ["float64", "complex128"])
+@pytest.mark.parametrize("m,k,pad", [(64, 40000, 0), (130, 30001, 3)])
+def test_ozaki_results_of_host_operands_are_those_of_device_operands(dt, m, k, pad):
+    """The same for the Ozaki path with the double types (rounded at C's last
+    bit once, not once per chunk)."""
+    import torch
+    assert torch.equal(*_host_and_device_results(dt, 2, m, k, pad))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dt,m,n,k", [("complex128", 320, 320, 40960), ("complex128", 400, 300, 40000),
+                                      ("float64", 700, 700, 22000)])
+def test_host_operands_take_the_path_of_device_operands(dt, m, n, k):
+    """AUTO resolves on all of k, not on the chunks it is cut into: the Ozaki path's
+    slicing events (17) are recorded after a marker set before the call."""
+    import ctypes as ct
+    import torch
+    import spla_b200 as spla
+    code = {"float64": 1, "complex128": 3}[dt]
+    op = 2 if dt == "complex128" else 1
+    L = spla.lib()
+    assert L.splab_gemm_path(code, spla.PATH_AUTO, op, 0, m, n, k) == spla.PATH_OZAKI
+    A = torch.randn((m, k), dtype=getattr(torch, dt)).pin_memory()
+    B = torch.randn((n, k), dtype=A.dtype).pin_memory()
+    C = torch.zeros((n, m), dtype=A.dtype).pin_memory()
+    nphase = 20
+    ev = [torch.cuda.Event(enable_timing=True) for _ in range(2 * nphase + 1)]
+    for e in ev:
+        e.record()
+    torch.cuda.synchronize()
+    ctx = spla.Context(spla.PU_GPU)
+    L.splab_set_phase_events((ct.c_void_p * (2 * nphase))(*[e.cuda_event for e in ev[:-1]]), nphase)
+    try:
+        spla.gemm(op, 0, m, n, k, 1.0, A, k, B, k, 0.0, C, m, ctx)
+    finally:
+        L.splab_set_phase_events(None, 0)
+    assert ev[-1].elapsed_time(ev[35]) > 0.0
