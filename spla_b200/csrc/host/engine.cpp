@@ -23,8 +23,8 @@
 #include "stream_chunks.hpp"
 
 namespace splab {
-// splab_api.cu: queue the copy of the status word of the last contraction on
-// `workspace` to `status` (page-locked; left alone on a path that keeps none).
+// splab_api.cu: queue the check of the status word of the last contraction on
+// `workspace`: *status (page-locked) is set to 1 if it is set, else left alone.
 cudaError_t gemm_status_async(int dtype, int path, int opA, int opB, int64_t m, int64_t n,
                               int64_t k, int moduli, void* workspace, int* status,
                               cudaStream_t stream);
@@ -72,14 +72,10 @@ struct DeviceGuard {
   ~DeviceGuard() { cudaSetDevice(prev); }
 };
 
-// Wait for the contraction on `st` and report a bounded device wait that gave up. The
-// status word comes with one copy behind the kernels, so that one wait does for
-// both.
-void finish(ContextInternal& ctx, int dtype, int path, int opA, int opB, int64_t m, int64_t n,
-            int64_t k, int moduli, void* ws, cudaStream_t st) {
-  int* status = ctx.status_word();
-  *status = 0;
-  check_cuda(splab::gemm_status_async(dtype, path, opA, opB, m, n, k, moduli, ws, status, st));
+// Wait for the contractions on `st` and report a bounded device wait that gave up in any
+// of them: the check of each one's status word is queued behind it, so that one wait
+// does for all.
+void finish(const int* status, cudaStream_t st) {
   check_cuda(cudaStreamSynchronize(st));
   if (*status) check_splab(SPLAB_ERR_TIMEOUT);
 }
@@ -122,6 +118,9 @@ void local_gemm(ContextInternal& ctx, SplaOperation opA, SplaOperation opB, int 
   const int moduli = ctx.ozaki_moduli();
   cudaStream_t cs = ctx.compute_stream();
 
+  int* status = ctx.status_word();
+  *status = 0;
+
   const bool devA = k == 0 || is_device_pointer(A);
   const bool devB = k == 0 || is_device_pointer(B);
   const bool devC = is_device_pointer(C);
@@ -144,7 +143,9 @@ void local_gemm(ContextInternal& ctx, SplaOperation opA, SplaOperation opB, int 
     void* w = ws ? ctx.device_pool().get(1, ws) : nullptr;
     check_splab(splab_gemm(dtype, path, opA, opB, m, n, k, &alpha, A, lda, B, ldb, &beta, dC,
                            dldc, fill, ro, co, moduli, w, ws, cs));
-    finish(ctx, dtype, path, opA, opB, m, n, k, moduli, w, cs);
+    check_cuda(
+        splab::gemm_status_async(dtype, path, opA, opB, m, n, k, moduli, w, status, cs));
+    finish(status, cs);
   } else {
     // Stream A and B in k-chunks: chunk c is copied on the copy stream into
     // buffer c % 2 while the compute stream contracts chunk c - 1; beta applies
@@ -206,9 +207,12 @@ void local_gemm(ContextInternal& ctx, SplaOperation opA, SplaOperation opB, int 
       check_cuda(cudaStreamWaitEvent(cs, ctx.event(b), 0));
       check_splab(splab_gemm(dtype, path, opA, opB, m, n, kcur, &alpha, pa, la, pb, lb,
                              c == 0 ? &beta : &one, dC, dldc, fill, ro, co, moduli, w, ws, cs));
+      // each contraction clears the word of the one before
+      check_cuda(
+          splab::gemm_status_async(dtype, path, opA, opB, m, n, kcur, moduli, w, status, cs));
       check_cuda(cudaEventRecord(ctx.event(2 + b), cs));  // buffer b consumed
     }
-    finish(ctx, dtype, path, opA, opB, m, n, klast, moduli, w, cs);
+    finish(status, cs);
     check_cuda(cudaStreamSynchronize(xs));
   }
 

@@ -2878,8 +2878,9 @@ cudaError_t ozaki_gemm(const GemmProblem& p_in, int moduli, void* ws, size_t ws_
     g.stall_test = 0;
     if (const char* v = std::getenv("SPLAB_OZAKI_STALL_TEST")) {
       // test hook for the failure path: no copies are issued, every wait runs
-      // into a 50 ms bound, the kernel reports SPLAB_ERR_TIMEOUT and returns
-      if (v[0] == '1') {
+      // into a 50 ms bound, the kernel reports SPLAB_ERR_TIMEOUT and returns ("2": only
+      // calls with beta = 0, such as the first k-chunk of streamed operands)
+      if (v[0] == '1' || (v[0] == '2' && p.beta[0] == 0.0 && p.beta[1] == 0.0)) {
         g.stall_test = 1;
         g.wait_limit_ns = 50000000ull;
       }

@@ -436,6 +436,12 @@ void block_cyclic_info_host(int64_t rb, int64_t cb, int64_t gr, int64_t gc, int6
   o[8] = (gbRow % gr) + (gbCol % gc) * gr;
 }
 
+// Sets *status (page-locked host memory) when a contraction left its status word set;
+// never clears it, so one word does for a sequence of contractions.
+__global__ void note_status(const int* word, int* status) {
+  if (*word) *status = 1;
+}
+
 // A batch plan: the grouped FP64 launch or a tensor-core sequence.
 struct BatchHandle {
   BatchPlanImpl* grouped = nullptr;
@@ -461,7 +467,8 @@ cudaError_t gemm_status_async(int dtype, int path, int opA, int opB, int64_t m, 
   char* pw = static_cast<char*>(workspace) + N.prefix;
   const int* word = rp == SPLAB_PATH_TF32X3 ? tf32x3_status_ptr(N.p, pw)
                                             : ozaki_status_ptr(N.p, moduli, pw);
-  return cudaMemcpyAsync(status, word, sizeof(int), cudaMemcpyDeviceToHost, stream);
+  note_status<<<1, 1, 0, stream>>>(word, status);
+  return cudaGetLastError();
 }
 
 }  // namespace splab

@@ -1,8 +1,10 @@
 """Host-resident operands, streamed in k-chunks: the chunk rule on the CPU
 (tests/cpp/test_stream_chunks.cpp), and what the chunks may not change in the
 result on the GPU."""
+import os
 import shutil
 import subprocess
+import sys
 from pathlib import Path
 
 import pytest
@@ -102,3 +104,33 @@ def test_host_operands_take_the_path_of_device_operands(dt, m, n, k):
     finally:
         L.splab_set_phase_events(None, 0)
     assert ev[-1].elapsed_time(ev[35]) > 0.0
+
+
+@pytest.mark.gpu
+def test_a_wait_that_gives_up_in_an_early_chunk_is_reported():
+    """The test hook lets the bounded waits of the first of eight chunks run out
+    (50 ms; no copies are issued): the call reports it although the later chunks,
+    whose contractions clear the status word, succeed."""
+    code = r"""
+import sys, torch
+sys.path.insert(0, %r)
+import spla_b200 as spla
+m, n, k = 64, 64, 2000
+A = torch.randn(m * k, dtype=torch.complex128).pin_memory()
+B = torch.randn(n * k, dtype=torch.complex128).pin_memory()
+C = torch.zeros(m * n, dtype=torch.complex128, device='cuda')
+ctx = spla.Context(spla.PU_GPU)
+ctx.set_fp64_path(spla.PATH_OZAKI)
+ctx.set_tile_size_gpu(64)  # chunks of 256
+try:
+    spla.gemm(2, 0, m, n, k, 1.0, A, k, B, k, 0.0, C, m, ctx)
+    print('NO_ERROR')
+except spla.GPULaunchError:
+    print('TIMEOUT_REPORTED')
+spla.gemm(2, 0, m, n, k, 1.0, A, k, B, k, 1.0, C, m, ctx)  # no stall with beta = 1
+print('CONTEXT_OK')
+""" % str(HERE.parent)
+    env = dict(os.environ, SPLAB_OZAKI_STALL_TEST="2")
+    out = subprocess.run([sys.executable, "-c", code], env=env, capture_output=True, text=True,
+                         timeout=300)
+    assert "TIMEOUT_REPORTED" in out.stdout and "CONTEXT_OK" in out.stdout, out.stdout + out.stderr
