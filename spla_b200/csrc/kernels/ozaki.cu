@@ -177,16 +177,16 @@ __device__ __forceinline__ void ssq_row(const TIn* __restrict__ x, int64_t len, 
   }
 }
 
-// Sum of squares of a sample of a row: nruns runs of run reals, gap apart;
-// blockDim.x / nruns threads per run (blockDim.x a multiple of nruns),
-// batches of 8 independent loads along it (the runs are short).
+// Sums of squares of a sample of a row: kRuns runs of run reals, gap apart, each the
+// sum (S, E) of 16 consecutive threads of the block's 256, in batches of 8
+// independent loads (the runs are short).
+constexpr int kRuns = 16;
 template <typename TIn>
-__device__ __forceinline__ void ssq_sample(const TIn* __restrict__ x, int nruns, int64_t run,
-                                           int64_t gap, double& S, int& E, double& inv) {
-  const int gsz = int(blockDim.x) / nruns;
-  const int c = int(threadIdx.x) / gsz;
-  if (c >= nruns) return;
-  x += c * gap;
+__device__ __forceinline__ void ssq_sample(const TIn* __restrict__ x, int64_t run, int64_t gap,
+                                           double& S, int& E, double& inv) {
+  constexpr int gsz = 256 / kRuns;
+  static_assert(gsz == 16, "a half warp per run");
+  x += int(threadIdx.x) / gsz * gap;
   for (int64_t l = threadIdx.x % gsz; l < run; l += 8 * gsz) {
     double v[8];
 #pragma unroll
@@ -204,6 +204,37 @@ __device__ __forceinline__ void ssq_sample(const TIn* __restrict__ x, int nruns,
       const double w = v[b] * inv;
       S = fma(w, w, S);
     }
+  }
+  for (int o = gsz / 2; o > 0; o >>= 1) {
+    const double S2 = __shfl_xor_sync(0xffffffffu, S, o);
+    const int E2 = __shfl_xor_sync(0xffffffffu, E, o);
+    scaled_add(S, E, S2, E2);
+  }
+}
+
+// The runs' sums (ssq_sample) added up into warp 0's (S, E), and the runs' relative
+// variance about their mean into its `spread` (1 + spread = kRuns sum_c (S_c / S)^2).
+__device__ __forceinline__ void block_sample(double& S, int& E, double& spread, double* redS,
+                                             int* redE) {
+  if ((threadIdx.x & 15) == 0) {
+    redS[threadIdx.x >> 4] = S;
+    redE[threadIdx.x >> 4] = E;
+  }
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    const double Sc = redS[threadIdx.x & (kRuns - 1)];  // both half warps alike
+    const int Ec = redE[threadIdx.x & (kRuns - 1)];
+    S = Sc;
+    E = Ec;
+    for (int o = kRuns / 2; o > 0; o >>= 1) {
+      const double S2 = __shfl_xor_sync(0xffffffffu, S, o);
+      const int E2 = __shfl_xor_sync(0xffffffffu, E, o);
+      scaled_add(S, E, S2, E2);
+    }
+    const double part = ldexp(Sc, 2 * (Ec - E)) / S;
+    double sq = part * part;
+    for (int o = kRuns / 2; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
+    spread = kRuns * sq - 1.0;
   }
 }
 
@@ -248,10 +279,6 @@ __device__ __forceinline__ int sigma_of(double S, int E, ScaleBits b) {
   return 0;
 }
 
-// Estimated norms whose mantissa (in [0.5, 1)) lies within this relative
-// distance of where the exponents change take the exact norm instead.
-constexpr double kEstimateBand = 1.0 / 32;
-
 // Row scale exponents of up to two k-major operands (len reals per row; rows = 0:
 // none) in one launch.
 struct RowScaleOp {
@@ -270,16 +297,15 @@ struct RowScaleParams {
   RowScaleOp op[2];
   int64_t len;
   ScaleBits bits;
-  int nruns;          // kEstimate: runs of `run` reals, `gap` apart
-  int64_t run, gap;
+  int64_t run, gap;   // kEstimate: runs of `run` reals, `gap` apart
   double lo, hi;      // kRecheck: range of ssq that proves an estimate
   int* status;        // cleared by kExact and kEstimate
 };
 
 // kExact: one block per row, the exact exponent. kEstimate: the exponent from a
-// sample of the row (the sum of squares of nruns runs extrapolated to len reals)
-// when the estimated norm is clear of the exponents' change by kEstimateBand
-// (exact[row] = 0), else, and for a zero or non-finite sample, the exact one
+// sample of the row (the sum of squares of kRuns runs extrapolated to len reals)
+// when the estimated norm is clear of the exponents' change (estimate_clear;
+// exact[row] = 0), else, and for a zero or non-finite sample, the exact one
 // (exact[row] = 1); clears the rows' sums of squares and the counts. kRecheck
 // (blocks grid-stride over the rows): a row whose exponent was estimated keeps
 // it when its sum of squares at that scale lies within [lo, hi] (the exponent is
@@ -311,17 +337,15 @@ __global__ void __launch_bounds__(256) oz_row_scale(const __grid_constant__ RowS
       if (op.exact[row] || (s >= P.lo && s <= P.hi)) continue;  // block-uniform
     }
     if (MODE == kEstimate) {
-      ssq_sample(x, P.nruns, P.run, P.gap, S, E, inv);
-      block_ssq(S, E, redS, redE);
+      double spread = 0.0;
+      ssq_sample(x, P.run, P.gap, S, E, inv);
+      block_sample(S, E, spread, redS, redE);
       if (threadIdx.x == 0) {
         bool use = false;
         if (S > 0.0 && S < 1e300) {
           int e0 = 0;
-          const double f =
-              frexp(sqrt(S * (double(P.len) / (double(P.nruns) * double(P.run)))), &e0);
-          // distance to thr, and to its neighbours one octave away
-          const double d = f < P.bits.thr ? f / P.bits.thr : f / (2.0 * P.bits.thr);
-          use = d > 0.5 * (1.0 + kEstimateBand) && d < 1.0 - kEstimateBand;
+          const double f = frexp(sqrt(S * (double(P.len) / (kRuns * double(P.run)))), &e0);
+          use = estimate_clear(f, P.bits.thr, spread / (kRuns - 1));
           if (use) op.sigma[row] = P.bits.q - (e0 + E) + (f < P.bits.thr ? 1 : 0);
         }
         op.exact[row] = use ? 0 : 1;
@@ -2512,29 +2536,29 @@ void slice_operands(const oz::Layout& L, const oz::Crt& crt, const GemmProblem& 
 // One-pass row scaling. The two-pass order reads every row twice: once for
 // its norm (the scale exponent), once to slice it. Here the exponent comes
 // from a sample of each row (16 evenly spread runs, 1/16 of its reals, the
-// sum of squares extrapolated to the whole row) unless the estimated norm
-// lies within kEstimateBand of a power of two, or the sample is zero or not
-// finite: such rows (all of them for rows normalised to 1) take the exact
-// norm at once. The default slicer also sums the squares of the scaled
-// values, and an estimated exponent stands when that sum lies in
-// [2^(2Q-2), 2^(2Q)) with a relative margin of 2^-30 at both ends (far above
-// the rounding of either sum; see onepass_fixup): the scaled norm then lies in
-// [2^(Q-1), 2^Q),
-// which is what the exact exponent gives. Other rows (a sample that
-// misjudged the row by more than the band) get the exact norm and are
-// sliced again. Each row thus ends with the exponent and residues of the
+// sum of squares extrapolated to the whole row) unless the estimate lies too
+// near the norms where the exponents change for what the spread of the runs
+// says of it (estimate_clear), or the sample is zero or not finite: such rows
+// take the exact norm at once. The default slicer also sums the squares of
+// the scaled values, and an estimated exponent stands when that sum lies in
+// [low^2, 4 low^2), low = thr 2^Q (Crt::thr), with a relative margin at both
+// ends far above the rounding of either sum (see launch_row_scale): the
+// scaled norm then lies in [low, 2 low), which is what the exact exponent
+// gives. Other rows (a sample that misjudged the row) get the exact norm and
+// are sliced again. Each row thus ends with the exponent and residues of the
 // two-pass order, whatever the order of the atomic sums. Used for each
-// k-major operand (an operand read in place keeps its norms) with the
-// default modulus count and unrolled slicer and rows of at least kOnePassMinLen reals; SPLAB_OZAKI_ONEPASS=0 (read per call) keeps
-// the two-pass order.
+// k-major operand (an operand read in place keeps its norms) with the default
+// modulus count and unrolled slicer and rows of at least kOnePassMinLen reals;
+// SPLAB_OZAKI_ONEPASS=0 (read per call) keeps the two-pass order.
 //
 // It pays from about 256 MB of k-major operands: the norms' second read (6 TB/s)
 // against the sample and two more launches (387 x 515 x 60013 complex double, 866
 // MB: 150 us of norms, 30 us of estimates and checks); rows of 16384 reals keep 64
-// reals per run. Rows of 131072 reals always take it.
+// reals per run. Real float rows that short gain nothing (2000 + 2000 rows of 40000: 1.53
+// ms against 1.51) and lose 14 % where the rows take their exact norms (1.58 against
+// 1.39). Rows of 131072 reals always take it.
 constexpr int64_t kOnePassMinLen = 16384, kOnePassLongLen = 131072;
 constexpr double kOnePassMinBytes = 256e6;
-constexpr int kOnePassRuns = 16;
 
 // The operands scaled in one pass: bit 1 A, bit 2 B (k-major ones only; the
 // rows read in place keep their k-sliced norms)
@@ -2546,7 +2570,7 @@ int onepass_operands(const oz::Layout& L, const GemmProblem& p) {
   if (p.k <= 0 || !unrolled || !slice_unroll() || L.K2 < kOnePassMinLen) return 0;
   const double bytes = double((L.mn ? 0 : L.rowsA) + (L.mnB ? 0 : L.rowsB)) * double(L.K2) *
                        (dtype_is_double(p.dtype) ? 8 : 4);
-  if (L.K2 < kOnePassLongLen && bytes < kOnePassMinBytes) return 0;
+  if (L.K2 < kOnePassLongLen && (p.dtype == kR32 || bytes < kOnePassMinBytes)) return 0;
   return (L.mn ? 0 : 1) | (L.mnB ? 0 : 2);
 }
 
@@ -2567,9 +2591,8 @@ void launch_row_scale(const oz::Layout& L, const oz::Crt& crt, const GemmProblem
              ssq + L.rowsA, list + L.rowsA, count + 1};
   P.len = L.K2;
   P.bits = {crt.q_bits, crt.thr};
-  P.nruns = kOnePassRuns;
-  P.run = (L.K2 / (16 * kOnePassRuns) + 7) / 8 * 8;
-  P.gap = L.K2 / kOnePassRuns;
+  P.run = (L.K2 / (16 * kRuns) + 7) / 8 * 8;
+  P.gap = L.K2 / kRuns;
   // the two sums of squares (norm kernel: runs of K2 / 256 terms per thread, then
   // trees; slicers: at most 64 terms per thread, trees, at most K2 / 2048 atomics
   // per row) differ by at most about (K2 / 256 + K2 / 2048 + 64) units of 2^-53
