@@ -552,7 +552,7 @@ double sparse_plan_us(const GemmProblem& pr, const DmmaPlan& plan, int num_sms) 
 
 }  // namespace
 
-DmmaPlan dmma_plan(const GemmProblem& pr, int num_sms, int force_splits) {
+DmmaPlan dmma_plan(const GemmProblem& pr, int num_sms, int force_splits, bool allow_small) {
   auto plan = [&](bool small) {
     DmmaPlan p = dispatch(pr, small, [&](auto cfg) {
       return plan_for<decltype(cfg)>(pr, num_sms, force_splits);
@@ -561,7 +561,7 @@ DmmaPlan dmma_plan(const GemmProblem& pr, int num_sms, int force_splits) {
     return p;
   };
   const DmmaPlan def = plan(false);
-  if (force_splits > 0 || pr.k <= 0) return def;
+  if (force_splits > 0 || pr.k <= 0 || !allow_small) return def;
   auto tiles = [&](int bm, int bn) { return ((pr.m + bm - 1) / bm) * ((pr.n + bn - 1) / bn); };
   // 32 x 32 tiles pay where the default ones pad C by 15 % more (they run at 0.92 to
   // 0.97 of the default tiles' rate: 1024 x 1024 x 4000 complex double 1059 against 1089
@@ -687,11 +687,15 @@ int dmma_gemm_noalloc(const GemmProblem& pr, int num_sms, cudaStream_t st) {
   if (pr.m <= 0 || pr.n <= 0) return 0;
   // The planner's split count first: a plan with one k-split (small k, or
   // k = 0) needs no partials and runs at any size. Otherwise one split's
-  // partials are m * n FP64 (complex: pairs); with fewer splits than the
-  // planner chose they are made to fit the static array, and problems where
-  // not even two fit are refused.
+  // partials are m * n FP64 (complex: pairs): a plan of 32 x 32 tiles that
+  // does not fit gives way to the default tiles, which may need fewer (68 x
+  // 36925 x 301 complex float: one split against two). With fewer splits than
+  // the planner chose they are made to fit the static array, and problems
+  // where not even two fit are refused.
   const size_t per_split = size_t(pr.m) * size_t(pr.n) * (dtype_is_complex(pr.dtype) ? 16 : 8);
   DmmaPlan plan = dmma_plan(pr, num_sms);
+  if (plan.small && plan.workspace_bytes > SPLAB_NOALLOC_SCRATCH_BYTES)
+    plan = dmma_plan(pr, num_sms, 0, false);
   if (plan.workspace_bytes > SPLAB_NOALLOC_SCRATCH_BYTES) {
     const size_t fit = size_t(SPLAB_NOALLOC_SCRATCH_BYTES) / per_split;
     if (fit < 2) return 2;

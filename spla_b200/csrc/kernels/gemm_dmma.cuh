@@ -42,7 +42,9 @@ struct DmmaPlan {
   bool small;  // the 32 x 32 tile configuration
 };
 
-DmmaPlan dmma_plan(const GemmProblem& prob, int num_sms, int force_splits = 0);
+// allow_small: false keeps the default tiles (as force_splits > 0 does).
+DmmaPlan dmma_plan(const GemmProblem& prob, int num_sms, int force_splits = 0,
+                   bool allow_small = true);
 cudaError_t dmma_gemm(const GemmProblem& prob, const DmmaPlan& plan, void* workspace,
                       cudaStream_t stream);
 
