@@ -165,8 +165,18 @@ double ozaki_ms(const GemmProblem& p, double most) {
   // Float types keep a tenth in reserve against 3xTF32, whose estimate is the closer.
   const OzakiShape shape = ozaki_shape(p);
   const bool dbl = dtype_is_double(p.dtype);
-  const double tall = slice + transpose + std::max(gemm, shape.gemm_seconds) +
-                      (dbl ? (c ? 20e-12 : 9.4e-12) : (c ? 14e-12 : 9e-12)) * mn;
+  const double by_element = slice + transpose + std::max(gemm, shape.gemm_seconds) +
+                            (dbl ? (c ? 20e-12 : 9.4e-12) : (c ? 14e-12 : 9e-12)) * mn;
+  // The norms of k-major rows take 4.3 ns a row, a block each, however short the row
+  // (200000 x 256 x 256 complex double, A^H: 0.85 ms; 3.6 ms on the Ozaki path, 3.2 on
+  // DMMA; with A read in place 2.7 against 3.2). They count beside the caller's reserve
+  // of a tenth, not on top of it: of 180 tall double shapes the six that DMMA did in 0.83
+  // to 0.92 of the time leave, and one of the others (0.89, at 10000 rows).
+  auto row_blocks = [&](double rows, bool k_major) {
+    return k_major ? std::max(0.0, 4.3e-9 * rows - norm_rows(rows, true)) : 0.0;
+  };
+  const double tall = std::max(by_element, 0.9 * (by_element + row_blocks(p.m, p.opA != 0) +
+                                                  row_blocks(p.n, p.opB == 0)));
   return (shape.bytes ? std::min(t, tall * (dbl ? 1.0 : 1.1)) : t) * 1e3 + 0.08;
 }
 
