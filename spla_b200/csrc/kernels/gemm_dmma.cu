@@ -568,8 +568,18 @@ DmmaPlan dmma_plan(const GemmProblem& pr, int num_sms, int force_splits, bool al
   // us; 129 x 129 x 30000 307 -> 229, 100 x 80 x 20000 110 -> 95, 33 x 500 x 5000 real
   // double 50 -> 40), and where the default plan has fewer CTAs than SMs and theirs
   // finish sooner (64 x 64 x 64 complex double: one CTA 16.6 us, four 7.6)
+  // Real types take more padding: their small tiles load twice as much per flop. With
+  // op(B) n-major they run at 0.78 to 0.85 of the default rate (800 x 800 x 30621 real
+  // double NT 1.08 times the default's time, 350 x 350 1.05, 2200 x 150 1.04), and in real
+  // double with two k-major operands at 0.73 to 0.93 when k is odd, so that rows packed
+  // back to back are not on 16-byte boundaries and load 8 bytes at a time (2000 x 140 x
+  // 30621 1.16 times the default's time, x 30000 0.91; 350 x 350 x 30621 1.07).
   const int64_t def_tiles = tiles(def.bm, def.bn);
-  const bool padded = double(def_tiles) * def.bm * def.bn >= 1.15 * 1024.0 * double(tiles(32, 32));
+  double least = 1.15;
+  if (!dtype_is_complex(pr.dtype) && pr.opB != 0) least = 1.26;
+  if (pr.dtype == kR64 && pr.opA != 0 && pr.opB == 0 && pr.k % 2 != 0) least = 1.31;
+  const bool padded =
+      double(def_tiles) * def.bm * def.bn >= least * 1024.0 * double(tiles(32, 32));
   if (!padded && def_tiles * def.splits >= num_sms) return def;
   const DmmaPlan small = plan(true);
   if (def_tiles * def.splits >= num_sms) return small;

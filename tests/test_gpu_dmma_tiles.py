@@ -1,0 +1,18 @@
+"""Which tiles the DMMA planner takes for C padded by the default ones, told by the
+splits of k in its workspace (times of the small tiles beside those of the default)."""
+import pytest
+
+import spla_b200 as spla
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dt,opA,opB,m,n,k,splits", [
+    ("float64", 1, 0, 2000, 140, 30621, 6),   # default tiles (small: 7 splits, 1.16)
+    ("float64", 1, 0, 2000, 140, 20000, 7),   # small tiles (default: 6 splits, 0.91)
+    ("float64", 1, 0, 350, 350, 69563, 16),   # default (small: 6, 1.09)
+    ("float64", 0, 1, 800, 800, 30621, 13),   # default (small: 7, 1.08)
+    ("float64", 0, 1, 140, 2000, 30621, 14)]) # small (default: 9, 0.76)
+def test_small_tiles_only_where_they_pay(dt, opA, opB, m, n, k, splits):
+    nbytes = spla.splab_gemm_workspace_size(dt, spla.PATH_DMMA, opA, opB, m, n, k)
+    assert nbytes == splits * m * n * 8
