@@ -67,3 +67,70 @@ def test_rows_of_uneven_weight_are_sliced_once(dt, m, n, k, profile):
         assert again <= 0.02 * (m + n) and exact <= 0.3 * (m + n)
     else:
         assert again == 0 and exact == m + n
+
+
+def _threshold(dt):
+    """thr of a type's default moduli, as ozaki_crt.cuh makes it: the exponents change at
+    row norms thr 2^e."""
+    import math
+    import re
+    from pathlib import Path
+    text = (Path(__file__).resolve().parent.parent / "spla_b200" / "csrc" / "kernels" /
+            "ozaki_crt.cuh").read_text()
+    cplx = dt.startswith("complex")
+    name, count = ("kSplitModuli", {"complex128": 16, "complex64": 10}) if cplx else \
+                  ("kModuli", {"float64": 15, "float32": 9})
+    table = [int(v) for v in re.search(name + r"\[\w+\]\s*=\s*\{([^}]*)\}",
+                                       text).group(1).split(",")]
+    half = (math.log2(math.prod(table[:count[dt]])) - 2.0) / 2.0
+    f = 2.0 ** (half - math.floor(half)) / 2.0 * (1.0 - 1.0 / 64)
+    return 0.75 if dt == "complex64" else 0.5 if f < 0.6 else f
+
+
+@pytest.mark.parametrize("dt", ["complex128", "float64", "complex64", "float32"])
+def test_norms_where_the_exponents_change(dt):
+    """Rows of even weight at, next to and off the norms thr 2^e (an estimate counts
+    from 3.1 % off: exact norms within 2 %, none beyond 6 %), and rows whose sample
+    gives 0.8 or 1.25 of a norm next to such a step, which only the check of the sums
+    of squares can send back, at either end of its range. All end with the two-pass
+    exponents: C is bit-identical."""
+    import torch
+    thr = _threshold(dt)
+    cplx = dt.startswith("complex")
+    k = 70000 if cplx else 140000
+    K2 = 140000
+    steps = torch.tensor([0.0] + [s * d for d in (1e-12, 1e-9, 3e-7, 1e-6, 1e-5, 1e-3)
+                                  for s in (1, -1)], dtype=torch.float64, device="cuda")
+    near = torch.cat([steps, torch.tensor([0.02, -0.02], device="cuda", dtype=torch.float64)])
+    off = torch.tensor([0.06, 0.2, 0.5, 0.85, -0.06, -0.2, -0.4, -0.47], device="cuda",
+                       dtype=torch.float64)
+    g = torch.Generator(device="cuda")
+    g.manual_seed(3)
+    # the sample: 16 runs of `run` reals, `gap` apart
+    run, gap = (K2 // 256 + 7) // 8 * 8, K2 // 16
+    sampled = torch.zeros(K2, dtype=torch.bool, device="cuda")
+    for c in range(16):
+        sampled[c * gap:c * gap + run] = True
+    even = torch.randn((len(near) + len(off), K2), dtype=torch.float64, device="cuda", generator=g)
+    even *= (thr * (1.0 + torch.cat([near, off])) /
+             torch.linalg.vector_norm(even, dim=1))[:, None]
+    parts = [even]
+    for est in (0.8, 1.25):
+        X = torch.randn((len(steps), K2), dtype=torch.float64, device="cuda", generator=g)
+        ins = torch.where(sampled, X, torch.zeros_like(X))
+        rest = X - ins
+        share = est * est * 16.0 * run / K2  # of the sum of squares, in the sample
+        ins *= (share ** 0.5 / torch.linalg.vector_norm(ins, dim=1))[:, None]
+        rest *= ((1.0 - share) ** 0.5 / torch.linalg.vector_norm(rest, dim=1))[:, None]
+        parts.append((ins + rest) * (thr * (1.0 + steps))[:, None])
+    rows = torch.cat(parts)
+    rows[::2] *= 2.0 ** 20  # other octaves
+    rows = rows.to(torch.float64 if dt in ("complex128", "float64") else torch.float32)
+    A = torch.view_as_complex(rows.view(len(rows), k, 2).contiguous()) if cplx else rows
+    B = A.flip(0).contiguous()
+    C, again, exact = _run(dt, A, B, True)
+    assert torch.equal(C, _run(dt, A, B, False)[0])
+    # A's and B's rows: exact norms for those within 2 % of a step, an estimate for the
+    # others; sent back: at least the rows on the wrong side (six steps of either sign)
+    assert exact == 2 * len(near)
+    assert 2 * 12 <= again <= 2 * 2 * len(steps)
