@@ -1989,11 +1989,13 @@ struct Layout {
   bool at;                 // op(A) = N too long for in-place tiles: A copied k-major
   bool mn;                 // op(A) = N: A read in place (m-major)
   bool mnB;                // op(B) = T or C: B read in place (n-major)
+  int ksA, ksB;            // k-slices of the in-place row norms of A and B (1: none)
   int nchunks, nt;         // k-chunks and tile width of the GEMM (choose_gemm)
   bool r8;                 // the residues of C are bytes, one plane per product and k-chunk
   int64_t ldR, planeR;     // elements between the columns of a plane and between planes
   int64_t ldAt;            // leading dimension of At (elements of A's type)
   size_t off_sigA, off_sigB, off_resA, off_resB, off_R, off_At, off_status, off_tiles;
+  size_t off_partA, off_partB;  // k-slice partial sums of the in-place row norms
   size_t off_ssq, off_list;     // one-pass row scaling (onepass_operands): scaled sums
                                 // of squares, rows sent back and their two counts
   size_t total;
@@ -2071,6 +2073,15 @@ bool mn_fits(const GemmProblem& p) {
   return (kp + kt - 1) / kt <= 65535;
 }
 
+// k-slices of the in-place row norms: about 2^18 threads in all (one per row
+// and slice), slices of at least 512 elements, at most 4096 slices (the grid's
+// y extent)
+int norm_slices(int64_t rows, int64_t k) {
+  if (rows >= kMnRows || k <= 512) return 1;
+  const int64_t want = std::min<int64_t>(((int64_t(1) << 18) + rows - 1) / rows, 4096);
+  return int(std::max<int64_t>(1, std::min<int64_t>(want, (k + 511) / 512)));
+}
+
 Layout layout_of(const GemmProblem& p, int moduli) {
   Layout L{};
   const bool dbl = dtype_is_double(p.dtype), cplx = dtype_is_complex(p.dtype);
@@ -2095,6 +2106,8 @@ Layout layout_of(const GemmProblem& p, int moduli) {
   L.mn = p.opA == 0 && mn_fits(p);
   L.at = p.opA == 0 && !L.mn;
   L.mnB = p.opB != 0;
+  L.ksA = L.mn ? norm_slices(p.m, p.k) : 1;
+  L.ksB = L.mnB ? norm_slices(p.n, p.k) : 1;
   choose_gemm(L, p.m, p.n);
   // bytes where the tensor-core reconstruction takes all planes (its columns lie on
   // 16-byte boundaries), else one int32 sum per product
@@ -2130,6 +2143,11 @@ Layout layout_of(const GemmProblem& p, int moduli) {
   off = align256(off + 256);
   L.off_tiles = off;
   off = align256(off + sizeof(int) * size_t((L.rowsA + 255) / 256) * ((L.nb + 255) / 256));
+  L.off_partA = off;
+  // (reserved: partial sums of the in-place norms, now in the residues' room)
+  off = align256(off + (L.ksA > 1 ? size_t(L.ksA) * L.rowsA * (sizeof(double) + sizeof(int)) : 0));
+  L.off_partB = off;
+  off = align256(off + (L.ksB > 1 ? size_t(L.ksB) * L.rowsB * (sizeof(double) + sizeof(int)) : 0));
   L.off_ssq = off;  // A's rows, then B's
   off = align256(off + sizeof(double) * (size_t(L.rowsA) + L.rowsB));
   L.off_list = off;  // lists of A's and B's rows, their exact flags, the two counts
