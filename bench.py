@@ -1142,8 +1142,10 @@ def main():
                 "peak_source": "measured here: cuBLASLt int8 GEMM 8192^3 via torch._int_mm",
                 "algorithmic_ops_per_launch": int8_ops}
         # row scales of both operands, two slicers, GEMM, reconstruction; with the one-pass
-        # scaling (rows of 131072 reals and more) also the check and two fix-up slicers
-        launches = (8 if 2 * K >= 131072 else 5) * args.steps
+        # scaling (rows of 131072 reals and more, or of 16384 in 256 MB of operands) also
+        # the check and two fix-up slicers
+        onepass = 2 * K >= 131072 or (2 * K >= 16384 and 16.0 * (M + N) * K >= 256e6)
+        launches = (8 if onepass else 5) * args.steps
         roof["gemm_launches_per_step"] = 1
         roof["note"] = "achieved = INT8 ops / duration of the GEMM launch"
         hr["phase_ms"] = hr["phase_ms"][:3] + gemm_launch_ms

@@ -63,7 +63,11 @@ SPLAB_API const char *splab_status_string(int status);
  * supported paths whose workspace fits in a quarter of the device memory, the
  * one with the least modelled time (a model of each path measured on B200;
  * a tensor-core path must beat DMMA by 10 %). The result depends only on the
- * problem and the device. */
+ * problem and the device. The error of the Ozaki path is relative to the product
+ * of the norms of a row of op(A) and a column of op(B), that of DMMA to the sum
+ * of |a| |b| of the element: rows whose entries differ by many orders of
+ * magnitude, with products that matter among the small ones, ask for
+ * SPLAB_PATH_DMMA. */
 SPLAB_API int splab_gemm_path(int dtype, int path, int opA, int opB, int64_t m, int64_t n,
                               int64_t k);
 
@@ -255,7 +259,8 @@ SPLAB_API int splab_gemm_dd(int dtype, int opA, int opB, int64_t m, int64_t n, i
  *               3 = the GEMM launch; inside phase 0:
  *               15 = k-major copy of A (op(A) = N with k too long to be read in
  *               place), 16 = row norms of A and B, 17 = residues of A,
- *               18 = residues of B
+ *               18 = residues of B, 19 = check of estimated row exponents and
+ *               second slicing (long k-major rows)
  * Pass events = NULL to stop. Returns SPLAB_OK.
  */
 SPLAB_API int splab_set_phase_events(void **events, int count);

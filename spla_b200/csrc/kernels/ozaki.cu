@@ -996,8 +996,8 @@ struct GemmParams {
   int m;             // rows of A per product plane
   int nb;            // rows of B per product plane
   int kblocks;       // kp / 128
-  int nchunks;       // ceil(kblocks / kChunkBlocks)
-  int chunk_blocks;  // k-blocks per chunk: ceil(kblocks / nchunks) <= kChunkBlocks
+  int nchunks;       // k-chunks (choose_gemm)
+  int chunk_blocks;  // k-blocks per chunk: ceil(kblocks / nchunks), within the INT32 bound
   int group;         // planes per group, and k-blocks per piece of a plane's row
   int kc_blocks;     // (ResidueLayout: G, kc / 128)
   int nmod;          // products: moduli x nsub (the A/B/R planes in order)
@@ -1252,8 +1252,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
 // NT = 1: pair tile 256 x 256, two accumulator buffers (2 x 256 TMEM
 // columns), 6 stages. NT = 2: pair tile 256 x 512 (two MMAs of N = 256 per
 // k-step on one A tile: a quarter less L2 -> SMEM traffic per operation), one
-// accumulator buffer of 512 columns (drained once per unit of 976 k-blocks),
-// 4 stages.
+// accumulator buffer of 512 columns (drained once per unit), 4 stages.
 constexpr int A_STAGE2 = 128 * BKB;  // 16 KiB per CTA
 constexpr int B_HALF2 = 128 * BKB;   // 16 KiB per CTA and N = 256 half
 template <int NT>
@@ -1989,13 +1988,13 @@ struct Layout {
   bool at;                 // op(A) = N too long for in-place tiles: A copied k-major
   bool mn;                 // op(A) = N: A read in place (m-major)
   bool mnB;                // op(B) = T or C: B read in place (n-major)
-  int ksA, ksB;            // k-slices of the in-place row norms of A and B (1: none)
+  int ksA, ksB;            // slices of off_partA and off_partB (1: none)
   int nchunks, nt;         // k-chunks and tile width of the GEMM (choose_gemm)
   bool r8;                 // the residues of C are bytes, one plane per product and k-chunk
   int64_t ldR, planeR;     // elements between the columns of a plane and between planes
   int64_t ldAt;            // leading dimension of At (elements of A's type)
   size_t off_sigA, off_sigB, off_resA, off_resB, off_R, off_At, off_status, off_tiles;
-  size_t off_partA, off_partB;  // k-slice partial sums of the in-place row norms
+  size_t off_partA, off_partB;  // room that is not used (layout_of)
   size_t off_ssq, off_list;     // one-pass row scaling (onepass_operands): scaled sums
                                 // of squares, rows sent back and their two counts
   size_t total;
@@ -2073,9 +2072,8 @@ bool mn_fits(const GemmProblem& p) {
   return (kp + kt - 1) / kt <= 65535;
 }
 
-// k-slices of the in-place row norms: about 2^18 threads in all (one per row
-// and slice), slices of at least 512 elements, at most 4096 slices (the grid's
-// y extent)
+// Slices of partial sums of the in-place row norms that the workspace has room for
+// (layout_of); the kernels cut finer and keep theirs elsewhere (in_place_slices).
 int norm_slices(int64_t rows, int64_t k) {
   if (rows >= kMnRows || k <= 512) return 1;
   const int64_t want = std::min<int64_t>(((int64_t(1) << 18) + rows - 1) / rows, 4096);
@@ -2093,8 +2091,7 @@ Layout layout_of(const GemmProblem& p, int moduli) {
   L.nmod = L.split ? (dbl ? kSplitCount : kSplitCountFloat) : count;
   L.nsub = L.split ? 2 : cplx ? 3 : 1;
   L.pairs = L.split && dbl;
-  // The workspace keeps the size of the three-product form for callers that
-  // hold one sized for it (32 planes of the split form lie in the room of 45)
+  // planes of the three-product form, whose size the workspace keeps (see below)
   const size_t planes = size_t(count) * (cplx ? 3 : 1);
   L.K2 = cplx ? 2 * p.k : p.k;
   L.kp = (p.k + BKB - 1) / BKB * BKB;
@@ -2122,9 +2119,10 @@ Layout layout_of(const GemmProblem& p, int moduli) {
   off = align256(off + sizeof(int) * L.rowsA);
   L.off_sigB = off;
   off = align256(off + sizeof(int) * L.rowsB);
-  // The workspace is not smaller than that of the three-product form, for callers that
-  // hold one sized for it: 45 planes to the split form's 32 (and int32 sums from the
-  // second k-chunk on), with room for the planes of its k-chunks in the difference.
+  // The size asked for is that of the three-product form (45 planes to the split form's
+  // 32, and int32 sums from the second k-chunk on), of which the planes of the split
+  // form's k-chunks take a part: AUTO holds it against a quarter of the device memory,
+  // so the problems that the limit turns away are the ones it was measured with.
   const bool one_chunk = (L.kp / BKB + kChunkBlocks - 1) / kChunkBlocks <= 1;
   const size_t reserved = align256(planes * L.rowsA * L.kp) + align256(planes * L.nb * L.kp) +
                           align256((one_chunk ? 1 : sizeof(int)) * planes * L.nb * L.rowsA);
@@ -2144,7 +2142,8 @@ Layout layout_of(const GemmProblem& p, int moduli) {
   L.off_tiles = off;
   off = align256(off + sizeof(int) * size_t((L.rowsA + 255) / 256) * ((L.nb + 255) / 256));
   L.off_partA = off;
-  // (reserved: partial sums of the in-place norms, now in the residues' room)
+  // room for partial sums of the in-place norms, part of the size that is asked for;
+  // nothing lies here (in_place_slices)
   off = align256(off + (L.ksA > 1 ? size_t(L.ksA) * L.rowsA * (sizeof(double) + sizeof(int)) : 0));
   L.off_partB = off;
   off = align256(off + (L.ksB > 1 ? size_t(L.ksB) * L.rowsB * (sizeof(double) + sizeof(int)) : 0));
@@ -2594,10 +2593,10 @@ void launch_row_scale(const oz::Layout& L, const oz::Crt& crt, const GemmProblem
   P.run = (L.K2 / (16 * kRuns) + 7) / 8 * 8;
   P.gap = L.K2 / kRuns;
   // the two sums of squares (norm kernel: runs of K2 / 256 terms per thread, then
-  // trees; slicers: at most 64 terms per thread, trees, at most K2 / 2048 atomics
-  // per row) differ by at most about (K2 / 256 + K2 / 2048 + 64) units of 2^-53
-  // relative; the margin is 2^-30, or K2 2^-59 for rows beyond 2^29 reals (float rows: a
-  // thread's sum of up to 16 squares is in FP32, 2^-20 at most)
+  // trees; slicers: at most 128 terms per thread, trees, at most K2 / 128 atomics per
+  // row) differ by at most about (K2 / 256 + K2 / 128 + 128) units of 2^-53 relative;
+  // the margin is 2^-30, or K2 2^-59 for rows beyond 2^29 reals (float rows: a thread's
+  // sum of up to 16 squares is in FP32, 2^-20 at most)
   const double delta = std::max(std::ldexp(1.0, sizeof(TIn) == 4 ? -19 : -30),
                                 std::ldexp(double(L.K2), -59));
   const double low = std::ldexp(crt.thr, crt.q_bits);  // scaled norms lie in [low, 2 low)

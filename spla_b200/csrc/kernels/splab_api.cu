@@ -111,7 +111,8 @@ GemmProblem make_problem(int dtype, int opA, int opB, int64_t m, int64_t n, int6
 // 2048 x 512 12.5 against 4.5. The slicing and three-product GEMM rates are those of
 // earlier kernels and now on the safe side: problems near the crossover stay where
 // they were. 3xTF32 as splitting (bytes at 5.5 TB/s), three TF32
-// products at 480 TFLOP/s scaled by the same fill, and 0.05 ms. The choice only
+// products at 480 TFLOP/s scaled by the same fill (of units of 2048 reals, as its
+// rates were fitted; the kernel's may be half as long), and 0.05 ms. The choice only
 // depends on the problem and the device (no free-memory query), so that
 // resolving a path, sizing its workspace and running it agree.
 namespace model {

@@ -11,8 +11,7 @@ problem is C = op(A) op(B) with op(A) = conjugate transpose (complex) or
 transpose (real) unless opA is given (0 = N: A is m x k, the pgemm_sbs
 shape) and op(B) = N unless opB is given (1 = T, 2 = C: B is n x k), Gaussian
 operands scaled by 1/sqrt(k), or with --normalised every row of op(A) and
-column of B scaled to norm 1 (norms on a power of two: the rows whose
-exponents the Ozaki path's one-pass scaling cannot estimate). One JSON line per spec: total time,
+column of B scaled to norm 1. One JSON line per spec: total time,
 TFLOP/s and the phase times the path reports (scale/slice, GEMM span,
 reduction or reconstruction, then one entry per GEMM launch) and, for the
 Ozaki path, the parts of the slicing phase.
