@@ -2002,7 +2002,34 @@ struct Layout {
 
 size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 
-Crt crt_of(const Layout& L) { return L.split ? make_crt_split(L.nmod) : make_crt(L.nmod); }
+// The moduli's constants, made once: the 16 split ones take the host 15 us.
+const Crt& crt_of(const Layout& L) {
+  struct Table {
+    Crt general[kMaxUsableModuli + 1], split, split_float;
+    Table() : split(make_crt_split(kSplitCount)), split_float(make_crt_split(kSplitCountFloat)) {
+      for (int n = 1; n <= kMaxUsableModuli; ++n) general[n] = make_crt(n);
+    }
+  };
+  static const Table t;
+  if (!L.split) return t.general[L.nmod];
+  return L.nmod == kSplitCount ? t.split : t.split_float;
+}
+
+// oz_slice_mma's rows for j (`sign` 1) or -j, made once (17 us of host time). V's
+// planes hold -v, as oz_slice's.
+const SliceRow* split_slice_rows(const Crt& crt, int sign) {
+  struct Table {
+    SliceRow row[kSlicePlanes];
+    Table(const Crt& c, int s) {
+      for (int t = 0; t < kSplitCount; ++t) {
+        row[2 * t] = make_slice_row(c.p[t], 1, s * c.j[t]);
+        row[2 * t + 1] = make_slice_row(c.p[t], -1, s * c.j[t]);
+      }
+    }
+  };
+  static const Table plus(crt, 1), minus(crt, -1);
+  return sign > 0 ? plus.row : minus.row;
+}
 
 // Complex double planes with the split moduli come in pairs: the 32 planes of a
 // row are written at once, and as many streams far apart cost the slicer (see
@@ -2454,11 +2481,7 @@ void launch_slice_mma(const oz::Layout& L, const oz::Crt& crt, const double* X, 
   P.steps_per_row = int(2 * L.kp / kStepReals);
   const int wpr = P.steps_per_row >= 4 ? 4 : 2;  // kp >= 128: at least two steps
   P.warps_per_row = wpr;
-  // V's planes hold -v, as oz_slice's
-  for (int t = 0; t < kSplitCount; ++t) {
-    P.row[2 * t] = make_slice_row(crt.p[t], 1, sign * crt.j[t]);
-    P.row[2 * t + 1] = make_slice_row(crt.p[t], -1, sign * crt.j[t]);
-  }
+  std::copy_n(split_slice_rows(crt, sign), kSlicePlanes, P.row);
   const long long slots = (long long)kSliceBlocks * sm_count();
   const long long steps = (long long)rows * P.steps_per_row;
   // equal segments of a row, of at most 32 steps per warp, and short enough for
@@ -2801,7 +2824,7 @@ cudaError_t ozaki_gemm(const GemmProblem& p_in, int moduli, void* ws, size_t ws_
   if (p_in.m <= 0 || p_in.n <= 0) return cudaSuccess;
   const Layout L = layout_of(p_in, moduli);
   if (ws_bytes < L.total || !ws) return cudaErrorInvalidValue;
-  const Crt crt = crt_of(L);
+  const Crt& crt = crt_of(L);
   const bool cplx = dtype_is_complex(p_in.dtype);
   char* w = static_cast<char*>(ws);
   int* sigA = reinterpret_cast<int*>(w + L.off_sigA);
