@@ -878,26 +878,28 @@ __global__ void __launch_bounds__(256) oz_row_scale_mn(const TIn* __restrict__ X
   }
 }
 
-// sigma of each row from its k-slice partial sums: 32 rows per block, eight
-// threads (of eight warps) to a row
-__global__ void __launch_bounds__(256) oz_row_scale_combine(const double* __restrict__ partS,
+// sigma of each row from its k-slice partial sums: 32 rows per block, one thread
+// of each of its warps (8 to 32) to a row
+__global__ void __launch_bounds__(1024) oz_row_scale_combine(const double* __restrict__ partS,
                                                             const int* __restrict__ partE, int m,
                                                             int slices, ScaleBits bits,
                                                             int* __restrict__ sigma) {
-  __shared__ double sumS[8][32];
-  __shared__ int sumE[8][32];
+  __shared__ double sumS[32][32];
+  __shared__ int sumE[32][32];
+  const int warps = int(blockDim.x) >> 5;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int i = blockIdx.x * 32 + lane;
   double S = 0.0;
   int E = -2100;
   if (i < m)
-    for (int sl = w; sl < slices; sl += 8)
+#pragma unroll 4
+    for (int sl = w; sl < slices; sl += warps)
       scaled_add(S, E, partS[int64_t(sl) * m + i], partE[int64_t(sl) * m + i]);
   sumS[w][lane] = S;
   sumE[w][lane] = E;
   __syncthreads();
   if (w != 0 || i >= m) return;
-  for (int v = 1; v < 8; ++v) scaled_add(S, E, sumS[v][lane], sumE[v][lane]);
+  for (int v = 1; v < warps; ++v) scaled_add(S, E, sumS[v][lane], sumE[v][lane]);
   sigma[i] = sigma_of(S, E, bits);
 }
 
@@ -2392,13 +2394,19 @@ void launch_slice_mn(int ndig, cudaStream_t st, const TIn* X, int64_t ld, int m,
 
 // k-slices of the in-place row norms: threads (one per row and slice) for two
 // full loads of the GPU, slices of at least 32 elements (a thread's loads go out in
-// batches of 8), at most 4096 (the grid's y extent). The partial sums lie where
-// the operand's residues go next. Slices of 512 elements and more had left a 1501
-// x 1207 operand with 24 blocks (39.8 us; now 9.6).
+// batches of 8), and 512 slices or slices of 512 elements (at most 4096, the grid's y
+// extent), since each costs a partial sum to add up. The partial sums lie where the
+// operand's residues go next. Slices of 512 elements and more throughout had left a
+// 1501 x 1207 operand with 24 blocks (39.8 us; now 9.6); up to 4096 slices, added up by
+// eight threads a row, took 446 us for both operands of 256 x 256 x 100000 complex
+// double NT (161 now, 169 for one of them before) and 463 for 89 x 93 x 122231 complex
+// float (126, 339). Up to 64 elements the second launch costs more than it saves (24
+// against 17 us).
 int in_place_slices(int64_t rows, int64_t k) {
-  if (rows >= oz::kMnRows) return 1;
+  if (rows >= oz::kMnRows || k <= 64) return 1;
   const int64_t want = (int64_t(oz::sm_count()) * 4096 + rows - 1) / rows;
-  return int(std::max<int64_t>(1, std::min({want, (k + 31) / 32, int64_t(4096)})));
+  const int64_t most = std::min<int64_t>(4096, std::max<int64_t>(512, k / 512));
+  return int(std::max<int64_t>(1, std::min({want, (k + 31) / 32, most})));
 }
 
 // Row scale exponents of the operands read in place.
@@ -2419,9 +2427,11 @@ void scale_in_place(const oz::Layout& L, const oz::Crt& crt, const GemmProblem& 
     else
       oz_row_scale_mn<TIn, false><<<grid, 256, 0, st>>>(static_cast<const TIn*>(X), ld, rows, p.k,
                                                         kspan, bits, sig, partS, partE);
-    if (ks > 1)
-      oz_row_scale_combine<<<unsigned((rows + 31) / 32), 256, 0, st>>>(partS, partE, rows, ks,
-                                                                       bits, sig);
+    if (ks > 1) {  // a warp per 16 slices: warp 0 adds up the warps' sums one by one
+      const int warps = std::min(32, std::max(8, ks / 16));
+      oz_row_scale_combine<<<unsigned((rows + 31) / 32), unsigned(32 * warps), 0, st>>>(
+          partS, partE, rows, ks, bits, sig);
+    }
   };
   if (L.mn) scale(p.A, p.lda, L.rowsA, resA, sigA);
   if (L.mnB) scale(p.B, p.ldb, L.rowsB, resB, sigB);
