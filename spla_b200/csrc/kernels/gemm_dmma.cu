@@ -568,16 +568,23 @@ DmmaPlan dmma_plan(const GemmProblem& pr, int num_sms, int force_splits, bool al
   // us; 129 x 129 x 30000 307 -> 229, 100 x 80 x 20000 110 -> 95, 33 x 500 x 5000 real
   // double 50 -> 40), and where the default plan has fewer CTAs than SMs and theirs
   // finish sooner (64 x 64 x 64 complex double: one CTA 16.6 us, four 7.6)
-  // Real types take more padding: their small tiles load twice as much per flop. With
-  // op(B) n-major they run at 0.78 to 0.85 of the default rate (800 x 800 x 30621 real
-  // double NT 1.08 times the default's time, 350 x 350 1.05, 2200 x 150 1.04), and in real
-  // double with two k-major operands at 0.73 to 0.93 when k is odd, so that rows packed
-  // back to back are not on 16-byte boundaries and load 8 bytes at a time (2000 x 140 x
-  // 30621 1.16 times the default's time, x 30000 0.91; 350 x 350 x 30621 1.07).
+  // Real types ask for more padding where the problem is long enough to run at the
+  // kernel's rate, since their small tiles load twice as much per flop. With op(B)
+  // n-major those run at 0.78 to 0.85 of the default tiles' rate: from k = 3000 and 256
+  // x 256 on they were slower up to 20 % of padding (800 x 800 x 30621 real double NT
+  // 1.08 times the default's time, 350 x 350 x 9001 1.09; x 501 0.98 and 1.02; 300 x 1500 x
+  // 20001, 23 %, 0.97). In real double with two k-major operands and odd k, rows packed back
+  // to back are not on 16-byte boundaries and load 8 bytes at a time: slower for tall C
+  // from 1.5e9 multiply-adds on (2000 x 140 x 30621 1.16 times, x 30000 0.91; 300 x 1500 x
+  // 20001 0.95). Square C keeps them (350 x 350 x 30621 1.07): with a fill mode, which the
+  // plan does not see, they save up to 40 % there.
   const int64_t def_tiles = tiles(def.bm, def.bn);
   double least = 1.15;
-  if (!dtype_is_complex(pr.dtype) && pr.opB != 0) least = 1.26;
-  if (pr.dtype == kR64 && pr.opA != 0 && pr.opB == 0 && pr.k % 2 != 0) least = 1.31;
+  if (!dtype_is_complex(pr.dtype) && pr.opB != 0 && pr.k >= 3000 && pr.m * pr.n >= 65536)
+    least = 1.21;
+  if (pr.dtype == kR64 && pr.opA != 0 && pr.opB == 0 && pr.k % 2 != 0 && pr.m >= 2 * pr.n &&
+      double(pr.m) * pr.n * pr.k >= 1.5e9)
+    least = 1.31;
   const bool padded =
       double(def_tiles) * def.bm * def.bn >= least * 1024.0 * double(tiles(32, 32));
   if (!padded && def_tiles * def.splits >= num_sms) return def;
