@@ -573,16 +573,17 @@ DmmaPlan dmma_plan(const GemmProblem& pr, int num_sms, int force_splits, bool al
   // n-major those run at 0.78 to 0.85 of the default tiles' rate: from k = 3000 and 256
   // x 256 on they were slower up to 20 % of padding (800 x 800 x 30621 real double NT
   // 1.08 times the default's time, 350 x 350 x 9001 1.09; x 501 0.98 and 1.02; 300 x 1500 x
-  // 20001, 23 %, 0.97). In real double with two k-major operands and odd k, rows packed back
-  // to back are not on 16-byte boundaries and load 8 bytes at a time: slower for tall C
-  // from 1.5e9 multiply-adds on (2000 x 140 x 30621 1.16 times, x 30000 0.91; 300 x 1500 x
-  // 20001 0.95). Square C keeps them (350 x 350 x 30621 1.07): with a fill mode, which the
-  // plan does not see, they save up to 40 % there.
+  // 20001, 23 %, 0.97). In real double with two k-major operands whose rows, packed back to
+  // back, start off 64-byte boundaries, the 128 bytes that a k-step reads of a row touch
+  // one more line, and the small tiles read 1.4 times the rows: slower for tall C from
+  // 1.5e9 multiply-adds on (2000 x 140 x 30621 1.16 times, x 30620 1.12, x 30616 1.05, x
+  // 30608 0.93; 300 x 1500 x 30621 0.93). Square C keeps them (350 x 350 x 30621 1.07): with
+  // a fill mode, which the plan does not see, they save up to 40 % there.
   const int64_t def_tiles = tiles(def.bm, def.bn);
   double least = 1.15;
   if (!dtype_is_complex(pr.dtype) && pr.opB != 0 && pr.k >= 3000 && pr.m * pr.n >= 65536)
     least = 1.21;
-  if (pr.dtype == kR64 && pr.opA != 0 && pr.opB == 0 && pr.k % 2 != 0 && pr.m >= 2 * pr.n &&
+  if (pr.dtype == kR64 && pr.opA != 0 && pr.opB == 0 && pr.k % 8 != 0 && pr.m >= 2 * pr.n &&
       double(pr.m) * pr.n * pr.k >= 1.5e9)
     least = 1.31;
   const bool padded =

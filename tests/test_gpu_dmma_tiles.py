@@ -9,7 +9,8 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("dt,opA,opB,m,n,k,splits", [
     ("float64", 1, 0, 2000, 140, 30621, 6),   # default tiles (small: 7 splits, 1.16)
-    ("float64", 1, 0, 2000, 140, 20000, 7),   # small tiles (default: 6 splits, 0.91)
+    ("float64", 1, 0, 2000, 140, 30620, 6),   # default (small: 7, 1.12)
+    ("float64", 1, 0, 2000, 140, 30608, 7),   # small tiles (default: 6 splits, 0.93)
     ("float64", 1, 0, 600, 140, 20001, 19),   # default (small: 15, 1.06)
     ("float64", 1, 0, 300, 1500, 20001, 11),  # small (default: 4, 0.95)
     ("float64", 1, 0, 350, 350, 9001, 6),     # small (default: 16, 0.96)
